@@ -29,6 +29,8 @@ cudaError_t row_equilibrate(int batch, int n, T* A, long long lda, long long sA,
 template <class T>
 cudaError_t col_scale(int batch, int n, T* X, long long ldx, long long sX, const double* s, cudaStream_t st);
 template <class T>
+cudaError_t row_scale(int batch, int rows, int cols, T* X, const double* s, cudaStream_t st);
+template <class T>
 cudaError_t perm_gather(int batch, int n, int nr, int nc, const T* M, long long sM, const int* perm, int r0, int c0,
                         T* out, long long sO, cudaStream_t st);
 template <class T>
@@ -200,12 +202,24 @@ struct Carver {
 // ---------------------------------------------------------------------------
 // Leaf DtN
 // ---------------------------------------------------------------------------
+// FP64 and complex128 leaves: the rows of A_ii and of W = -A_ie P are brought
+// to one scale before the elimination (powers of two: exact), the inverse's
+// columns back afterwards.  Collocation rows near the leaf's boundary are
+// about p^2 / 2 times those at its centre, so the inverse's columns and W's
+// rows are graded the opposite way, and the digit products (gemm_f64_tc.cu),
+// which keep a row's or column's entries relative to its largest, would drop
+// what the small ones carry: against long double Y is off by 5.8e-16 with the
+// scaling, 8.3e-16 without, and was by 7.8e-16 from FP64 chains (T: 0.96e-15,
+// 1.02e-15, 1.81e-15; 42 leaves of seven problems, p = 9 to 16).
+static bool leaf_rows_scaled(int dtype) { return dtype == F64 || dtype == C128; }
+
 static size_t leaf_dtn_ws(const hps_leaf_dtn_args* a, Carver* cv) {
   const size_t es = dtype_size(a->dtype);
   const int n_i = a->n_pts - a->n_cb;
   cv->take(es * (size_t)a->n_leaves * n_i * a->n_cb);      // A_ie
   cv->take(es * (size_t)a->n_leaves * n_i * a->n_gauss);   // W = -A_ie P
   cv->take(inverse_workspace_bytes(a->dtype, n_i, a->n_leaves));
+  if (leaf_rows_scaled(a->dtype)) cv->take(sizeof(double) * (size_t)a->n_leaves * n_i);
   return cv->used + 256;
 }
 
@@ -220,6 +234,8 @@ static int leaf_dtn_impl(const hps_leaf_dtn_args* a, cudaStream_t st) {
   T* W = (T*)cv.take(sizeof(T) * (size_t)nl * ni * ng);
   const size_t invb = inverse_workspace_bytes(a->dtype, ni, nl);
   void* invws = cv.take(invb);
+  constexpr int dt = DTypeOf<T>::value;
+  double* rscale = leaf_rows_scaled(dt) ? (double*)cv.take(sizeof(double) * (size_t)nl * ni) : nullptr;
   T* Aii = (T*)a->Aii_inv;
   cudaError_t e;
   if (a->coef_complex)
@@ -229,9 +245,6 @@ static int leaf_dtn_impl(const hps_leaf_dtn_args* a, cudaStream_t st) {
     e = leaf_assemble<T, double>(nl, np, ncb, ni, ncb, a->n_ops, a->ops, (const double*)a->coeffs, Aie, ncb,
                                  (long long)ni * ncb, Aii, ni, (long long)ni * ni, st);
   HPS_CHECK(e);
-  // the leaf blocks may use the tensor-memory kernel (FP32, 64 < n <= 224)
-  HPS_CHECK(inverse_batched<T>(ni, Aii, ni, (long long)ni * ni, Aii, ni, (long long)ni * ni, nl, a->info, invws,
-                               invb, st, INV_TENSOR_MEMORY));
   const T one_ = one<T>(), zero_ = zero<T>(), mone = make_scalar<T>(-1.0, 0.0);
   const T* P = (const T*)a->P;
   const T* Q = (const T*)a->Q;
@@ -239,10 +252,18 @@ static int leaf_dtn_impl(const hps_leaf_dtn_args* a, cudaStream_t st) {
   // W = -A_ie P
   HPS_CHECK(gemm_batched<T>(ni, ng, ncb, mone, Aie, ncb, (long long)ni * ncb, P, ng, 0, zero_, nullptr, 0, 0, W,
                             ng, (long long)ni * ng, nl, st));
+  if (rscale) {
+    HPS_CHECK(row_equilibrate<T>(nl, ni, Aii, ni, (long long)ni * ni, rscale, st));
+    HPS_CHECK(row_scale<T>(nl, ni, ng, W, rscale, st));
+  }
+  // the leaf blocks may use the tensor-memory kernel (FP32, 64 < n <= 224)
+  HPS_CHECK(inverse_batched<T>(ni, Aii, ni, (long long)ni * ni, Aii, ni, (long long)ni * ni, nl, a->info, invws,
+                               invb, st, INV_TENSOR_MEMORY));
   // Y[n_cb:] = A_ii^-1 W ;  Y[:n_cb] = P
   HPS_CHECK(gemm_batched<T>(ni, ng, ni, one_, Aii, ni, (long long)ni * ni, W, ng, (long long)ni * ng, zero_,
                             nullptr, 0, 0, Y + (size_t)ncb * ng, ng, (long long)np * ng, nl, st));
   HPS_CHECK(set_rows<T>(nl, ncb, ng, P, ng, Y, ng, (long long)np * ng, st));
+  if (rscale) HPS_CHECK(col_scale<T>(nl, ni, Aii, ni, (long long)ni * ni, rscale, st));
   // T = Q Y
   HPS_CHECK(gemm_batched<T>(ng, ng, np, one_, Q, np, 0, Y, ng, (long long)np * ng, zero_, nullptr, 0, 0,
                             (T*)a->T, ng, (long long)ng * ng, nl, st));

@@ -505,8 +505,8 @@ static cudaError_t launch_skinny(int M, int N, int K, T alpha, const T* A, long 
   return cudaGetLastError();
 }
 
-// Which products run on the tensor cores (gemm_tc.cu): 0 none, 1 the shapes
-// where they were measured faster (default), 2 every FP32 / complex64 product,
+// Which products run on the tensor cores (gemm_tc.cu, gemm_f64_tc.cu): 0 none,
+// 1 the shapes where they were measured faster (default), 2 every product,
 // 3 none and the FP32 8x8 tiles with 4-byte shared loads (gemm_kernel) in
 // place of gemm_f32_v4_kernel, for comparisons.  HPS_GEMM_TC=0 in the
 // environment starts the process at 0; hps_gemm_policy() changes it.
@@ -642,6 +642,31 @@ static cudaError_t run_variant_f32(int v, int M, int N, int K, float alpha, cons
   }
 }
 
+// FP64 and complex128 products: digits on the tensor cores (gemm_f64_tc.cu)
+// against the FP64 pipe.  From K = 16 on the digits win at every size measured
+// (one 16^3 product 18 against 26 us, 4096 of 196 x 56 x 196 in 1.34 against
+// 21.6 ms, 224^3 x 1024 in 1.45 against 24.2 ms); K = 8 is even.  Products
+// with N <= 8 columns read A once either way and their FP64 time grows with N,
+// so both times are estimated, in us: a round of 128-row tiles on 152 SMs
+// takes 0.077 per step of K; the one-row-per-warp kernel 4.2e-6 (N = 1) to
+// 28e-6 (N = 8) per element of A (complex: 11.7e-6 to 74e-6).  Measured at
+// M = K = 196: N = 1 0.67 (FP64) against 0.93 ms, N = 2 1.20 against 0.92, N = 8
+// 4.4 against 0.94 (batch 4096); M = 1792, K = 3584, N = 8, one matrix: 0.13
+// against 0.28 ms.
+static bool f64_on_tensor_cores(int M, int N, int K, int batch, bool cplx) {
+  const int pol = gemm_policy();
+  if (K <= 0 || (pol != 1 && pol != 2)) return false;
+  if (pol == 2) return true;
+  if (N > 8) return K >= 16;
+  if (K < 32) return false;
+  const double tiles = (double)((M + 127) / 128) * batch;
+  const double rounds = (double)(((long long)tiles + 151) / 152);
+  const double tc = 15.0 + rounds * K * (cplx ? 0.154 : 0.077);
+  const double per = cplx ? (N == 1 ? 11.7e-6 : N == 2 ? 20.7e-6 : N <= 4 ? 38e-6 : 74e-6)
+                          : (N == 1 ? 4.2e-6 : N == 2 ? 7.6e-6 : N <= 4 ? 14.5e-6 : 28e-6);
+  return tc < 10.0 + per * M * (double)K * batch;
+}
+
 template <class T>
 cudaError_t gemm_batched(int M, int N, int K, T alpha, const T* A, long long lda, long long sA,
                          const T* B, long long ldb, long long sB, T beta, const T* C, long long ldc,
@@ -655,6 +680,14 @@ cudaError_t gemm_batched(int M, int N, int K, T alpha, const T* A, long long lda
       if (v >= 0)
         return run_variant_f32(v, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
     }
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    if (f64_on_tensor_cores(M, N, K, batch, false))
+      return gemm_f64_tc(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
+  }
+  if constexpr (std::is_same<T, c128>::value) {
+    if (alpha.y == 0.0 && beta.y == 0.0 && f64_on_tensor_cores(M, N, K, batch, true))
+      return gemm_c128_tc(M, N, K, alpha.x, A, lda, sA, B, ldb, sB, beta.x, C, ldc, sC, D, ldd, sD, batch, st);
   }
   if (N <= 8 && K >= 32) {
     if (N == 1)

@@ -1,0 +1,696 @@
+// FP64 and complex128 batched products on the FP16 tensor cores:
+// D = alpha * A @ B + beta * C with every product formed from 8-bit slices
+// (the error-free splitting of Ozaki, Ogita, Oishi and Rump, "Error-free
+// transformations of matrix multiplication by using fast routines of matrix
+// multiplication", 2012).
+//
+// What bounds the plain kernel: GB300 issues two FP64 multiply-adds per SM
+// and clock (1.25 TFLOP/s in all) while kind::f16 MMAs run 2,048 times as
+// many.  Here each row of A and each column of B is scaled by a power of two
+// to 62-bit integers, written as eight balanced base-256 digits (-128..127,
+// exact in FP16), and the 36 digit products of the eight leading weights
+// t + u <= 7 are MMAs.  A product of digits is at most 2^14, so the 8 * 128
+// products that meet in one FP32 accumulator over 128 steps of K stay within
+// 2^24: every accumulator is an exact integer.  After each 128 steps the
+// accumulators are added in 64-bit integers, and the sum is rounded to FP64
+// once, at the end.  What is lost is the tail below 2^-62 of a row's or a
+// column's largest entry and the digit products below the eighth weight
+// (about 2^-60 of the largest product): the FP64 chain's own rounding is
+// 2^-53 of its partial sums at every step.  An entry of D all of whose large
+// factors meet small ones keeps the bound K 2^-56 max|a_i| max|b_j| only:
+// callers bring rows of such operands to one scale first (leaf_dtn_impl).
+//
+// Measured (FP64 chain before, digits): 4096 x (196 x 56 x 196) 21.6 -> 1.34 ms
+// (13.2 TFLOP/s), 512 x (512 x 384 x 512) 82.7 -> 4.5 ms (22.7), 1792^3 10.7
+// -> 0.56 ms, complex 1024 x (256 x 56 x 256) 27.6 -> 1.54 ms, 4096 x (196 x 8 x
+// 196) 4.4 -> 0.94 ms.  The tensor pipe is busy 40% of the large product's
+// time: the conversion (about 24 integer operations an element on the
+// half-rate ALU, A once per 64 columns) bounds it.
+#include "hps_common.cuh"
+#include "hps_internal.h"
+#include "tc_common.cuh"
+
+namespace hps {
+
+namespace {
+
+using tc::mbar_init;
+using tc::smem_u32;
+
+constexpr int OZ_BM = 128;               // rows of an output tile (TMEM lanes)
+constexpr int OZ_BK = 16;                // K steps of a stage (one MMA): a digit row is 32 bytes
+constexpr int OZ_SL = 8;                 // digits
+constexpr int OZ_CHUNK = 8;              // stages summed in the FP32 accumulators (128 steps of K)
+constexpr int OZ_DW = 8;                 // warps 0-7 read the accumulators
+constexpr int OZ_CW = 8;                 // warps 8-15 convert A and B
+constexpr int OZ_CT = OZ_CW * 32;
+constexpr int OZ_MW = OZ_DW + OZ_CW;     // warp 16 issues the MMAs (17-19 fill its warpgroup)
+constexpr int OZ_NT = (OZ_MW + 4) * 32;
+constexpr int OZ_EB = 8;                 // tiles whose exponents are kept (up to NS + 3 are in use)
+constexpr int OZ_APL = OZ_BM * 32;       // bytes of one digit plane of A
+
+template <int BN>
+struct OzCfg {
+  static constexpr int BPL = BN * 32;                       // bytes of one digit plane of B
+  static constexpr int STAGE = OZ_SL * (OZ_APL + BPL);      // digits of 16 steps of K
+  static constexpr int RAW = (OZ_BM + BN) * OZ_BK * 8;      // the same as FP64
+  static constexpr int NS = 3;                              // digit stages
+  static constexpr int NR = (BN <= 16) ? 5 : 3;             // FP64 stages (NR - 1 in flight)
+  static constexpr size_t SMEM = (size_t)NS * STAGE + (size_t)NR * RAW + 1024;
+  static constexpr int COLS = OZ_SL * BN;                   // TMEM columns: one block of BN per weight
+  static constexpr int CW = BN / 2;                         // output columns per reading thread
+  static constexpr int KB = BN * OZ_BK / OZ_CT;             // B values per converting thread and stage
+};
+
+// K-major tile with 32-byte rows, 32-byte swizzle: 8-row groups 256 bytes
+// apart; the 16-byte chunk c of row r lies at chunk c ^ ((r / 4) mod 2).
+// Upper word: group stride, version bits, swizzle code 6; lower word: address.
+constexpr uint32_t OZ_DESC_HI = (256u >> 4) | (1u << 14) | (6u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFF) >> 4) | (1u << 16); }
+
+// D F32 (bits 4-5 = 1), A and B F16 (0), both K-major.
+__host__ __device__ constexpr uint32_t idesc_f16(int N) {
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
+}
+
+__device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %4, 0;\n mov.b64 da, {%1, %5};\n mov.b64 db, {%2, %5};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n" ::"r"(d),
+      "r"(a), "r"(b), "r"(idesc), "r"(acc), "r"(OZ_DESC_HI)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr)
+               : "memory");
+}
+
+// Asynchronous copies of 16 or 8 bytes; `in` false writes zeros and reads nothing.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(in ? 8 : 0) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// |x| (its two words) as floor(|x| * 2^(62 - E)) with |x| < 2^E, E = emax - 1022,
+// plus 0x80 in every byte: byte 7 - t is digit t + 128.  emax > 64, so that a
+// zero or subnormal x is shifted out.
+__device__ __forceinline__ uint2 to_digits(uint32_t lo, uint32_t hi, uint32_t emax20) {
+  const uint32_t mh = (hi & 0xfffffu) | 0x100000u;
+  const uint32_t d = (emax20 - (hi & 0x7ff00000u)) >> 20;
+  uint32_t yl, yh;
+  asm("{\n .reg .b64 m;\n mov.b64 m, {%2, %3};\n shr.u64 m, m, %4;\n add.u64 m, m, 0x8080808080808080;\n"
+      " mov.b64 {%0, %1}, m;\n}\n"
+      : "=r"(yl), "=r"(yh)
+      : "r"(lo << 9), "r"(__funnelshift_l(lo, mh, 9)), "r"(d));
+  return make_uint2(yl, yh);
+}
+
+// Two elements' signs as FP16 factors +-1 and the offsets -+1152.
+__device__ __forceinline__ void sign_pair(uint32_t hi0, uint32_t hi1, uint32_t& one, uint32_t& off) {
+  const uint32_t p = __byte_perm(hi0, hi1, 0x7030) & 0x80008000u;
+  one = p | 0x3C003C00u;
+  off = p ^ 0xE480E480u;
+}
+
+// Two bytes of z as FP16 digits: (1024 + byte) * sign - 1152 * sign.
+__device__ __forceinline__ uint32_t f16_digits(uint32_t z, uint32_t sel, uint32_t one, uint32_t off) {
+  uint32_t h = __byte_perm(z, 0x64646464u, sel), r;
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(h), "r"(one), "r"(off));
+  return r;
+}
+
+// The 96-bit integer (s2, s1, s0) times 2^e, rounded to nearest even.  `odd`
+// is set where the result's exponent is not that of a normal number.
+__device__ __forceinline__ double round_sum(uint32_t s0, uint32_t s1, uint32_t s2, int e, bool& odd) {
+  const uint32_t sg = (uint32_t)((int)s2 >> 31);
+  // magnitude
+  uint32_t m0, m1, m2;
+  asm("sub.cc.u32 %0, %3, %6;\n subc.cc.u32 %1, %4, %6;\n subc.u32 %2, %5, %6;"
+      : "=r"(m0), "=r"(m1), "=r"(m2)
+      : "r"(s0 ^ sg), "r"(s1 ^ sg), "r"(s2 ^ sg), "r"(sg));
+  // top bit to bit 95
+  const bool t2 = m2 != 0, t1 = m1 != 0;
+  const uint32_t a = t2 ? m2 : t1 ? m1 : m0, b = t2 ? m1 : t1 ? m0 : 0u, c = t2 ? m0 : 0u;
+  const int z = __clz(a), w = t2 ? 95 : t1 ? 63 : 31;
+  const uint32_t h = __funnelshift_l(b, a, z), l = __funnelshift_l(c, b, z), r = c << (z & 31);
+  const int x = e + w - z;   // value in [2^x, 2^(x+1))
+  // 53 bits of h:l; 11 dropped bits and the rest
+  const uint32_t up = (((l & 0x7ffu) << 1) | (r ? 1u : 0u)) + ((l >> 11) & 1u) > 0x800u ? 1u : 0u;
+  uint32_t ml = __funnelshift_r(l, h, 11), mh = (h >> 11) + ((uint32_t)(x + 1022) << 20);
+  asm("add.cc.u32 %0, %0, %2;\n addc.u32 %1, %1, 0;" : "+r"(ml), "+r"(mh) : "r"(up));
+  odd = odd || x < -1022 || x > 1022;
+  const bool nz = a != 0;
+  return __hiloint2double(nz ? (int)(mh | (sg & 0x80000000u)) : 0, nz ? (int)ml : 0);
+}
+
+// The same for results outside the normal range (and any other).
+__device__ __noinline__ double round_sum_any(uint32_t s0, uint32_t s1, uint32_t s2, int e) {
+  bool odd = false;
+  const double r = round_sum(s0, s1, s2, 0, odd);
+  return scalbn(r, e);
+}
+
+struct OzArgs {
+  int M, N, K;              // real sizes (complex: N and K doubled)
+  double alpha, beta;
+  const double* A;
+  long long lda, sA;
+  const double* B;
+  long long ldb, sB;
+  const double* C;
+  long long ldc, sC;
+  double* D;
+  long long ldd, sD;
+  int batch, vec_a, vec_d;
+  int* err;
+  const long long* limit;
+};
+
+// One entry of D whose row of A or column of B holds an infinity or a NaN:
+// the multiply-add chain of gemm_kernel.
+template <bool CPLX>
+__device__ __noinline__ double plain_entry(const OzArgs& p, const double* A, const double* B, int m, int n) {
+  const double* a = A + (long long)m * p.lda;
+  if constexpr (CPLX) {
+    const c128* ac = reinterpret_cast<const c128*>(a);
+    c128 s = zero<c128>();
+    for (int k = 0; k < p.K / 2; ++k)
+      s = fma_(ac[k], *reinterpret_cast<const c128*>(B + k * p.ldb + (n & ~1)), s);
+    s = mul(c128{p.alpha, 0.0}, s);
+    return (n & 1) ? s.y : s.x;
+  } else {
+    double s = 0.0;
+    for (int k = 0; k < p.K; ++k) s = fma(a[k], B[k * p.ldb + n], s);
+    return p.alpha * s;
+  }
+}
+
+// One persistent CTA of 20 warps per SM.  For each 128 x BN tile of D
+//   * warps 8-15 stream the tile's rows of A and columns of B through a ring
+//     of FP64 stages twice (cp.async, NR - 1 stages ahead, each warp only
+//     what it uses itself): once for the largest exponents (`expo`), once to
+//     write the eight FP16 digit planes of each into a ring of stages of 16
+//     steps of K (`full`, `empty`);
+//   * one lane of warp 16 issues the MMAs of a stage;
+//   * warps 0-7 read the eight accumulators (one per weight) after every 128
+//     steps, add them into 96-bit integers (`accf`, `acce`), and after the
+//     tile's last ones round the sums and write D.
+// The weights 0-3 and 4-7 are two halves of the tensor memory: the next
+// chunk's MMAs start on the first half while the second is read.  A digit
+// plane of A meets the planes of B with t + u <= 7 side by side, as MMAs of
+// up to 256 columns into consecutive weights' accumulators: A's plane is read
+// from shared memory once for all of them.
+// Registers: 32 columns of 96-bit sums take 96 registers in each of the 256
+// reading threads; the 640 x 96 registers of the launch are divided 144 / 80 / 24.
+// Every wait is bounded: after one that runs out a warp goes through its loop
+// without waiting (so that the named barrier is met by all) and the CTA frees
+// its tensor memory.
+template <int BN, bool CPLX>
+__global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
+  using Cfg = OzCfg<BN>;
+  constexpr int NS = Cfg::NS, NR = Cfg::NR, CW = Cfg::CW, KB = Cfg::KB;
+  extern __shared__ unsigned char oz_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(oz_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t full[NS], empty[NS], accf[2], acce[2], expo[OZ_EB];
+  __shared__ uint32_t committed[NS], acc_committed[2];
+  __shared__ short row_e[OZ_EB][OZ_BM], col_e[OZ_EB][BN];
+  __shared__ uint2 col_part[2][OZ_CT];
+  __shared__ uint32_t tmem_s;
+  __shared__ int fail_s;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const long long limit = *(const volatile long long*)p.limit;
+  if (tid == 0) {
+    for (int i = 0; i < NS; ++i) {
+      mbar_init(&full[i], OZ_CW);
+      mbar_init(&empty[i], 1);
+      committed[i] = 0;
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&accf[i], 1);
+      mbar_init(&acce[i], OZ_DW);
+      acc_committed[i] = 0;
+    }
+    for (int i = 0; i < OZ_EB; ++i) mbar_init(&expo[i], OZ_CW);
+    fail_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == OZ_MW) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)),
+                 "r"(Cfg::COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tmem_s;
+  const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + OZ_BM - 1) / OZ_BM;
+  const long long per_b = (long long)tiles_m * tiles_n, n_units = per_b * p.batch;
+  const int nk = (p.K + OZ_BK - 1) / OZ_BK;
+  bool ok = true;
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    if (ok) ok = (bool)__all_sync(0xffffffffu, tc::mbar_wait(bar, parity, limit));
+  };
+
+  if (warp < OZ_DW) {
+    // ---------------- accumulators -> 96-bit sums -> D ----------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    const int q = warp & 3, cg = warp >> 2;   // TMEM lanes 32 q .., columns CW cg ..
+    const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cg * CW);
+    uint32_t s0[CW], s1[CW], s2[CW];
+    uint32_t ch = 0, tile = 0;
+    for (long long u = blockIdx.x; u < n_units; u += gridDim.x, ++tile) {
+#pragma unroll
+      for (int j = 0; j < CW; ++j) s0[j] = s1[j] = s2[j] = 0;
+      for (int kt = 0; kt < nk; kt += OZ_CHUNK, ++ch) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          wait(&accf[h], ch & 1);
+          tc::fence_after();
+#pragma unroll
+          for (int c = 0; c < CW; c += 4) {
+            uint32_t v[4][4];
+#pragma unroll
+            for (int l = 0; l < 4; ++l) tmem_ld4(tb + (uint32_t)((h * 4 + l) * BN + c), v[l]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              long long x = __float2int_rn(__uint_as_float(v[3][j]));
+#pragma unroll
+              for (int l = 0; l < 3; ++l)
+                asm("mad.wide.s32 %0, %1, %2, %0;"
+                    : "+l"(x)
+                    : "r"(__float2int_rn(__uint_as_float(v[l][j]))), "r"(1 << (8 * (3 - l))));
+              const uint32_t xl = (uint32_t)x, xh = (uint32_t)((unsigned long long)x >> 32);
+              if (h == 0) {
+                asm("add.cc.u32 %0, %0, %2;\n addc.u32 %1, %1, %3;" : "+r"(s1[c + j]), "+r"(s2[c + j]) : "r"(xl), "r"(xh));
+              } else {
+                asm("add.cc.u32 %0, %0, %3;\n addc.cc.u32 %1, %1, %4;\n addc.u32 %2, %2, %5;"
+                    : "+r"(s0[c + j]), "+r"(s1[c + j]), "+r"(s2[c + j])
+                    : "r"(xl), "r"(xh), "r"((uint32_t)((int)xh >> 31)));
+              }
+            }
+          }
+          tc::fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acce[h]);
+          __syncwarp();
+        }
+      }
+      const int eb = tile % OZ_EB;
+      wait(&expo[eb], (tile / OZ_EB) & 1);
+      const long long b = u / per_b;
+      const int r = (int)(u % per_b), m0 = (r / tiles_n) * OZ_BM, n0 = (r % tiles_n) * BN;
+      const int row = m0 + q * 32 + lane, c0 = n0 + cg * CW;
+      if (!ok || row >= p.M || c0 >= p.N) continue;
+      const int re = row_e[eb][q * 32 + lane];
+      const double* Cr = p.C ? p.C + b * p.sC + (long long)row * p.ldc + c0 : nullptr;
+      double* Dr = p.D + b * p.sD + (long long)row * p.ldd + c0;
+      const bool neg = p.alpha == -1.0;
+#pragma unroll
+      for (int g = 0; g < CW; g += 4) {
+        if (c0 + g >= p.N) break;
+        double v[4];
+        bool odd = re >= 0x7ff;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int ce = col_e[eb][cg * CW + g + j];
+          odd = odd || ce >= 0x7ff;
+          v[j] = round_sum(s0[g + j], s1[g + j], s2[g + j], re + ce - 2112, odd);
+        }
+        if (odd || !(neg || p.alpha == 1.0)) {
+          // results beyond the range as the chain gives them, too (a complex
+          // one spreads an infinity to both of its parts)
+          bool plain[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int ce = col_e[eb][cg * CW + g + j];
+            plain[j] = re >= 0x7ff || ce >= 0x7ff;
+            if (!plain[j]) {
+              v[j] = p.alpha * round_sum_any(s0[g + j], s1[g + j], s2[g + j], re + ce - 2112);
+              plain[j] = !isfinite(v[j]);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if ((plain[j] || (CPLX && plain[j ^ 1])) && c0 + g + j < p.N)
+              v[j] = plain_entry<CPLX>(p, p.A + b * p.sA, p.B + b * p.sB, row, c0 + g + j);
+        } else if (neg) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] = -v[j];
+        }
+        if (c0 + g + 4 <= p.N && p.vec_d) {
+          if (Cr) {
+            const double2 x = *reinterpret_cast<const double2*>(Cr + g), y = *reinterpret_cast<const double2*>(Cr + g + 2);
+            v[0] = fma(p.beta, x.x, v[0]);
+            v[1] = fma(p.beta, x.y, v[1]);
+            v[2] = fma(p.beta, y.x, v[2]);
+            v[3] = fma(p.beta, y.y, v[3]);
+          }
+          *reinterpret_cast<double2*>(Dr + g) = make_double2(v[0], v[1]);
+          *reinterpret_cast<double2*>(Dr + g + 2) = make_double2(v[2], v[3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (c0 + g + j < p.N) Dr[g + j] = Cr ? fma(p.beta, Cr[g + j], v[j]) : v[j];
+        }
+      }
+    }
+  } else if (warp < OZ_MW) {
+    // ---------------- FP64 -> exponents, digit planes ----------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+    const int ct = tid - OZ_DW * 32, cw = ct >> 5;
+    const int ar = ct >> 1, ah = ct & 1;                // A: one row, steps 8 ah .. 8 ah + 7
+    const int bn = ct % BN, bk = (ct / BN) * KB;        // B: one column, KB steps
+    const uint32_t a_off = (uint32_t)(ar * 32 + ((ah ^ ((ar >> 2) & 1)) << 4));
+    const uint32_t b_off = (uint32_t)(OZ_SL * OZ_APL + bn * 32 + (((bk >> 3) ^ ((bn >> 2) & 1)) << 4) + (bk & 7) * 2);
+    // this warp's part of an FP64 stage: 16 rows of A (128 bytes each, 16-byte
+    // pieces c at c ^ (row mod 8)), then KB x 32 values of B
+    unsigned char* raw = smem + NS * Cfg::STAGE + cw * (16 * 128 + KB * 256);
+    const uint32_t raw_s = smem_u32(raw);
+    const int rr = ar & 15;
+
+    // the stage that is copied next: a tile's nk stages twice
+    long long lu = blockIdx.x;
+    int lkt = 0, lslot = 0;
+    const double *lA = nullptr, *lB = nullptr;   // this lane's first piece of A, the thread's column of B, at the stage's first step
+    int lrows = 0;                              // rows of this warp inside A
+    bool lb_in = false;
+    const int pr = p.vec_a ? lane >> 3 : lane >> 4, pc = p.vec_a ? lane & 7 : lane & 15;   // row and piece of a copy
+    auto tile_ptrs = [&]() {
+      const long long b = lu / per_b;
+      const int r = (int)(lu % per_b), m = (r / tiles_n) * OZ_BM + 16 * cw, n = (r % tiles_n) * BN + bn;
+      lrows = p.M - m - pr;
+      lA = p.A + b * p.sA + (long long)(m + pr) * p.lda + (p.vec_a ? 2 * pc : pc);
+      lb_in = n < p.N;
+      lB = p.B + b * p.sB + (CPLX ? (long long)(bk >> 1) * p.ldb + (n & ~1) : (long long)bk * p.ldb + n);
+    };
+    if (lu < n_units) tile_ptrs();
+    const double* safe = p.A;   // an address for copies that read nothing
+    auto copy_stage = [&]() {
+      if (lu < n_units) {
+        const uint32_t dst = raw_s + lslot * Cfg::RAW;
+        const int k0 = (lkt < nk ? lkt : lkt - nk) * OZ_BK;
+        const bool whole = k0 + OZ_BK <= p.K;
+        if (p.vec_a) {
+          const uint32_t d = dst + pr * 128;
+          if (whole) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)   // row pr + 4 i: its swizzle is pr ^ 4 (i & 1)
+              cp_async16(d + i * 512 + ((pc ^ pr ^ (4 * (i & 1))) << 4), 4 * i < lrows ? lA + (long long)(4 * i) * p.lda : safe,
+                         4 * i < lrows);
+          } else {
+            const int left = p.K - k0 - 2 * pc;   // values of this piece inside the row
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t x = d + i * 512 + ((pc ^ pr ^ (4 * (i & 1))) << 4);
+              const double* src = lA + (long long)(4 * i) * p.lda;
+              const bool in = 4 * i < lrows;
+              cp_async8(x, in && left > 0 ? src : safe, in && left > 0);
+              cp_async8(x + 8, in && left > 1 ? src + 1 : safe, in && left > 1);
+            }
+          }
+        } else {
+          const bool kin = k0 + pc < p.K;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const bool in = kin && 2 * i < lrows;
+            cp_async8(dst + (2 * i + pr) * 128 + (((pc >> 1) ^ ((2 * i + pr) & 7)) << 4) + (pc & 1) * 8,
+                      in ? lA + (long long)(2 * i) * p.lda : safe, in);
+          }
+        }
+        const int left = lb_in ? p.K - k0 - bk : 0;
+#pragma unroll
+        for (int i = 0; i < KB; ++i) {
+          const double* src = CPLX ? lB + (long long)(KB > 1 ? i >> 1 : 0) * p.ldb + ((bk + i + bn) & 1) : lB + (long long)i * p.ldb;
+          cp_async8(dst + 16 * 128 + i * 256 + lane * 8, i < left ? src : safe, i < left);
+        }
+        lslot = lslot + 1 == NR ? 0 : lslot + 1;
+        lA += OZ_BK;
+        lB += (long long)(CPLX ? OZ_BK / 2 : OZ_BK) * p.ldb;
+        ++lkt;
+        if (lkt == nk) tile_ptrs();
+        if (lkt == 2 * nk) {
+          lkt = 0;
+          lu += gridDim.x;
+          if (lu < n_units) tile_ptrs();
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < NR - 1; ++i) copy_stage();
+    int slot = 0;
+    // the next FP64 stage, and the copy into the slot read before it
+    auto next_raw = [&]() {
+      asm volatile("cp.async.wait_group %0;" ::"n"(NR - 2) : "memory");
+      __syncwarp();   // the warp's copies are visible to all of its lanes, and all have read the slot refilled next
+      const unsigned char* rw = raw + slot * Cfg::RAW;
+      slot = slot + 1 == NR ? 0 : slot + 1;
+      copy_stage();
+      return rw;
+    };
+    // 0x7ff for a row or column that cannot be scaled (infinities, NaN, or nothing but tiny values)
+    auto code = [](uint32_t top, uint32_t low) {
+      const int x = (int)(top >> 20);
+      return (top | low) == 0 ? 1024 : x <= 64 ? 0x7ff : x;
+    };
+
+    uint32_t it = 0, tile = 0;
+    for (long long u = blockIdx.x; u < n_units; u += gridDim.x, ++tile) {
+      uint32_t ae, be;
+      {
+        uint32_t at = 0, al = 0, bt = 0, bl = 0;
+        for (int kt = 0; kt < nk; ++kt) {
+          const unsigned char* rw = next_raw();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint4 v = *reinterpret_cast<const uint4*>(rw + rr * 128 + (((4 * ah + i) ^ (rr & 7)) << 4));
+            at = max(at, max(v.y & 0x7fffffffu, v.w & 0x7fffffffu));
+            al |= v.x | v.z;
+          }
+#pragma unroll
+          for (int i = 0; i < KB; ++i) {
+            const uint2 v = *reinterpret_cast<const uint2*>(rw + 16 * 128 + i * 256 + lane * 8);
+            bt = max(bt, v.y & 0x7fffffffu);
+            bl |= v.x;
+          }
+        }
+        at = max(at, __shfl_xor_sync(0xffffffffu, at, 1));
+        al |= __shfl_xor_sync(0xffffffffu, al, 1);
+        if (CPLX) {   // the two columns of a complex one share their scale
+          bt = max(bt, __shfl_xor_sync(0xffffffffu, bt, 1));
+          bl |= __shfl_xor_sync(0xffffffffu, bl, 1);
+        }
+        col_part[tile & 1][ct] = make_uint2(bt, bl);
+        asm volatile("bar.sync 1, %0;" ::"n"(OZ_CT) : "memory");
+#pragma unroll
+        for (int g = 1; g < OZ_CT / BN; ++g) {
+          const uint2 v = col_part[tile & 1][(ct + g * BN) % OZ_CT];
+          bt = max(bt, v.x);
+          bl |= v.y;
+        }
+        const int ac = code(at, al), bc = code(bt, bl), e = tile % OZ_EB;
+        if (ah == 0) row_e[e][ar] = (short)ac;
+        if (ct < BN) col_e[e][bn] = (short)bc;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&expo[e]);
+        ae = (uint32_t)ac << 20;
+        be = (uint32_t)bc << 20;
+      }
+      for (int kt = 0; kt < nk; ++kt, ++it) {
+        const int s = it % NS;
+        const unsigned char* rw = next_raw();
+        if (it >= NS) wait(&empty[s], (it / NS - 1) & 1);
+        unsigned char* sb = smem + s * Cfg::STAGE;
+        {
+          uint32_t x[16], one[4], off[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint4 v = *reinterpret_cast<const uint4*>(rw + rr * 128 + (((4 * ah + i) ^ (rr & 7)) << 4));
+            x[4 * i] = v.x, x[4 * i + 1] = v.y, x[4 * i + 2] = v.z, x[4 * i + 3] = v.w;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sign_pair(x[4 * i + 1], x[4 * i + 3], one[i], off[i]);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint2 y = to_digits(x[2 * i], x[2 * i + 1], ae);
+            x[2 * i] = y.x, x[2 * i + 1] = y.y;
+          }
+          unsigned char* d = sb + a_off;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {   // digits 2w, 2w + 1
+            uint32_t z[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              z[i] = __byte_perm(x[4 * i + (w < 2)], x[4 * i + 2 + (w < 2)], (w & 1) ? 0x4051 : 0x6273);
+            *reinterpret_cast<uint4*>(d + (2 * w) * OZ_APL) =
+                make_uint4(f16_digits(z[0], 0x4140, one[0], off[0]), f16_digits(z[1], 0x4140, one[1], off[1]),
+                           f16_digits(z[2], 0x4140, one[2], off[2]), f16_digits(z[3], 0x4140, one[3], off[3]));
+            *reinterpret_cast<uint4*>(d + (2 * w + 1) * OZ_APL) =
+                make_uint4(f16_digits(z[0], 0x4342, one[0], off[0]), f16_digits(z[1], 0x4342, one[1], off[1]),
+                           f16_digits(z[2], 0x4342, one[2], off[2]), f16_digits(z[3], 0x4342, one[3], off[3]));
+          }
+        }
+        {
+          constexpr int PB = (KB + 1) / 2;
+          uint2 x[2 * PB];
+          uint32_t one[PB], off[PB];
+#pragma unroll
+          for (int i = 0; i < KB; ++i) {
+            x[i] = *reinterpret_cast<const uint2*>(rw + 16 * 128 + i * 256 + lane * 8);
+            // real view of a complex column: rows 2k, 2k + 1 are (re, -im) or (im, re)
+            if (CPLX && ((bk + i) & 1) && !(bn & 1)) x[i].y ^= 0x80000000u;
+          }
+          if constexpr (KB == 1) x[1] = x[0];
+#pragma unroll
+          for (int i = 0; i < PB; ++i) sign_pair(x[2 * i].y, x[2 * i + 1].y, one[i], off[i]);
+#pragma unroll
+          for (int i = 0; i < 2 * PB; ++i) x[i] = to_digits(x[i].x, x[i].y, be);
+          unsigned char* d = sb + b_off;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            uint32_t d0[PB], d1[PB];
+#pragma unroll
+            for (int i = 0; i < PB; ++i) {
+              const uint32_t z = __byte_perm(w < 2 ? x[2 * i].y : x[2 * i].x, w < 2 ? x[2 * i + 1].y : x[2 * i + 1].x,
+                                             (w & 1) ? 0x4051 : 0x6273);
+              d0[i] = f16_digits(z, 0x4140, one[i], off[i]);
+              d1[i] = f16_digits(z, 0x4342, one[i], off[i]);
+            }
+            unsigned char* o = d + (2 * w) * Cfg::BPL;
+            if constexpr (KB == 4) {
+              *reinterpret_cast<uint2*>(o) = make_uint2(d0[0], d0[1]);
+              *reinterpret_cast<uint2*>(o + Cfg::BPL) = make_uint2(d1[0], d1[1]);
+            } else {
+              static_assert(KB == 1 || KB == 4, "B split");
+              *reinterpret_cast<unsigned short*>(o) = (unsigned short)d0[0];
+              *reinterpret_cast<unsigned short*>(o + Cfg::BPL) = (unsigned short)d1[0];
+            }
+          }
+        }
+        // generic-proxy stores -> visible to the tensor core (async proxy)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[s]);
+        __syncwarp();
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else {
+    // ---------------- MMA issuer ----------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    if (warp == OZ_MW) {
+      uint32_t it = 0, ch = 0;
+      int s = 0;
+      for (long long u = blockIdx.x; u < n_units; u += gridDim.x) {
+        for (int kt = 0; kt < nk; ++kt, ++it) {
+          const bool first = kt % OZ_CHUNK == 0, last = kt % OZ_CHUNK == OZ_CHUNK - 1 || kt == nk - 1;
+          wait(&full[s], (it / NS) & 1);
+          const uint32_t a0 = desc_lo(smem_u32(smem + s * Cfg::STAGE)), b0 = a0 + ((OZ_SL * OZ_APL) >> 4);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (first && ch > 0) wait(&acce[h], (ch - 1) & 1);
+            tc::fence_after();
+            if (ok && lane == 0) {
+#pragma unroll
+              for (int t = 0; t < OZ_SL; ++t) {
+                // weights w of this half with u = w - t >= 0
+                const int w0 = h * 4 > t ? h * 4 : t, nw = h * 4 + 4 - w0;
+                if (nw <= 0) continue;
+                mma_f16(tmem + w0 * BN, a0 + ((t * OZ_APL) >> 4), b0 + (((w0 - t) * Cfg::BPL) >> 4), idesc_f16(nw * BN),
+                        (t == 0 && first) ? 0u : 1u);
+              }
+              if (last) {
+                tc::mma_commit(&accf[h]);
+                acc_committed[h] += 1;
+              }
+              if (h == 1) {
+                tc::mma_commit(&empty[s]);
+                committed[s] += 1;
+              }
+            }
+            __syncwarp();
+          }
+          if (last) ++ch;
+          s = s + 1 == NS ? 0 : s + 1;
+        }
+      }
+    }
+  }
+  if (!ok) fail_s = 1;
+  __syncthreads();
+  if (fail_s && tid == 0) {
+    atomicExch(p.err, 1);
+    // a second bounded chance for the MMAs in flight to finish before the
+    // tensor memory they write is freed
+    for (int s = 0; s < NS; ++s)
+      if (committed[s]) tc::mbar_wait(&empty[s], (committed[s] - 1) & 1, limit);
+    for (int a = 0; a < 2; ++a)
+      if (acc_committed[a]) tc::mbar_wait(&accf[a], (acc_committed[a] - 1) & 1, limit);
+  }
+  tc::fence_before();
+  __syncthreads();
+  if (warp == OZ_MW) {
+    tc::fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::COLS) : "memory");
+  }
+}
+
+template <int BN, bool CPLX>
+cudaError_t launch_oz(OzArgs p, cudaStream_t st) {
+  using Cfg = OzCfg<BN>;
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(gemm_oz_kernel<BN, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+  if (e == cudaSuccess) e = tc_wait_state(&p.err, &p.limit);
+  if (e != cudaSuccess) return e;
+  const long long units = (long long)p.batch * ((p.M + OZ_BM - 1) / OZ_BM) * ((p.N + BN - 1) / BN);
+  note_launch();
+  gemm_oz_kernel<BN, CPLX><<<(unsigned)(units < sms ? units : sms), OZ_NT, Cfg::SMEM, st>>>(p);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+template <bool CPLX>
+static cudaError_t gemm_oz(int M, int N, int K, double alpha, const double* A, long long lda, long long sA,
+                           const double* B, long long ldb, long long sB, double beta, const double* C, long long ldc,
+                           long long sC, double* D, long long ldd, long long sD, int batch, cudaStream_t st) {
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  OzArgs p{M, N, K, alpha, beta, A, lda, sA, B, ldb, sB, C, ldc, sC, D, ldd, sD, batch, 0, 0, nullptr, nullptr};
+  p.vec_a = al16(A) && lda % 2 == 0 && (batch == 1 || sA % 2 == 0);
+  p.vec_d = al16(D) && ldd % 2 == 0 && (batch == 1 || sD % 2 == 0) &&
+            (!C || (al16(C) && ldc % 2 == 0 && (batch == 1 || sC % 2 == 0)));
+  ProfScope ps(KC_GEMM, st, 2.0 * M * (double)N * K * batch * (CPLX ? 2.0 : 1.0));
+  if (N <= 16) return launch_oz<16, CPLX>(p, st);
+  return launch_oz<64, CPLX>(p, st);
+}
+
+cudaError_t gemm_f64_tc(int M, int N, int K, double alpha, const double* A, long long lda, long long sA,
+                        const double* B, long long ldb, long long sB, double beta, const double* C, long long ldc,
+                        long long sC, double* D, long long ldd, long long sD, int batch, cudaStream_t st) {
+  return gemm_oz<false>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
+}
+
+// complex128 as the real product of the interleaved views, sizes (M, 2N, 2K).
+cudaError_t gemm_c128_tc(int M, int N, int K, double alpha, const c128* A, long long lda, long long sA, const c128* B,
+                         long long ldb, long long sB, double beta, const c128* C, long long ldc, long long sC, c128* D,
+                         long long ldd, long long sD, int batch, cudaStream_t st) {
+  return gemm_oz<true>(M, 2 * N, 2 * K, alpha, reinterpret_cast<const double*>(A), 2 * lda, 2 * sA,
+                       reinterpret_cast<const double*>(B), 2 * ldb, 2 * sB, beta, reinterpret_cast<const double*>(C),
+                       2 * ldc, 2 * sC, reinterpret_cast<double*>(D), 2 * ldd, 2 * sD, batch, st);
+}
+
+}  // namespace hps

@@ -413,6 +413,15 @@ int gemm_tc_error_reset() {
   return h;
 }
 
+cudaError_t tc_wait_state(int** err, const long long** limit) {
+  void *e = nullptr, *l = nullptr;
+  cudaError_t c = cudaGetSymbolAddress(&e, g_tc_err);
+  if (c == cudaSuccess) c = cudaGetSymbolAddress(&l, g_tc_spin_limit);
+  *err = static_cast<int*>(e);
+  *limit = static_cast<const long long*>(l);
+  return c;
+}
+
 cudaError_t set_tc_spin_limit(long long polls, long long* previous) {
   long long old = 0;
   cudaError_t e = cudaMemcpyFromSymbol(&old, g_tc_spin_limit, sizeof(old));

@@ -46,6 +46,16 @@ bool gemm_tma_supported(int M, int N, int K, const float* A, long long lda, long
 cudaError_t gemm_tma_f32(int M, int N, int K, float alpha, const float* A, long long lda, long long sA,
                          const float* B, long long ldb, long long sB, float beta, const float* C, long long ldc,
                          long long sC, float* D, long long ldd, long long sD, int batch, cudaStream_t st);
+// FP64 / complex128 products (real alpha, beta) from 8-bit digits on the FP16
+// tensor cores (gemm_f64_tc.cu).  K >= 1; D may alias C only.
+cudaError_t gemm_f64_tc(int M, int N, int K, double alpha, const double* A, long long lda, long long sA,
+                        const double* B, long long ldb, long long sB, double beta, const double* C, long long ldc,
+                        long long sC, double* D, long long ldd, long long sD, int batch, cudaStream_t st);
+cudaError_t gemm_c128_tc(int M, int N, int K, double alpha, const c128* A, long long lda, long long sA, const c128* B,
+                         long long ldb, long long sB, double beta, const c128* C, long long ldc, long long sC, c128* D,
+                         long long ldd, long long sD, int batch, cudaStream_t st);
+// Device addresses of the tensor-core kernels' failure flag and wait limit.
+cudaError_t tc_wait_state(int** err, const long long** limit);
 int gemm_tc_error();
 // Reads the flag and clears it (both synchronise with the device).
 int gemm_tc_error_reset();

@@ -256,6 +256,24 @@ __global__ void col_scale_kernel(int batch, int n, T* X, long long ldx, long lon
   }
 }
 
+// X[b] (rows x cols, contiguous) with row r scaled by s[b * rows + r].
+template <class T>
+__global__ void row_scale_kernel(long long total, int cols, T* X, const double* __restrict__ s) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x)
+    X[e] = scale_by(X[e], s[e / cols]);
+}
+
+template <class T>
+cudaError_t row_scale(int batch, int rows, int cols, T* X, const double* s, cudaStream_t st) {
+  const long long total = (long long)batch * rows * cols;
+  if (total <= 0) return cudaSuccess;
+  const long long g = (total + 255) / 256;
+  ProfScope ps(KC_MOVE, st, 2.0 * (double)total * sizeof(T));
+  note_launch();
+  row_scale_kernel<T><<<(int)(g < 16384 ? g : 16384), 256, 0, st>>>(total, cols, X, s);
+  return cudaGetLastError();
+}
+
 template <class T>
 cudaError_t row_equilibrate(int batch, int n, T* A, long long lda, long long sA, double* s, cudaStream_t st) {
   if (batch <= 0 || n <= 0) return cudaSuccess;
@@ -721,6 +739,7 @@ cudaError_t convert(long long n, const S* src, D* dst, cudaStream_t st) {
   template cudaError_t set_rows<T>(int, int, int, const T*, long long, T*, long long, long long, cudaStream_t); \
   template cudaError_t row_equilibrate<T>(int, int, T*, long long, long long, double*, cudaStream_t);              \
   template cudaError_t col_scale<T>(int, int, T*, long long, long long, const double*, cudaStream_t);           \
+  template cudaError_t row_scale<T>(int, int, int, T*, const double*, cudaStream_t);                            \
   template cudaError_t perm_gather<T>(int, int, int, int, const T*, long long, const int*, int, int, T*,       \
                                       long long, cudaStream_t);                                                  \
   template cudaError_t perm_scatter<T>(int, int, int, int, T*, long long, const int*, int, int, const T*,       \
