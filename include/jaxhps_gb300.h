@@ -45,6 +45,16 @@ extern "C" {
 /* element types */
 enum { HPS_F64 = 0, HPS_F32 = 1, HPS_C128 = 2, HPS_C64 = 3 };
 
+/* May be OR'ed into the dtype of the leaf and merge stages' arguments (no
+ * effect but for FP64 and complex128, with info and blocks of n > 64): the
+ * stage's inverses are refined from the
+ * single-precision inverse instead of eliminated in double.  A matrix on
+ * which the refinement does not reach double precision gets info = -2 and the
+ * stage's output for it is not valid: call the stage again without the flag.
+ * The workspace size differs, ask with the flag set.  No counterpart in the
+ * reference. */
+#define HPS_INVERSE_REFINED 0x100
+
 /* status codes */
 enum {
   HPS_OK = 0,

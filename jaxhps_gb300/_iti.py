@@ -33,12 +33,17 @@ def merge_stage_uniform_2D_ItI(T_arr, h_arr, l: int, device=None, host_device=No
         if h.dim() == 2:
             h = h.unsqueeze(-1)
         h = h.reshape(T.shape[0], T.shape[1], -1).contiguous()
-    S_lst, g_lst = [], []
-    for _ in range(max(int(l), 1)):
-        maps = quad_merge_maps_iti(T.shape[1] // 4)
-        S, g_t, T, h, _, _ = st.merge_level_dtn(T, h, maps, iti=True)
-        S_lst.append(S)
-        g_lst.append(g_t if (g_t is None or multi) else g_t[..., 0])
+    T_leaf, h_leaf = T, h
+    for refined in ([], None):
+        T, h = T_leaf, h_leaf
+        S_lst, g_lst = [], []
+        for _ in range(max(int(l), 1)):
+            maps = quad_merge_maps_iti(T.shape[1] // 4)
+            S, g_t, T, h, _, _ = st.merge_level_dtn(T, h, maps, iti=True, refined=refined)
+            S_lst.append(S)
+            g_lst.append(g_t if (g_t is None or multi) else g_t[..., 0])
+        if not st.unrefined(refined):
+            break
     if subtree_recomp:
         return T, (h if (h is None or multi) else h[..., 0])
     out = (S_lst, g_lst)

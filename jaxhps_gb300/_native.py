@@ -21,6 +21,9 @@ _lib = None
 HPS_F64, HPS_F32, HPS_C128, HPS_C64 = 0, 1, 2, 3
 HPS_CODE_PAD = -(2 ** 31)
 HPS_UP_B_IS_BD_INV, HPS_UP_ITI = 1, 2
+HPS_INVERSE_REFINED = 0x100   # for blocks of n > REFINED_ABOVE
+INFO_NOT_REFINED = -2
+REFINED_ABOVE = 64
 
 TORCH_TO_HPS = {
     torch.float64: HPS_F64,

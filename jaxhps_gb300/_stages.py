@@ -40,6 +40,21 @@ def colour_perm_device(maps, dev):
 
 REAL_TO_COMPLEX = {torch.float64: torch.complex128, torch.float32: torch.complex64}
 
+def refines(dtype, n: int) -> bool:
+    """Whether a stage's inverses of size n are first refined from the
+    single-precision inverse; a stage in which some matrix does not get there
+    (info = -2, ``unrefined``) is run again by elimination."""
+    return dtype in (torch.float64, torch.complex128) and n > nat.REFINED_ABOVE
+
+
+def unrefined(infos) -> bool:
+    """Whether a status word says that an inverse was not refined to double
+    precision (one device sync, none without words)."""
+    if not infos:
+        return False
+    return int(torch.cat([i.reshape(-1) for i in infos]).min()) == nat.INFO_NOT_REFINED
+
+
 # Device bytes the leaf stage's workspace (the assembled leaf operators) may
 # take at once; above it the leaves go in chunks.
 LEAF_WORKSPACE_BUDGET = 16 << 30
@@ -220,39 +235,42 @@ def _local_solve_dtn(pde_problem, P_np, Q_np, device, dtype, keep_inverse, sourc
     h = torch.empty((n_leaves, ng, ns), dtype=dtype, device=dev) if ns else None
     Aii = torch.empty((n_leaves, n_i, n_i), dtype=dtype, device=dev)
     info = torch.zeros(n_leaves, dtype=torch.int32, device=dev)
-    a = nat.LeafDtnArgs(
-        dtype=nat.TORCH_TO_HPS[dtype], coef_complex=int(cplx), n_leaves=n_leaves, n_pts=n_pts, n_cb=n_cb,
-        n_gauss=ng, nsrc=ns, n_ops=ops_t.shape[0], ops=ops_t.data_ptr(), coeffs=coeffs.data_ptr(),
-        source=nat.ptr(f), P=P.data_ptr(), Q=Q.data_ptr(), Y=Y.data_ptr(), T=T.data_ptr(), v=nat.ptr(v),
-        h=nat.ptr(h), Aii_inv=Aii.data_ptr(), info=info.data_ptr(), workspace=None, workspace_bytes=0)
-    wsb = L.hps_local_solve_dtn_workspace_size(C.byref(a))
-    if wsb <= LEAF_WORKSPACE_BUDGET or n_leaves == 1:
-        ws = nat.workspace(wsb, dev)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-        nat.check(L.hps_local_solve_dtn(C.byref(a), nat.stream_ptr()), "hps_local_solve_dtn")
-    else:
-        # the assembled leaf operators of every leaf would not fit the budget:
-        # leaves in chunks (the reference chunks its leaf stage as well,
-        # _device_config.py:65-90), one workspace reused by all chunks
-        chunk = max(1, int(n_leaves * LEAF_WORKSPACE_BUDGET // wsb))
-        es = torch.empty((), dtype=dtype).element_size()
-        for lo in range(0, n_leaves, chunk):
-            hi = min(n_leaves, lo + chunk)
-            cc = coeffs[:, lo:hi].contiguous()
-            b = nat.LeafDtnArgs(
-                dtype=a.dtype, coef_complex=a.coef_complex, n_leaves=hi - lo, n_pts=n_pts, n_cb=n_cb, n_gauss=ng,
-                nsrc=ns, n_ops=a.n_ops, ops=a.ops, coeffs=cc.data_ptr(),
-                source=None if f is None else f.data_ptr() + lo * n_pts * ns * es, P=a.P, Q=a.Q,
-                Y=Y.data_ptr() + lo * n_pts * ng * es, T=T.data_ptr() + lo * ng * ng * es,
-                v=None if v is None else v.data_ptr() + lo * n_pts * ns * es,
-                h=None if h is None else h.data_ptr() + lo * ng * ns * es,
-                Aii_inv=Aii.data_ptr() + lo * n_i * n_i * es, info=info.data_ptr() + lo * 4, workspace=None,
-                workspace_bytes=0)
-            wsc = L.hps_local_solve_dtn_workspace_size(C.byref(b))
-            ws = nat.workspace(wsc, dev)
-            b.workspace, b.workspace_bytes = ws.data_ptr(), ws.numel()
-            nat.check(L.hps_local_solve_dtn(C.byref(b), nat.stream_ptr()), "hps_local_solve_dtn")
-            del cc
+    for flag in ((nat.HPS_INVERSE_REFINED, 0) if refines(dtype, n_i) else (0,)):
+        a = nat.LeafDtnArgs(
+            dtype=nat.TORCH_TO_HPS[dtype] | flag, coef_complex=int(cplx), n_leaves=n_leaves, n_pts=n_pts, n_cb=n_cb,
+            n_gauss=ng, nsrc=ns, n_ops=ops_t.shape[0], ops=ops_t.data_ptr(), coeffs=coeffs.data_ptr(),
+            source=nat.ptr(f), P=P.data_ptr(), Q=Q.data_ptr(), Y=Y.data_ptr(), T=T.data_ptr(), v=nat.ptr(v),
+            h=nat.ptr(h), Aii_inv=Aii.data_ptr(), info=info.data_ptr(), workspace=None, workspace_bytes=0)
+        wsb = L.hps_local_solve_dtn_workspace_size(C.byref(a))
+        if wsb <= LEAF_WORKSPACE_BUDGET or n_leaves == 1:
+            ws = nat.workspace(wsb, dev)
+            a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+            nat.check(L.hps_local_solve_dtn(C.byref(a), nat.stream_ptr()), "hps_local_solve_dtn")
+        else:
+            # the assembled leaf operators of every leaf would not fit the budget:
+            # leaves in chunks (the reference chunks its leaf stage as well,
+            # _device_config.py:65-90), one workspace reused by all chunks
+            chunk = max(1, int(n_leaves * LEAF_WORKSPACE_BUDGET // wsb))
+            es = torch.empty((), dtype=dtype).element_size()
+            for lo in range(0, n_leaves, chunk):
+                hi = min(n_leaves, lo + chunk)
+                cc = coeffs[:, lo:hi].contiguous()
+                b = nat.LeafDtnArgs(
+                    dtype=a.dtype, coef_complex=a.coef_complex, n_leaves=hi - lo, n_pts=n_pts, n_cb=n_cb, n_gauss=ng,
+                    nsrc=ns, n_ops=a.n_ops, ops=a.ops, coeffs=cc.data_ptr(),
+                    source=None if f is None else f.data_ptr() + lo * n_pts * ns * es, P=a.P, Q=a.Q,
+                    Y=Y.data_ptr() + lo * n_pts * ng * es, T=T.data_ptr() + lo * ng * ng * es,
+                    v=None if v is None else v.data_ptr() + lo * n_pts * ns * es,
+                    h=None if h is None else h.data_ptr() + lo * ng * ns * es,
+                    Aii_inv=Aii.data_ptr() + lo * n_i * n_i * es, info=info.data_ptr() + lo * 4, workspace=None,
+                    workspace_bytes=0)
+                wsc = L.hps_local_solve_dtn_workspace_size(C.byref(b))
+                ws = nat.workspace(wsc, dev)
+                b.workspace, b.workspace_bytes = ws.data_ptr(), ws.numel()
+                nat.check(L.hps_local_solve_dtn(C.byref(b), nat.stream_ptr()), "hps_local_solve_dtn")
+                del cc
+        if not flag or not unrefined([info]):
+            break
     if v is not None and not multi:
         v, h = v[..., 0], h[..., 0]
     out = (Y, T, v, h)
@@ -299,16 +317,19 @@ def local_solve_stage_uniform_2D_ItI(pde_problem, host_device=None, device=None,
     h = torch.empty((n_leaves, ng, ns), dtype=dtype, device=dev) if ns else None
     Binv = torch.empty((n_leaves, n_pts, n_pts), dtype=dtype, device=dev)
     info = torch.zeros(n_leaves, dtype=torch.int32, device=dev)
-    a = nat.LeafItiArgs(
-        dtype=nat.TORCH_TO_HPS[dtype], coef_complex=int(cplx), n_leaves=n_leaves, n_pts=n_pts, n_cb=n_cb,
-        n_gauss=ng, nsrc=ns, n_ops=ops_t.shape[0], ops=ops_t.data_ptr(), coeffs=coeffs.data_ptr(),
-        source=nat.ptr(f), G=G.data_ptr(), P=P.data_ptr(), QH=QH.data_ptr(), Y=Y.data_ptr(), T=T.data_ptr(),
-        v=nat.ptr(v), h=nat.ptr(h), B_inv=Binv.data_ptr(), info=info.data_ptr(), workspace=None,
-        workspace_bytes=0)
-    wsb = L.hps_local_solve_iti_workspace_size(C.byref(a))
-    ws = nat.workspace(wsb, dev)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-    nat.check(L.hps_local_solve_iti(C.byref(a), nat.stream_ptr()), "hps_local_solve_iti")
+    for flag in ((nat.HPS_INVERSE_REFINED, 0) if refines(dtype, n_pts) else (0,)):
+        a = nat.LeafItiArgs(
+            dtype=nat.TORCH_TO_HPS[dtype] | flag, coef_complex=int(cplx), n_leaves=n_leaves, n_pts=n_pts, n_cb=n_cb,
+            n_gauss=ng, nsrc=ns, n_ops=ops_t.shape[0], ops=ops_t.data_ptr(), coeffs=coeffs.data_ptr(),
+            source=nat.ptr(f), G=G.data_ptr(), P=P.data_ptr(), QH=QH.data_ptr(), Y=Y.data_ptr(), T=T.data_ptr(),
+            v=nat.ptr(v), h=nat.ptr(h), B_inv=Binv.data_ptr(), info=info.data_ptr(), workspace=None,
+            workspace_bytes=0)
+        wsb = L.hps_local_solve_iti_workspace_size(C.byref(a))
+        ws = nat.workspace(wsb, dev)
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        nat.check(L.hps_local_solve_iti(C.byref(a), nat.stream_ptr()), "hps_local_solve_iti")
+        if not flag or not unrefined([info]):
+            break
     if v is not None and not multi:
         v, h = v[..., 0], h[..., 0]
     out = (Y, T, v, h)
@@ -347,11 +368,14 @@ def raise_on_sync_timeout(infos) -> None:
 
 @phases.ranged("merge level")
 def merge_level_dtn(T_children: torch.Tensor, h_children, maps, keep_D_inv=False, keep_BD_inv=False,
-                    keep_B=False, iti=False, need_T=True, infos=None):
+                    keep_B=False, iti=False, need_T=True, infos=None, refined=None):
     """One batched merge level.  T_children: (n_merges*nch, nb, nb);
     h_children: (n_merges*nch, nb, nsrc) or None.  Returns
     (S, g_tilde, T_out, h_out, D_inv, BD_inv) and B when ``keep_B``.
-    With ``need_T=False`` the merged map is not formed (T_out is None)."""
+    With ``need_T=False`` the merged map is not formed (T_out is None).  ``refined``,
+    a list, lets the inverse be refined where ``refines`` says so and receives
+    its status words: the caller looks at them (``unrefined``) and merges again
+    without the list where one was not refined to double precision."""
     L = nat.lib()
     dev = T_children.device
     dtype = T_children.dtype
@@ -383,6 +407,9 @@ def merge_level_dtn(T_children: torch.Tensor, h_children, maps, keep_D_inv=False
         cp = colour_perm_device(maps, dev)
         if cp is not None:
             a.n_x, a.colour_perm = n_int // 2, cp.data_ptr()
+    if refined is not None and refines(dtype, a.n_x or n_int):
+        a.dtype |= nat.HPS_INVERSE_REFINED
+        refined.append(info)
     wsb = L.hps_merge_level_dtn_workspace_size(C.byref(a))
     ws = nat.workspace(wsb, dev)
     a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
@@ -440,14 +467,20 @@ def merge_stage_generic(T_arr, h_arr, n_levels: int, maps_fn, device=None, subtr
         if h.dim() == 2:
             h = h.unsqueeze(-1)
         h = h.reshape(T.shape[0], T.shape[1], -1).contiguous()
-    S_lst, g_lst, Dinv_lst, infos = [], [], [], []
-    for lvl in range(n_levels):
-        maps = maps_fn(T.shape[1])
-        need_T = lvl < n_levels - 1 or return_T or subtree_recomp
-        S, g_t, T, h, D_inv, _ = merge_level_dtn(T, h, maps, keep_D_inv=keep_D_inv, need_T=need_T, infos=infos)
-        S_lst.append(S)
-        g_lst.append(g_t if (g_t is None or multi) else g_t[..., 0])
-        Dinv_lst.append(D_inv)
+    T_leaf, h_leaf = T, h
+    for refined in ([], None):
+        T, h = T_leaf, h_leaf
+        S_lst, g_lst, Dinv_lst, infos = [], [], [], []
+        for lvl in range(n_levels):
+            maps = maps_fn(T.shape[1])
+            need_T = lvl < n_levels - 1 or return_T or subtree_recomp
+            S, g_t, T, h, D_inv, _ = merge_level_dtn(T, h, maps, keep_D_inv=keep_D_inv, need_T=need_T, infos=infos,
+                                                     refined=refined)
+            S_lst.append(S)
+            g_lst.append(g_t if (g_t is None or multi) else g_t[..., 0])
+            Dinv_lst.append(D_inv)
+        if not unrefined(refined):
+            break
     raise_on_sync_timeout(infos)
     if subtree_recomp:
         return T, (h if (h is None or multi) else h[..., 0])

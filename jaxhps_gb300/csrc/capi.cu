@@ -213,13 +213,33 @@ struct Carver {
 // 1.02e-15, 1.81e-15; 42 leaves of seven problems, p = 9 to 16).
 static bool leaf_rows_scaled(int dtype) { return dtype == F64 || dtype == C128; }
 
+// The dtype field of the stage arguments: element type and HPS_INVERSE_REFINED.
+static int base_dtype(int dtype) { return dtype & ~HPS_INVERSE_REFINED; }
+static bool wants_refined(int dtype, int n, const int* info) {
+  return (dtype & HPS_INVERSE_REFINED) && info && inverse_refined_takes(base_dtype(dtype), n);
+}
+static size_t stage_inverse_bytes(int dtype, int n, int batch, const int* info) {
+  return wants_refined(dtype, n, info) ? inverse_refined_workspace_bytes(base_dtype(dtype), n, batch)
+                                       : inverse_workspace_bytes(base_dtype(dtype), n, batch);
+}
+template <class T>
+static cudaError_t stage_inverse(int dtype, int n, T* X, int batch, int* info, void* ws, size_t bytes, cudaStream_t st,
+                                 int flags) {
+  const long long nn = (long long)n * n;
+  if constexpr (DTypeOf<T>::value == F64 || DTypeOf<T>::value == C128) {
+    if (wants_refined(dtype, n, info))
+      return inverse_refined<T>(n, X, n, nn, X, n, nn, batch, info, ws, bytes, st);
+  }
+  return inverse_batched<T>(n, X, n, nn, X, n, nn, batch, info, ws, bytes, st, flags);
+}
+
 static size_t leaf_dtn_ws(const hps_leaf_dtn_args* a, Carver* cv) {
-  const size_t es = dtype_size(a->dtype);
+  const size_t es = dtype_size(base_dtype(a->dtype));
   const int n_i = a->n_pts - a->n_cb;
   cv->take(es * (size_t)a->n_leaves * n_i * a->n_cb);      // A_ie
   cv->take(es * (size_t)a->n_leaves * n_i * a->n_gauss);   // W = -A_ie P
-  cv->take(inverse_workspace_bytes(a->dtype, n_i, a->n_leaves));
-  if (leaf_rows_scaled(a->dtype)) cv->take(sizeof(double) * (size_t)a->n_leaves * n_i);
+  cv->take(stage_inverse_bytes(a->dtype, n_i, a->n_leaves, a->info));
+  if (leaf_rows_scaled(base_dtype(a->dtype))) cv->take(sizeof(double) * (size_t)a->n_leaves * n_i);
   return cv->used + 256;
 }
 
@@ -232,7 +252,7 @@ static int leaf_dtn_impl(const hps_leaf_dtn_args* a, cudaStream_t st) {
   Carver cv(wsb);
   T* Aie = (T*)cv.take(sizeof(T) * (size_t)nl * ni * ncb);
   T* W = (T*)cv.take(sizeof(T) * (size_t)nl * ni * ng);
-  const size_t invb = inverse_workspace_bytes(a->dtype, ni, nl);
+  const size_t invb = stage_inverse_bytes(a->dtype, ni, nl, a->info);
   void* invws = cv.take(invb);
   constexpr int dt = DTypeOf<T>::value;
   double* rscale = leaf_rows_scaled(dt) ? (double*)cv.take(sizeof(double) * (size_t)nl * ni) : nullptr;
@@ -257,8 +277,7 @@ static int leaf_dtn_impl(const hps_leaf_dtn_args* a, cudaStream_t st) {
     HPS_CHECK(row_scale<T>(nl, ni, ng, W, rscale, st));
   }
   // the leaf blocks may use the tensor-memory kernel (FP32, 64 < n <= 224)
-  HPS_CHECK(inverse_batched<T>(ni, Aii, ni, (long long)ni * ni, Aii, ni, (long long)ni * ni, nl, a->info, invws,
-                               invb, st, INV_TENSOR_MEMORY));
+  HPS_CHECK(stage_inverse<T>(a->dtype, ni, Aii, nl, a->info, invws, invb, st, INV_TENSOR_MEMORY));
   // Y[n_cb:] = A_ii^-1 W ;  Y[:n_cb] = P
   HPS_CHECK(gemm_batched<T>(ni, ng, ni, one_, Aii, ni, (long long)ni * ni, W, ng, (long long)ni * ng, zero_,
                             nullptr, 0, 0, Y + (size_t)ncb * ng, ng, (long long)np * ng, nl, st));
@@ -285,7 +304,7 @@ static int leaf_dtn_impl(const hps_leaf_dtn_args* a, cudaStream_t st) {
 // Leaf ItI
 // ---------------------------------------------------------------------------
 static size_t leaf_iti_ws(const hps_leaf_iti_args* a, Carver* cv) {
-  cv->take(inverse_workspace_bytes(a->dtype, a->n_pts, a->n_leaves));
+  cv->take(stage_inverse_bytes(a->dtype, a->n_pts, a->n_leaves, a->info));
   cv->take(sizeof(double) * (size_t)a->n_leaves * a->n_pts);
   return cv->used + 256;
 }
@@ -297,7 +316,7 @@ static int leaf_iti_impl(const hps_leaf_iti_args* a, cudaStream_t st) {
   unsigned char* wsb = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(a->workspace) + 255) & ~uintptr_t(255));
   Carver cv(wsb);
-  const size_t invb = inverse_workspace_bytes(a->dtype, np, nl);
+  const size_t invb = stage_inverse_bytes(a->dtype, np, nl, a->info);
   void* invws = cv.take(invb);
   double* rscale = (double*)cv.take(sizeof(double) * (size_t)nl * np);
   T* Bm = (T*)a->B_inv;
@@ -314,7 +333,7 @@ static int leaf_iti_impl(const hps_leaf_iti_args* a, cudaStream_t st) {
   // inv(B) = inv(diag(s) B) diag(s): the impedance rows (~p^2/h) and the PDE
   // rows (~p^4/h^2) are brought to one scale before elimination
   HPS_CHECK(row_equilibrate<T>(nl, np, Bm, np, sB, rscale, st));
-  HPS_CHECK(inverse_batched<T>(np, Bm, np, sB, Bm, np, sB, nl, a->info, invws, invb, st));
+  HPS_CHECK(stage_inverse<T>(a->dtype, np, Bm, nl, a->info, invws, invb, st, 0));
   HPS_CHECK(col_scale<T>(nl, np, Bm, np, sB, rscale, st));
   const T one_ = one<T>(), zero_ = zero<T>();
   HPS_CHECK(gemm_batched<T>(np, ng, ncb, one_, Bm, np, sB, (const T*)a->P, ng, 0, zero_, nullptr, 0, 0,
@@ -337,7 +356,7 @@ static int leaf_iti_impl(const hps_leaf_iti_args* a, cudaStream_t st) {
 // Merge level (DtN)
 // ---------------------------------------------------------------------------
 static size_t merge_ws(const hps_merge_args* a, Carver* cv) {
-  const size_t es = dtype_size(a->dtype);
+  const size_t es = dtype_size(base_dtype(a->dtype));
   const size_t nm = (size_t)a->n_merges;
   if (!a->D_inv) cv->take(es * nm * a->n_int * a->n_int);
   cv->take(es * nm * a->n_int * a->n_ext);                       // C
@@ -346,9 +365,9 @@ static size_t merge_ws(const hps_merge_args* a, Carver* cv) {
   if (a->n_x > 0) {
     // two-colour inverse: D12, D21, W, P (n_x^2 each) and W's inverse scratch
     for (int k = 0; k < 4; ++k) cv->take(es * nm * a->n_x * a->n_x);
-    cv->take(inverse_workspace_bytes(a->dtype, a->n_x, a->n_merges));
+    cv->take(stage_inverse_bytes(a->dtype, a->n_x, a->n_merges, a->info));
   } else {
-    cv->take(inverse_workspace_bytes(a->dtype, a->n_int, a->n_merges));
+    cv->take(stage_inverse_bytes(a->dtype, a->n_int, a->n_merges, a->info));
   }
   return cv->used + 256;
 }
@@ -372,7 +391,7 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
     Wm = (T*)cv.take(sizeof(T) * (size_t)nm * nx * nx);
     Pm = (T*)cv.take(sizeof(T) * (size_t)nm * nx * nx);
   }
-  const size_t invb = inverse_workspace_bytes(a->dtype, nx > 0 ? nx : ni, nm);
+  const size_t invb = stage_inverse_bytes(a->dtype, nx > 0 ? nx : ni, nm, a->info);
   void* invws = cv.take(invb);
   const bool with_h = ns > 0 && a->h_children && a->h_out && a->g_tilde;
   // with the block rectangles, the zero blocks of C (and of B unless B is
@@ -397,7 +416,7 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
     HPS_CHECK(perm_gather<T>(nm, ni, nx, nx, D, sD, cp, nx, 0, X21, sx, st));
     HPS_CHECK(gemm_batched<T>(nx, nx, nx, mone, X12, nx, sx, X21, nx, sx, zero_, nullptr, 0, 0, Wm, nx, sx, nm, st));
     HPS_CHECK(add_identity<T>(nm, nx, Wm, sx, st));
-    HPS_CHECK(inverse_batched<T>(nx, Wm, nx, sx, Wm, nx, sx, nm, a->info, invws, invb, st));
+    HPS_CHECK(stage_inverse<T>(a->dtype, nx, Wm, nm, a->info, invws, invb, st, 0));
     HPS_CHECK(gemm_batched<T>(nx, nx, nx, mone, Wm, nx, sx, X12, nx, sx, zero_, nullptr, 0, 0, Pm, nx, sx, nm, st));
     HPS_CHECK(perm_scatter<T>(nm, ni, nx, nx, D, sD, cp, 0, 0, Wm, sx, 0, st));
     HPS_CHECK(perm_scatter<T>(nm, ni, nx, nx, D, sD, cp, 0, nx, Pm, sx, 0, st));
@@ -407,8 +426,7 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
     HPS_CHECK(perm_scatter<T>(nm, ni, nx, nx, D, sD, cp, nx, nx, Wm, sx, 1, st));
   } else {
     // interface matrices: the recursive block inversion may serve FP32
-    HPS_CHECK(inverse_batched<T>(ni, D, ni, (long long)ni * ni, D, ni, (long long)ni * ni, nm, a->info, invws, invb,
-                                 st, INV_BLOCK_RECURSIVE));
+    HPS_CHECK(stage_inverse<T>(a->dtype, ni, D, nm, a->info, invws, invb, st, INV_BLOCK_RECURSIVE));
   }
   T* S = (T*)a->S;
   const long long sDD = (long long)ni * ni, sC = (long long)ni * ne, sB = (long long)ne * ni, sT = (long long)ne * ne;
@@ -771,7 +789,7 @@ int hps_local_solve_dtn(const hps_leaf_dtn_args* a, void* stream) {
               hps_local_solve_dtn_workspace_size(a));
     return HPS_ERR_WORKSPACE;
   }
-  DISPATCH(a->dtype, leaf_dtn_impl, a, (cudaStream_t)stream)
+  DISPATCH(base_dtype(a->dtype), leaf_dtn_impl, a, (cudaStream_t)stream)
 }
 
 size_t hps_local_solve_iti_workspace_size(const hps_leaf_iti_args* a) {
@@ -782,7 +800,7 @@ size_t hps_local_solve_iti_workspace_size(const hps_leaf_iti_args* a) {
 int hps_local_solve_iti(const hps_leaf_iti_args* a, void* stream) {
   if (!a || a->n_leaves <= 0 || a->n_pts <= a->n_cb || a->n_cb <= 0 || a->n_gauss <= 0 || a->n_ops <= 0 ||
       !a->ops || !a->coeffs || !a->G || !a->P || !a->QH || !a->Y || !a->T || !a->B_inv ||
-      (a->dtype != HPS_C128 && a->dtype != HPS_C64)) {
+      (base_dtype(a->dtype) != HPS_C128 && base_dtype(a->dtype) != HPS_C64)) {
     set_error("hps_local_solve_iti: invalid arguments");
     return HPS_ERR_ARG;
   }
@@ -794,7 +812,7 @@ int hps_local_solve_iti(const hps_leaf_iti_args* a, void* stream) {
     set_error("hps_local_solve_iti: workspace too small");
     return HPS_ERR_WORKSPACE;
   }
-  if (a->dtype == HPS_C128) return leaf_iti_impl<c128>(a, (cudaStream_t)stream);
+  if (base_dtype(a->dtype) == HPS_C128) return leaf_iti_impl<c128>(a, (cudaStream_t)stream);
   return leaf_iti_impl<c64>(a, (cudaStream_t)stream);
 }
 
@@ -851,7 +869,7 @@ int hps_merge_level_dtn(const hps_merge_args* a, void* stream) {
     set_error("hps_merge_level_dtn: the two-colour inverse applies to ItI merges only");
     return HPS_ERR_ARG;
   }
-  DISPATCH(a->dtype, merge_impl, a, (cudaStream_t)stream, false)
+  DISPATCH(base_dtype(a->dtype), merge_impl, a, (cudaStream_t)stream, false)
 }
 
 int hps_merge_level_iti(const hps_merge_args* a, void* stream) {
@@ -870,7 +888,7 @@ int hps_merge_level_iti(const hps_merge_args* a, void* stream) {
     set_error("hps_merge_level_iti: two-colour structure needs n_x = n_int / 2 and colour_perm");
     return HPS_ERR_ARG;
   }
-  DISPATCH(a->dtype, merge_impl, a, (cudaStream_t)stream, true)
+  DISPATCH(base_dtype(a->dtype), merge_impl, a, (cudaStream_t)stream, true)
 }
 
 int hps_up_level(const hps_up_args* a, void* stream) {

@@ -642,10 +642,16 @@ static cudaError_t run_variant_f32(int v, int M, int N, int K, float alpha, cons
   }
 }
 
+bool f64_products_on_tensor_cores() {
+  const int pol = gemm_policy();
+  return pol == 1 || pol == 2;
+}
+
 // FP64 and complex128 products: digits on the tensor cores (gemm_f64_tc.cu)
 // against the FP64 pipe.  From K = 16 on the digits win at every size measured
 // (one 16^3 product 18 against 26 us, 4096 of 196 x 56 x 196 in 1.34 against
-// 21.6 ms, 224^3 x 1024 in 1.45 against 24.2 ms); K = 8 is even.  Products
+// 21.6 ms, 224^3 x 1024 in 1.45 against 24.2 ms), below it with a million
+// outputs or more (112 x 112 x 4 x 256 50 against 75 us, x 16 23 against 20).  Products
 // with N <= 8 columns read A once either way and their FP64 time grows with N,
 // so both times are estimated, in us: a round of 128-row tiles on 152 SMs
 // takes 0.077 per step of K; the one-row-per-warp kernel 4.2e-6 (N = 1) to
@@ -654,10 +660,9 @@ static cudaError_t run_variant_f32(int v, int M, int N, int K, float alpha, cons
 // 4.4 against 0.94 (batch 4096); M = 1792, K = 3584, N = 8, one matrix: 0.13
 // against 0.28 ms.
 static bool f64_on_tensor_cores(int M, int N, int K, int batch, bool cplx) {
-  const int pol = gemm_policy();
-  if (K <= 0 || (pol != 1 && pol != 2)) return false;
-  if (pol == 2) return true;
-  if (N > 8) return K >= 16;
+  if (K <= 0 || !f64_products_on_tensor_cores()) return false;
+  if (gemm_policy() == 2) return true;
+  if (N > 8) return K >= 16 || (K >= 4 && (double)M * N * batch >= 1 << 20);
   if (K < 32) return false;
   const double tiles = (double)((M + 127) / 128) * batch;
   const double rounds = (double)(((long long)tiles + 151) / 152);

@@ -171,6 +171,7 @@ struct OzArgs {
   double* D;
   long long ldd, sD;
   int batch, vec_a, vec_d;
+  const int* skip;          // products of the batch that are left out, or null
   int* err;
   const long long* limit;
 };
@@ -256,6 +257,13 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
   const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + OZ_BM - 1) / OZ_BM;
   const long long per_b = (long long)tiles_m * tiles_n, n_units = per_b * p.batch;
   const int nk = (p.K + OZ_BK - 1) / OZ_BK;
+  // the first of the CTA's tiles u, u + gridDim.x, ... that is not left out
+  auto tile_from = [&](long long u) {
+    if (p.skip)
+      while (u < n_units && p.skip[u / per_b]) u += gridDim.x;
+    return u;
+  };
+  const long long u0 = tile_from(blockIdx.x);
   bool ok = true;
   auto wait = [&](uint64_t* bar, uint32_t parity) {
     if (ok) ok = (bool)__all_sync(0xffffffffu, tc::mbar_wait(bar, parity, limit));
@@ -268,7 +276,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
     const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cg * CW);
     uint32_t s0[CW], s1[CW], s2[CW];
     uint32_t ch = 0, tile = 0;
-    for (long long u = blockIdx.x; u < n_units; u += gridDim.x, ++tile) {
+    for (long long u = u0; u < n_units; u = tile_from(u + gridDim.x), ++tile) {
 #pragma unroll
       for (int j = 0; j < CW; ++j) s0[j] = s1[j] = s2[j] = 0;
       for (int kt = 0; kt < nk; kt += OZ_CHUNK, ++ch) {
@@ -380,7 +388,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
     const int rr = ar & 15;
 
     // the stage that is copied next: a tile's nk stages twice
-    long long lu = blockIdx.x;
+    long long lu = u0;
     int lkt = 0, lslot = 0;
     const double *lA = nullptr, *lB = nullptr;   // this lane's first piece of A, the thread's column of B, at the stage's first step
     int lrows = 0;                              // rows of this warp inside A
@@ -441,7 +449,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
         if (lkt == nk) tile_ptrs();
         if (lkt == 2 * nk) {
           lkt = 0;
-          lu += gridDim.x;
+          lu = tile_from(lu + gridDim.x);
           if (lu < n_units) tile_ptrs();
         }
       }
@@ -466,7 +474,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
     };
 
     uint32_t it = 0, tile = 0;
-    for (long long u = blockIdx.x; u < n_units; u += gridDim.x, ++tile) {
+    for (long long u = u0; u < n_units; u = tile_from(u + gridDim.x), ++tile) {
       uint32_t ae, be;
       {
         uint32_t at = 0, al = 0, bt = 0, bl = 0;
@@ -592,7 +600,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
     if (warp == OZ_MW) {
       uint32_t it = 0, ch = 0;
       int s = 0;
-      for (long long u = blockIdx.x; u < n_units; u += gridDim.x) {
+      for (long long u = u0; u < n_units; u = tile_from(u + gridDim.x)) {
         for (int kt = 0; kt < nk; ++kt, ++it) {
           const bool first = kt % OZ_CHUNK == 0, last = kt % OZ_CHUNK == OZ_CHUNK - 1 || kt == nk - 1;
           wait(&full[s], (it / NS) & 1);
@@ -667,9 +675,9 @@ cudaError_t launch_oz(OzArgs p, cudaStream_t st) {
 template <bool CPLX>
 static cudaError_t gemm_oz(int M, int N, int K, double alpha, const double* A, long long lda, long long sA,
                            const double* B, long long ldb, long long sB, double beta, const double* C, long long ldc,
-                           long long sC, double* D, long long ldd, long long sD, int batch, cudaStream_t st) {
+                           long long sC, double* D, long long ldd, long long sD, int batch, cudaStream_t st, const int* skip) {
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  OzArgs p{M, N, K, alpha, beta, A, lda, sA, B, ldb, sB, C, ldc, sC, D, ldd, sD, batch, 0, 0, nullptr, nullptr};
+  OzArgs p{M, N, K, alpha, beta, A, lda, sA, B, ldb, sB, C, ldc, sC, D, ldd, sD, batch, 0, 0, skip, nullptr, nullptr};
   p.vec_a = al16(A) && lda % 2 == 0 && (batch == 1 || sA % 2 == 0);
   p.vec_d = al16(D) && ldd % 2 == 0 && (batch == 1 || sD % 2 == 0) &&
             (!C || (al16(C) && ldc % 2 == 0 && (batch == 1 || sC % 2 == 0)));
@@ -680,17 +688,18 @@ static cudaError_t gemm_oz(int M, int N, int K, double alpha, const double* A, l
 
 cudaError_t gemm_f64_tc(int M, int N, int K, double alpha, const double* A, long long lda, long long sA,
                         const double* B, long long ldb, long long sB, double beta, const double* C, long long ldc,
-                        long long sC, double* D, long long ldd, long long sD, int batch, cudaStream_t st) {
-  return gemm_oz<false>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
+                        long long sC, double* D, long long ldd, long long sD, int batch, cudaStream_t st,
+                        const int* skip) {
+  return gemm_oz<false>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st, skip);
 }
 
 // complex128 as the real product of the interleaved views, sizes (M, 2N, 2K).
 cudaError_t gemm_c128_tc(int M, int N, int K, double alpha, const c128* A, long long lda, long long sA, const c128* B,
                          long long ldb, long long sB, double beta, const c128* C, long long ldc, long long sC, c128* D,
-                         long long ldd, long long sD, int batch, cudaStream_t st) {
+                         long long ldd, long long sD, int batch, cudaStream_t st, const int* skip) {
   return gemm_oz<true>(M, 2 * N, 2 * K, alpha, reinterpret_cast<const double*>(A), 2 * lda, 2 * sA,
                        reinterpret_cast<const double*>(B), 2 * ldb, 2 * sB, beta, reinterpret_cast<const double*>(C),
-                       2 * ldc, 2 * sC, reinterpret_cast<double*>(D), 2 * ldd, 2 * sD, batch, st);
+                       2 * ldc, 2 * sC, reinterpret_cast<double*>(D), 2 * ldd, 2 * sD, batch, st, skip);
 }
 
 }  // namespace hps

@@ -28,6 +28,16 @@ template <class T>
 cudaError_t inverse_batched(int n, const T* A, long long lda, long long sA, T* X, long long ldx,
                             long long sX, int batch, int* info, void* ws, size_t ws_bytes,
                             cudaStream_t st, int flags = 0);
+// FP64 / complex128 inverses refined from the single-precision one
+// (inverse_refined.cu), for n > 64: info[b] = 0, or INV_NOT_REFINED where the
+// refinement does not reach FP64 (X[b] is then not the inverse).  X may alias
+// A; info is needed.
+constexpr int INV_NOT_REFINED = -2;
+bool inverse_refined_takes(int dtype, int n);
+size_t inverse_refined_workspace_bytes(int dtype, int n, int batch);
+template <class T>
+cudaError_t inverse_refined(int n, const T* A, long long lda, long long sA, T* X, long long ldx, long long sX, int batch,
+                            int* info, void* ws, size_t ws_bytes, cudaStream_t st);
 int inverse_rec_policy();
 int set_inverse_rec_policy(int policy);
 
@@ -47,13 +57,16 @@ cudaError_t gemm_tma_f32(int M, int N, int K, float alpha, const float* A, long 
                          const float* B, long long ldb, long long sB, float beta, const float* C, long long ldc,
                          long long sC, float* D, long long ldd, long long sD, int batch, cudaStream_t st);
 // FP64 / complex128 products (real alpha, beta) from 8-bit digits on the FP16
-// tensor cores (gemm_f64_tc.cu).  K >= 1; D may alias C only.
+// tensor cores (gemm_f64_tc.cu).  K >= 1; D may alias C only.  `skip`: device
+// flags, one per product of the batch; where set, the product is left out.
 cudaError_t gemm_f64_tc(int M, int N, int K, double alpha, const double* A, long long lda, long long sA,
                         const double* B, long long ldb, long long sB, double beta, const double* C, long long ldc,
-                        long long sC, double* D, long long ldd, long long sD, int batch, cudaStream_t st);
+                        long long sC, double* D, long long ldd, long long sD, int batch, cudaStream_t st,
+                        const int* skip = nullptr);
 cudaError_t gemm_c128_tc(int M, int N, int K, double alpha, const c128* A, long long lda, long long sA, const c128* B,
                          long long ldb, long long sB, double beta, const c128* C, long long ldc, long long sC, c128* D,
-                         long long ldd, long long sD, int batch, cudaStream_t st);
+                         long long ldd, long long sD, int batch, cudaStream_t st,
+                         const int* skip = nullptr);
 // Device addresses of the tensor-core kernels' failure flag and wait limit.
 cudaError_t tc_wait_state(int** err, const long long** limit);
 int gemm_tc_error();
@@ -80,6 +93,8 @@ int gemm_tune_set(int M, int N, int K, int batch, int variant);
 void gemm_tune_clear();
 int gemm_force_variant(int variant);
 long long gemm_shapes(int mode, long long* out, long long cap);
+// Whether that policy lets FP64 products use the tensor cores.
+bool f64_products_on_tensor_cores();
 // Sets the tensor-core policy of gemm_batched (0, 1, 2); returns the old one.
 int set_gemm_policy(int p);
 

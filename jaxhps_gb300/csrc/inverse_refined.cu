@@ -1,0 +1,238 @@
+// FP64 and complex128 batched inverses from the single-precision inverse and
+// the residual iteration (Schulz, 1933; its fourth-order form first):
+//
+//   X0 = inverse of A in FP32 / complex64         (pivoted kernels of inverse*.cu)
+//   R  = I - A X0,  X1 = X0 + X0 (R + R^2 + R^3)
+//   R  = I - A X1,  X  = X1 + X1 R                where the first R was not small
+//
+// The products with A and with X run on the digit kernel (gemm_f64_tc.cu,
+// FP64 and better), the powers of R, corrections of R, in single precision:
+// they leave an error of about |R|^2 2^-21, so a matrix whose R has row sums
+// of at most 5e-5 is done after the first step (leaves: 2e-6 per entry, row
+// sums 2e-5) and left out of the second; the others (interface and impedance
+// matrices, up to 1e-2) have |R| of at most 1e-8 there, and R^2 is left.  The
+// result carries the rounding of R (1e-16) and no elimination's growth.
+//
+// Why: elimination is a chain of n dependent pivots.  Its panels are bound by
+// the FP64 pipe (two multiply-adds per SM and clock) for many matrices and by
+// the pivot exchange for few (6.6 us a column on a 16-CTA cluster), and its
+// rank-32 updates read and write the whole matrix n / 32 times; the products
+// of size n do not wait for one another's columns.
+// A matrix whose second residual is not small (or whose single-precision
+// inverse met a zero pivot or an overflow) gets info = INV_NOT_REFINED, and
+// the caller runs the elimination.
+#include "hps_common.cuh"
+#include "hps_internal.h"
+
+namespace hps {
+
+namespace {
+
+template <class T> struct Low;
+template <> struct Low<double> { using type = float; };
+template <> struct Low<c128> { using type = c64; };
+
+__device__ __forceinline__ float to_low(double v) { return (float)v; }
+__device__ __forceinline__ c64 to_low(c128 v) { return c64{(float)v.x, (float)v.y}; }
+__device__ __forceinline__ double to_high(float v) { return (double)v; }
+__device__ __forceinline__ c128 to_high(c64 v) { return c128{(double)v.x, (double)v.y}; }
+__device__ __forceinline__ float mag(float v) { return fabsf(v); }
+__device__ __forceinline__ float mag(c64 v) { return fabsf(v.x) + fabsf(v.y); }
+
+constexpr int RF_NT = 256;
+
+// out (contiguous) = A in single precision
+template <class T, class L>
+__global__ void __launch_bounds__(RF_NT) lower_kernel(int n, const T* __restrict__ A, long long lda, long long sA, L* out) {
+  const long long b = blockIdx.y, nn = (long long)n * n;
+  for (long long e = blockIdx.x * (long long)RF_NT + threadIdx.x; e < nn; e += (long long)gridDim.x * RF_NT) {
+    const long long i = e / n;
+    out[b * nn + e] = to_low(A[b * sA + i * lda + (e - i * n)]);
+  }
+}
+
+// out = in, with zeros for what is not finite (a singular or overflowing
+// matrix: its residual is then not small, and no product meets infinities)
+template <class T, class L>
+__global__ void __launch_bounds__(RF_NT) raise_kernel(long long total, const L* __restrict__ in, T* out) {
+  for (long long e = blockIdx.x * (long long)RF_NT + threadIdx.x; e < total; e += (long long)gridDim.x * RF_NT)
+    out[e] = mag(in[e]) < __int_as_float(0x7f800000) ? to_high(in[e]) : zero<T>();
+}
+
+// R (= -A X) += I, its single-precision copy (first step), and the largest row
+// sum per matrix (as the bits of a float; NaN as infinity): a warp per row
+template <class T, class L>
+__global__ void __launch_bounds__(RF_NT) residual_kernel(int n, T* R, L* low, int* top, const int* __restrict__ skip) {
+  const long long b = blockIdx.y, nn = (long long)n * n;
+  if (skip && skip[b]) return;
+  const int lane = threadIdx.x & 31;
+  float most = 0.f;
+  for (int i = blockIdx.x * (RF_NT / 32) + (threadIdx.x >> 5); i < n; i += gridDim.x * (RF_NT / 32)) {
+    T* r = R + b * nn + (long long)i * n;
+    float sum = 0.f;
+    for (int j = lane; j < n; j += 32) {
+      T v = r[j];
+      if (j == i) r[j] = v = add(v, one<T>());
+      const L l = to_low(v);
+      if (low) low[b * nn + (long long)i * n + j] = l;
+      sum += mag(l);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    most = fmaxf(most, sum == sum ? sum : __int_as_float(0x7f800000));
+  }
+  if (lane == 0 && most > 0.f) atomicMax(top + b, __float_as_int(most));
+}
+
+// R += Q
+template <class T, class L>
+__global__ void __launch_bounds__(RF_NT) add_powers_kernel(long long total, T* R, const L* __restrict__ Q) {
+  for (long long e = blockIdx.x * (long long)RF_NT + threadIdx.x; e < total; e += (long long)gridDim.x * RF_NT)
+    R[e] = add(R[e], to_high(Q[e]));
+}
+
+// X (strided) = the first iterate where that is the result
+template <class T>
+__global__ void __launch_bounds__(RF_NT) keep_kernel(int n, const T* __restrict__ Q, T* X, long long ldx, long long sX,
+                                                     const int* __restrict__ skip) {
+  const long long b = blockIdx.y, nn = (long long)n * n;
+  if (!skip[b]) return;
+  for (long long e = blockIdx.x * (long long)RF_NT + threadIdx.x; e < nn; e += (long long)gridDim.x * RF_NT) {
+    const long long i = e / n;
+    X[b * sX + i * ldx + (e - i * n)] = Q[b * nn + e];
+  }
+}
+
+// After the first residual: the matrices that need no second step.
+__global__ void done_kernel(int batch, const int* __restrict__ low_info, int* top, int* skip) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= batch) return;
+  skip[b] = (low_info[b] == 0 && __int_as_float(top[b]) <= 5e-5f) ? 1 : 0;
+  if (!skip[b]) top[b] = 0;
+}
+
+// After the second one.
+__global__ void verdict_kernel(int batch, const int* __restrict__ low_info, const int* __restrict__ top,
+                               const int* __restrict__ skip, int* info) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= batch) return;
+  info[b] = (skip[b] || (low_info[b] == 0 && __int_as_float(top[b]) <= 1e-8f)) ? 0 : INV_NOT_REFINED;
+}
+
+template <class T>
+cudaError_t digits_gemm(int n, double alpha, const T* A, long long lda, long long sA, const T* B, long long sB,
+                        const T* C, T* D, long long ldd, long long sD, int batch, cudaStream_t st, const int* skip) {
+  if constexpr (DTypeOf<T>::value == F64)
+    return gemm_f64_tc(n, n, n, alpha, A, lda, sA, B, n, sB, 1.0, C, n, sB, D, ldd, sD, batch, st, skip);
+  else
+    return gemm_c128_tc(n, n, n, alpha, A, lda, sA, B, n, sB, 1.0, C, n, sB, D, ldd, sD, batch, st, skip);
+}
+
+size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
+
+// Matrices at a time: 4.5 FP64 copies of each, about 2 GB (one matrix always).
+int chunk_of(size_t es, int n, int batch) {
+  const size_t per = 4 * es * (size_t)n * n, most = (size_t)2 << 30;
+  const size_t c = most / per;
+  return c < 1 ? 1 : c > (size_t)batch ? batch : c > 32768 ? 32768 : (int)c;
+}
+
+template <class T>
+cudaError_t run(int n, const T* A, long long lda, long long sA, T* X, long long ldx, long long sX, int batch, int* info,
+                unsigned char* base, size_t bytes, cudaStream_t st) {
+  using L = typename Low<T>::type;
+  const int cap = chunk_of(sizeof(T), n, batch), low_dt = DTypeOf<L>::value;
+  const long long nn = (long long)n * n;
+  unsigned char* w = base;
+  auto take = [&](size_t b) {
+    unsigned char* r = w;
+    w += al256(b);
+    return r;
+  };
+  T* P = (T*)take(sizeof(T) * (size_t)nn * cap);
+  T* Q = (T*)take(sizeof(T) * (size_t)nn * cap);
+  T* R = (T*)take(sizeof(T) * (size_t)nn * cap);
+  L* l0 = (L*)take(sizeof(L) * (size_t)nn * cap);
+  L* l1 = (L*)take(sizeof(L) * (size_t)nn * cap);
+  L* l2 = (L*)take(sizeof(L) * (size_t)nn * cap);
+  int* low_info = (int*)take(sizeof(int) * (size_t)cap);
+  int* top = (int*)take(sizeof(int) * (size_t)cap);
+  int* skip = (int*)take(sizeof(int) * (size_t)cap);
+  const size_t lowb = inverse_workspace_bytes(low_dt, n, cap);
+  void* lows = take(lowb);
+  if ((size_t)(w - base) > bytes) return cudaErrorInvalidValue;
+  const L one_ = one<L>(), zero_ = zero<L>();
+  const int gr = (n + RF_NT / 32 - 1) / (RF_NT / 32);   // CTAs for the rows of one matrix
+  const int gx = (int)((nn + RF_NT * 4 - 1) / (RF_NT * 4) < 256 ? (nn + RF_NT * 4 - 1) / (RF_NT * 4) : 256);
+  cudaError_t e;
+#define RF_TRY(x)                              \
+  do {                                         \
+    if ((e = (x)) != cudaSuccess) return e;    \
+  } while (0)
+  for (int b0 = 0; b0 < batch; b0 += cap) {
+    const int nb = batch - b0 < cap ? batch - b0 : cap;
+    const T* Ab = A + (long long)b0 * sA;
+    const long long total = nn * nb;
+    const int gt = (int)((total + RF_NT * 4 - 1) / (RF_NT * 4) < 16384 ? (total + RF_NT * 4 - 1) / (RF_NT * 4) : 16384);
+    RF_TRY(cudaMemsetAsync(top, 0, sizeof(int) * (size_t)nb, st));
+    note_launch();
+    lower_kernel<T, L><<<dim3(gx, nb), RF_NT, 0, st>>>(n, Ab, lda, sA, l0);
+    RF_TRY(inverse_batched<L>(n, l0, n, nn, l0, n, nn, nb, low_info, lows, lowb, st,
+                              INV_TENSOR_MEMORY | INV_BLOCK_RECURSIVE));
+    note_launch();
+    raise_kernel<T, L><<<gt, RF_NT, 0, st>>>(total, l0, P);
+    // first step: l0 = R, l1 = R + R^2, then l0 = R (R + R^2); P holds X0, Q gets X1
+    RF_TRY(digits_gemm<T>(n, -1.0, Ab, lda, sA, P, nn, nullptr, R, n, nn, nb, st, nullptr));
+    note_launch();
+    residual_kernel<T, L><<<dim3(gr, nb), RF_NT, 0, st>>>(n, R, l0, top, nullptr);
+    note_launch();
+    done_kernel<<<(nb + 255) / 256, 256, 0, st>>>(nb, low_info, top, skip);
+    RF_TRY(gemm_batched<L>(n, n, n, one_, l0, n, nn, l0, n, nn, one_, l0, n, nn, l1, n, nn, nb, st));
+    RF_TRY(gemm_batched<L>(n, n, n, one_, l0, n, nn, l1, n, nn, zero_, nullptr, 0, 0, l2, n, nn, nb, st));
+    note_launch();
+    add_powers_kernel<T, L><<<gt, RF_NT, 0, st>>>(total, R, l2);
+    RF_TRY(digits_gemm<T>(n, 1.0, P, n, nn, R, nn, P, Q, n, nn, nb, st, nullptr));
+    // second step, for the matrices that need it
+    T* Xb = X + (long long)b0 * sX;
+    RF_TRY(digits_gemm<T>(n, -1.0, Ab, lda, sA, Q, nn, nullptr, R, n, nn, nb, st, skip));
+    note_launch();
+    residual_kernel<T, L><<<dim3(gr, nb), RF_NT, 0, st>>>(n, R, (L*)nullptr, top, skip);
+    RF_TRY(digits_gemm<T>(n, 1.0, Q, n, nn, R, nn, Q, Xb, ldx, sX, nb, st, skip));
+    note_launch();
+    keep_kernel<T><<<dim3(gx, nb), RF_NT, 0, st>>>(n, Q, Xb, ldx, sX, skip);
+    note_launch();
+    verdict_kernel<<<(nb + 255) / 256, 256, 0, st>>>(nb, low_info, top, skip, info + b0);
+  }
+#undef RF_TRY
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+bool inverse_refined_takes(int dtype, int n) {
+  return (dtype == F64 || dtype == C128) && n > 64 && f64_products_on_tensor_cores();
+}
+
+size_t inverse_refined_workspace_bytes(int dtype, int n, int batch) {
+  const size_t es = dtype_size(dtype), nn = (size_t)n * n;
+  const int cap = chunk_of(es, n, batch), low_dt = dtype == F64 ? F32 : C64;
+  return 3 * al256(es * nn * cap) + 3 * al256(es / 2 * nn * cap) + 3 * al256(sizeof(int) * (size_t)cap) + al256(inverse_workspace_bytes(low_dt, n, cap)) + 512;
+}
+
+template <class T>
+cudaError_t inverse_refined(int n, const T* A, long long lda, long long sA, T* X, long long ldx, long long sX, int batch,
+                            int* info, void* ws, size_t ws_bytes, cudaStream_t st) {
+  if (batch <= 0) return cudaSuccess;
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~uintptr_t(255));
+  const size_t lost = (size_t)(base - reinterpret_cast<unsigned char*>(ws));
+  if (!ws || !info || ws_bytes < lost) return cudaErrorInvalidValue;
+  ProfScope whole(KC_INVERSE, st, 2.0 * (DTypeOf<T>::value == C128 ? 4.0 : 1.0) * (double)n * n * n * batch);
+  return run<T>(n, A, lda, sA, X, ldx, sX, batch, info, base, ws_bytes - lost, st);
+}
+
+template cudaError_t inverse_refined<double>(int, const double*, long long, long long, double*, long long, long long,
+                                             int, int*, void*, size_t, cudaStream_t);
+template cudaError_t inverse_refined<c128>(int, const c128*, long long, long long, c128*, long long, long long, int, int*,
+                                           void*, size_t, cudaStream_t);
+
+}  // namespace hps
