@@ -112,7 +112,7 @@ HPS_API int hps_inverse_policy(int policy);
 /* Whether the FP32 interface-matrix inverses of the DtN merges
  * (hps_merge_level_dtn, n >= 224) use the recursive 2 x 2 block inversion:
  * two half-size inversions and six half-size batched products per level,
- * down to blocks of n < 224 inverted by pivoted Gauss-Jordan, with no
+ * down to blocks of n <= 128 inverted by pivoted Gauss-Jordan, with no
  * pivoting across blocks (the leading blocks of an interface matrix are
  * interface operators themselves).  1 on (default; HPS_INVERSE_RECURSIVE=0 in
  * the environment starts a process at 0), 0 off (pivoted Gauss-Jordan over the

@@ -215,7 +215,7 @@ __device__ __noinline__ double plain_entry(const OzArgs& p, const double* A, con
 // Every wait is bounded: after one that runs out a warp goes through its loop
 // without waiting (so that the named barrier is met by all) and the CTA frees
 // its tensor memory.
-template <int BN, bool CPLX>
+template <int BN, bool CPLX, bool SKIP>
 __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
   using Cfg = OzCfg<BN>;
   constexpr int NS = Cfg::NS, NR = Cfg::NR, CW = Cfg::CW, KB = Cfg::KB;
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
   const int nk = (p.K + OZ_BK - 1) / OZ_BK;
   // the first of the CTA's tiles u, u + gridDim.x, ... that is not left out
   auto tile_from = [&](long long u) {
-    if (p.skip)
+    if constexpr (SKIP)
       while (u < n_units && p.skip[u / per_b]) u += gridDim.x;
     return u;
   };
@@ -654,19 +654,19 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
   }
 }
 
-template <int BN, bool CPLX>
+template <int BN, bool CPLX, bool SKIP>
 cudaError_t launch_oz(OzArgs p, cudaStream_t st) {
   using Cfg = OzCfg<BN>;
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(gemm_oz_kernel<BN, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+    e = cudaFuncSetAttribute(gemm_oz_kernel<BN, CPLX, SKIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
   if (e == cudaSuccess) e = tc_wait_state(&p.err, &p.limit);
   if (e != cudaSuccess) return e;
   const long long units = (long long)p.batch * ((p.M + OZ_BM - 1) / OZ_BM) * ((p.N + BN - 1) / BN);
   note_launch();
-  gemm_oz_kernel<BN, CPLX><<<(unsigned)(units < sms ? units : sms), OZ_NT, Cfg::SMEM, st>>>(p);
+  gemm_oz_kernel<BN, CPLX, SKIP><<<(unsigned)(units < sms ? units : sms), OZ_NT, Cfg::SMEM, st>>>(p);
   return cudaGetLastError();
 }
 
@@ -682,8 +682,9 @@ static cudaError_t gemm_oz(int M, int N, int K, double alpha, const double* A, l
   p.vec_d = al16(D) && ldd % 2 == 0 && (batch == 1 || sD % 2 == 0) &&
             (!C || (al16(C) && ldc % 2 == 0 && (batch == 1 || sC % 2 == 0)));
   ProfScope ps(KC_GEMM, st, 2.0 * M * (double)N * K * batch * (CPLX ? 2.0 : 1.0));
-  if (N <= 16) return launch_oz<16, CPLX>(p, st);
-  return launch_oz<64, CPLX>(p, st);
+  if (skip) return launch_oz<64, CPLX, true>(p, st);
+  if (N <= 16) return launch_oz<16, CPLX, false>(p, st);
+  return launch_oz<64, CPLX, false>(p, st);
 }
 
 cudaError_t gemm_f64_tc(int M, int N, int K, double alpha, const double* A, long long lda, long long sA,

@@ -1218,8 +1218,8 @@ static size_t flat_workspace_bytes(int dtype, int n, int batch) {
 // i.e. two half-size inversions (recursively) and six half-size products, all
 // batched over the matrices of the call: 2 n^3 flops as Gauss-Jordan, but
 // carried by the GEMM kernels instead of n dependent pivot columns.  Pivots
-// are searched within the blocks the recursion ends at (n < REC_MIN, the
-// Gauss-Jordan kernels), not across them, which suits the interface matrices
+// are searched within the blocks the recursion ends at (n <= REC_BLOCK, the
+// block Gauss-Jordan), not across them, which suits the interface matrices
 // of the DtN merges (their leading blocks are themselves interface operators
 // of the same kind); a zero pivot in a block is reported through info with
 // the block's column offset.  Used for FP32 while inverse_rec_policy() is 1.
@@ -1454,7 +1454,12 @@ static cudaError_t launch_block16(int n, const float* A, long long lda, long lon
   return cudaGetLastError();
 }
 
+// The recursion serves n >= REC_MIN and ends at blocks of n <= REC_BLOCK, all
+// on the block Gauss-Jordan (85 us for one block of 112).  Ending at n < 224
+// left blocks of 129 to 223 to the per-column kernel, 325 us each: 84 of them
+// took 27 of 239 ms of the 512-leaf 3D mixed build, the 168 half-size ones 11.
 constexpr int REC_MIN = 224;
+constexpr int REC_BLOCK = 128;
 static int g_inverse_rec_policy = -1;
 
 int inverse_rec_policy() {
@@ -1476,7 +1481,7 @@ static int rec_split(int n) { return (n / 2) & ~3; }
 // FP32 workspace of the recursion below for (n, batch): W, S, V of this level,
 // the block info scratch, then the larger of the two half-size sub-problems.
 static size_t rec_workspace_bytes(int n, int batch) {
-  if (n < REC_MIN) return al256(sizeof(int) * (size_t)batch) + flat_workspace_bytes(F32, n, batch);
+  if (n <= REC_BLOCK) return al256(sizeof(int) * (size_t)batch) + flat_workspace_bytes(F32, n, batch);
   const int h1 = rec_split(n), h2 = n - h1;
   const size_t lvl = al256(sizeof(float) * (size_t)batch * ((size_t)h1 * h2 + (size_t)h2 * h2 + (size_t)h2 * h1)) +
                      al256(sizeof(int) * (size_t)batch);
@@ -1508,15 +1513,11 @@ static cudaError_t info_merge(int batch, const int* tmp, int* info, int offset, 
 static cudaError_t inverse_rec_f32(int n, const float* A, long long lda, long long sA, float* X, long long ldx,
                                    long long sX, int batch, int* info, unsigned char* ws, size_t ws_bytes,
                                    int col0, cudaStream_t st) {
-  if (n < REC_MIN) {
-    // a block the recursion ends at: block Gauss-Jordan (n <= 128) or the
-    // pivoted per-column kernels; info via scratch
+  if (n <= REC_BLOCK) {
+    // a block the recursion ends at; info via scratch
+    static_assert(REC_BLOCK <= B16_NMAX, "block Gauss-Jordan");
     int* tinfo = reinterpret_cast<int*>(ws);
-    const size_t ib = al256(sizeof(int) * (size_t)batch);
-    cudaError_t e = (n <= B16_NMAX)
-                        ? launch_block16(n, A, lda, sA, X, ldx, sX, batch, info ? tinfo : nullptr, st)
-                        : inverse_batched_flat<float>(n, A, lda, sA, X, ldx, sX, batch, info ? tinfo : nullptr,
-                                                      ws + ib, ws_bytes - ib, st, false);
+    const cudaError_t e = launch_block16(n, A, lda, sA, X, ldx, sX, batch, info ? tinfo : nullptr, st);
     if (e != cudaSuccess || !info) return e;
     return info_merge(batch, tinfo, info, col0, st);
   }
