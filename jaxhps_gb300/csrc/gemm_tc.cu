@@ -467,6 +467,10 @@ cudaError_t gemm_tf32x3(int M, int N, int K, float alpha, const float* A, long l
                         long long sC, float* D, long long ldd, long long sD, int batch, cudaStream_t st) {
   if (M <= 0 || N <= 0 || batch <= 0) return cudaSuccess;
   if (K <= 0) return cudaErrorInvalidValue;   // callers keep K = 0 on the SIMT path
+  if (N > 64) {
+    const cudaError_t e = gemm_wide_f32(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
+    if (e != cudaErrorNotSupported) return e;
+  }
   if (N >= 128)
     return launch_tc<128, false>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
   return launch_tc<64, false>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
@@ -479,6 +483,10 @@ cudaError_t gemm_tf32x3_c64(int M, int N, int K, float alpha, const c64* A, long
                             long long sC, c64* D, long long ldd, long long sD, int batch, cudaStream_t st) {
   if (M <= 0 || N <= 0 || batch <= 0) return cudaSuccess;
   if (K <= 0) return cudaErrorInvalidValue;
+  if (N > 32) {
+    const cudaError_t e = gemm_wide_c64(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
+    if (e != cudaErrorNotSupported) return e;
+  }
   const float* Af = reinterpret_cast<const float*>(A);
   const float* Bf = reinterpret_cast<const float*>(B);
   const float* Cf = reinterpret_cast<const float*>(C);
@@ -842,7 +850,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-static bool encode_map(CUtensorMap* map, const float* base, long long d0, long long d1, long long d2, long long ld,
+bool tma_map_f32(CUtensorMap* map, const float* base, long long d0, long long d1, long long d2, long long ld,
                        long long sb, int box0, int box1, bool swizzle) {
   const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (!encode) return false;
@@ -867,8 +875,8 @@ cudaError_t gemm_tma_f32(int M, int N, int K, float alpha, const float* A, long 
   if (!gemm_tma_supported(M, N, K, A, lda, sA, B, ldb, sB, batch)) return cudaErrorNotSupported;
   const int a_batched = (batch > 1 && sA != 0) ? 1 : 0, b_batched = (batch > 1 && sB != 0) ? 1 : 0;
   CUtensorMap tmA, tmB;
-  if (!encode_map(&tmA, A, K, M, a_batched ? batch : 1, lda, sA, LT_BK, LT_BM, true) ||
-      !encode_map(&tmB, B, N, K, b_batched ? batch : 1, ldb, sB, LT_BN, LT_BK, false))
+  if (!tma_map_f32(&tmA, A, K, M, a_batched ? batch : 1, lda, sA, LT_BK, LT_BM, true) ||
+      !tma_map_f32(&tmB, B, N, K, b_batched ? batch : 1, ldb, sB, LT_BN, LT_BK, false))
     return cudaErrorNotSupported;
   static int sms = 0;
   if (!sms) {

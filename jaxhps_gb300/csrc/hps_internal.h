@@ -7,6 +7,8 @@
 
 #include "hps_common.cuh"
 
+struct CUtensorMap_st;   // CUtensorMap of cuda.h
+
 namespace hps {
 
 // D = alpha*A@B + beta*C over a strided batch (row-major).  C may be null
@@ -56,6 +58,19 @@ bool gemm_tma_supported(int M, int N, int K, const float* A, long long lda, long
 cudaError_t gemm_tma_f32(int M, int N, int K, float alpha, const float* A, long long lda, long long sA,
                          const float* B, long long ldb, long long sB, float beta, const float* C, long long ldc,
                          long long sC, float* D, long long ldd, long long sD, int batch, cudaStream_t st);
+// The same products in 128 x 128 tiles with TMA loads and specialised warps
+// (gemm_tc_wide.cu); cudaErrorNotSupported for layouts TMA does not take
+// (16-byte aligned bases, rows and batch strides).
+cudaError_t gemm_wide_f32(int M, int N, int K, float alpha, const float* A, long long lda, long long sA, const float* B,
+                          long long ldb, long long sB, float beta, const float* C, long long ldc, long long sC, float* D,
+                          long long ldd, long long sD, int batch, cudaStream_t st);
+cudaError_t gemm_wide_c64(int M, int N, int K, float alpha, const c64* A, long long lda, long long sA, const c64* B,
+                          long long ldb, long long sB, float beta, const c64* C, long long ldc, long long sC, c64* D,
+                          long long ldd, long long sD, int batch, cudaStream_t st);
+// Tensor map of a batch of row-major FP32 matrices (d0 inner): box0 x box1
+// boxes, 128-byte swizzled or plain; false where TMA does not take it.
+bool tma_map_f32(::CUtensorMap_st* map, const float* base, long long d0, long long d1, long long d2, long long ld,
+                 long long sb, int box0, int box1, bool swizzle);
 // FP64 / complex128 products (real alpha, beta) from 8-bit digits on the FP16
 // tensor cores (gemm_f64_tc.cu).  K >= 1; D may alias C only.  `skip`: device
 // flags, one per product of the batch; where set, the product is left out.
