@@ -666,6 +666,14 @@ HPS_API int hps_interp_rows(long long n_rows, int n_src, const double* to_pts, c
 HPS_API int hps_gather_cols(long long n_groups, int n_in, int n_out, const int* idx, const double* in, double* out,
                             void* stream);
 
+/* Interpolation nodes (n_leaves, dim, p) of every leaf, the affine images of
+ * the p ascending reference nodes on [-1, 1] (2D: the second axis descending),
+ * and their barycentric weights prod_{k != j} (x_k - x_j), for
+ * hps_interp_from_leaves.  Replaces the per-leaf affine_transform and weights
+ * of _interpolation_methods.py:23-94, :144-225. */
+HPS_API int hps_interp_leaf_nodes(int dim, long long n_leaves, int p, const double* leaf_bounds,
+                                  const double* ref_nodes, double* leaf_nodes, double* leaf_weights, void* stream);
+
 /* Values at n_targets points (targets: (n_targets, dim)) of the piecewise
  * polynomial given by f (n_leaves, p^dim, nsrc) on the leaves' Chebyshev
  * grids (exterior-first order, rearrange: meshgrid index of each point).

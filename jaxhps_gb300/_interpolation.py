@@ -3,9 +3,9 @@ src/jaxhps/_interpolation_methods.py:23-340 and Domain.interp_* in
 src/jaxhps/_domain.py:99-294).
 
 The arithmetic runs in the native library (``hps_interp_rows``,
-``hps_gather_cols``, ``hps_interp_from_leaves`` and batched GEMMs); host code
-builds the small per-leaf node arrays, the barycentric weights and a table
-of the finest cells of the root box for locating target points.
+``hps_gather_cols``, ``hps_interp_leaf_nodes``, ``hps_interp_from_leaves`` and
+batched GEMMs); host code builds a table of the finest cells of the root box
+for locating target points.
 
 Conventions kept from the reference:
 * 2D leaf grids have y descending (the leaf's x nodes ascending, y nodes
@@ -86,13 +86,25 @@ def _cell_table(bounds: np.ndarray, dim: int, max_cells: int = 1 << 26):
         raise NotImplementedError("interpolation: the tree is too deep for the cell table")
     h = (hi - lo) / nc
     cells = np.full(tuple(int(n) for n in nc), -1, dtype=np.int32)
-    for leaf, b in enumerate(bounds):
-        sl = []
-        for a in range(dim):
-            i0 = int(np.rint((b[2 * a] - lo[a]) / h[a]))
-            i1 = int(np.rint((b[2 * a + 1] - lo[a]) / h[a]))
-            sl.append(slice(max(i0, 0), max(min(i1, int(nc[a])), i0 + 1)))
-        cells[tuple(sl)] = leaf
+    i0 = np.rint((bounds[:, 0::2] - lo) / h).astype(np.int64)
+    i1 = np.rint((bounds[:, 1::2] - lo) / h).astype(np.int64)
+    i1 = np.minimum(np.maximum(np.minimum(i1, nc), i0 + 1), nc)
+    i0 = np.maximum(i0, 0)
+    if np.prod(i1 - i0, axis=1).sum() == cells.size:
+        # leaves that tile the box: those of one size in one assignment (4096
+        # leaves one by one took 20 ms)
+        spans, group = np.unique(i1 - i0, axis=0, return_inverse=True)
+        for k, span in enumerate(spans):
+            sel = np.nonzero(group.reshape(-1) == k)[0]
+            at = []
+            for a in range(dim):
+                shape = [1] * (dim + 1)
+                shape[a + 1] = -1
+                at.append(i0[sel, a].reshape([-1] + [1] * dim) + np.arange(span[a]).reshape(shape))
+            cells[tuple(at)] = sel.astype(np.int32).reshape([-1] + [1] * dim)
+    else:
+        for leaf in range(bounds.shape[0]):
+            cells[tuple(slice(i0[leaf, a], i1[leaf, a]) for a in range(dim))] = leaf
     if (cells < 0).any():
         raise ValueError("interpolation: the leaves do not tile their bounding box")
     return np.ascontiguousarray(cells), nc.astype(np.int32), lo, h
@@ -104,25 +116,39 @@ def _device_f64(x, dev) -> torch.Tensor:
     return torch.as_tensor(np.ascontiguousarray(np.asarray(x, dtype=np.float64)), device=dev)
 
 
-def _from_hps(bounds: np.ndarray, p: int, f_evals, targets: np.ndarray, dim: int, device=None) -> torch.Tensor:
+def _device_targets(axes: Sequence[np.ndarray], dev) -> torch.Tensor:
+    """(n_targets, dim) points of meshgrid(*axes), axes exchanged as numpy's default indexing does."""
+    return torch.stack(torch.meshgrid(*[_device_f64(a.reshape(-1), dev) for a in axes], indexing="xy"),
+                       dim=-1).reshape(-1, len(axes))
+
+
+def _host_targets(axes: Sequence[np.ndarray]) -> np.ndarray:
+    return np.stack(np.meshgrid(*axes), axis=len(axes))
+
+
+def _from_hps(bounds: np.ndarray, p: int, f_evals, axes: Sequence[np.ndarray], device=None) -> torch.Tensor:
     L = nat.lib()
     dev = st._device(device)
+    dim = len(axes)
     f = f_evals if isinstance(f_evals, torch.Tensor) else torch.as_tensor(np.asarray(f_evals))
     if f.is_complex():
-        re = _from_hps(bounds, p, f.real, targets, dim, device)
-        im = _from_hps(bounds, p, f.imag, targets, dim, device)
+        re = _from_hps(bounds, p, f.real, axes, device)
+        im = _from_hps(bounds, p, f.imag, axes, device)
         return torch.complex(re, im)
     f = _device_f64(f, dev)
     nl = bounds.shape[0]
     if f.shape[0] != nl or f.shape[1] != p ** dim:
         raise ValueError(f"f_evals has shape {tuple(f.shape)}, expected ({nl}, {p ** dim}[, n_src])")
     ns = f.shape[2] if f.dim() == 3 else 1
-    nodes, wts = _leaf_nodes(bounds, p, dim)
     cells, nc, lo, h = _cell_table(bounds, dim)
-    tb, tn, tw = (_device_f64(x, dev) for x in (bounds, nodes, wts))
+    tb, tref = _device_f64(bounds, dev), _device_f64(chebyshev_points(p), dev)
+    tn = torch.empty((nl, dim, p), dtype=torch.float64, device=dev)
+    tw = torch.empty_like(tn)
+    nat.check(L.hps_interp_leaf_nodes(dim, nl, p, tb.data_ptr(), tref.data_ptr(), tn.data_ptr(), tw.data_ptr(),
+                                      nat.stream_ptr()), "hps_interp_leaf_nodes")
     tr = torch.as_tensor(_rearrange(p, dim), device=dev)
     tc = torch.as_tensor(cells, device=dev)
-    tt = _device_f64(targets.reshape(-1, dim), dev)
+    tt = _device_targets(axes, dev)
     out = torch.empty((tt.shape[0], ns), dtype=torch.float64, device=dev)
     ncb = (C.c_int * dim)(*[int(x) for x in nc])
     lob = (C.c_double * dim)(*[float(x) for x in lo])
@@ -139,9 +165,8 @@ def interp_from_hps_2D(leaves, p: int, f_evals, x_vals, y_vals, device=None, hos
     target_pts (n_y, n_x, 2)) (reference _interpolation_methods.py:23-94)."""
     x = np.asarray(x_vals.cpu() if isinstance(x_vals, torch.Tensor) else x_vals, dtype=np.float64)
     y = np.asarray(y_vals.cpu() if isinstance(y_vals, torch.Tensor) else y_vals, dtype=np.float64)
-    X, Y = np.meshgrid(x, y)
-    target = np.stack([X, Y], axis=2)
-    vals = _from_hps(_leaf_bounds(leaves), p, f_evals, target, 2, device)
+    vals = _from_hps(_leaf_bounds(leaves), p, f_evals, (x, y), device)
+    target = _host_targets((x, y))          # while the device works
     shape = (x.shape[0], y.shape[0]) + tuple(vals.shape[1:])
     return st._to_host(vals.reshape(shape), host_device), target
 
@@ -151,9 +176,8 @@ def interp_from_hps_3D(leaves, p: int, f_evals, x_vals, y_vals, z_vals, device=N
     shape (n_y, n_x, n_z, 3), values reshaped to (n_x, n_y, n_z[, n_src])."""
     x, y, z = (np.asarray(v.cpu() if isinstance(v, torch.Tensor) else v, dtype=np.float64)
                for v in (x_vals, y_vals, z_vals))
-    X, Y, Z = np.meshgrid(x, y, z)
-    target = np.stack([X, Y, Z], axis=3)
-    vals = _from_hps(_leaf_bounds(leaves), p, f_evals, target, 3, device)
+    vals = _from_hps(_leaf_bounds(leaves), p, f_evals, (x, y, z), device)
+    target = _host_targets((x, y, z))
     shape = (x.shape[0], y.shape[0], z.shape[0]) + tuple(vals.shape[1:])
     return st._to_host(vals.reshape(shape), host_device), target
 

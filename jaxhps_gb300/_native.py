@@ -219,6 +219,8 @@ def _declare(lib):
     lib.hps_interp_rows.restype = ci
     lib.hps_gather_cols.argtypes = [cll, ci, ci, vp, vp, vp, vp]
     lib.hps_gather_cols.restype = ci
+    lib.hps_interp_leaf_nodes.argtypes = [ci, cll, ci, vp, vp, vp, vp, vp]
+    lib.hps_interp_leaf_nodes.restype = ci
     lib.hps_interp_from_leaves.argtypes = [ci, cll, ci, vp, ci, vp, vp, vp, vp, vp, P(ci), P(C.c_double),
                                            P(C.c_double), vp, vp, vp]
     lib.hps_interp_from_leaves.restype = ci
@@ -266,7 +268,7 @@ EXPORTED_SYMBOLS = (
     "hps_assemble_u_2d_df", "hps_residual_df_prepare", "hps_assemble_u_2d", "hps_interior_f32", "hps_assemble_rows",
     "hps_refine_points_3d", "hps_refine_check_3d", "hps_mlp_param_count", "hps_mlp_sample_points",
     "hps_mlp_features", "hps_mlp_forward", "hps_mlp_bce", "hps_mlp_backward", "hps_mlp_adam", "hps_panel_map",
-    "hps_scale_batched", "hps_gemm_tc_status", "hps_gemm_tc_status_reset", "hps_set_spin_limits", "hps_inverse_policy", "hps_gemm_tune_set", "hps_gemm_tune_clear", "hps_gemm_force_variant", "hps_gemm_shapes", "hps_iti_combine", "hps_residual_iti_2d", "hps_gemm_policy", "hps_accumulate_max", "hps_refine_points_2d", "hps_refine_check_2d", "hps_interp_rows", "hps_gather_cols", "hps_interp_from_leaves", "hps_assemble_rows_complex",
+    "hps_scale_batched", "hps_gemm_tc_status", "hps_gemm_tc_status_reset", "hps_set_spin_limits", "hps_inverse_policy", "hps_gemm_tune_set", "hps_gemm_tune_clear", "hps_gemm_force_variant", "hps_gemm_shapes", "hps_iti_combine", "hps_residual_iti_2d", "hps_gemm_policy", "hps_accumulate_max", "hps_refine_points_2d", "hps_refine_check_2d", "hps_interp_rows", "hps_gather_cols", "hps_interp_leaf_nodes", "hps_interp_from_leaves", "hps_assemble_rows_complex",
 )
 
 

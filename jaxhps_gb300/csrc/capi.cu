@@ -94,6 +94,8 @@ cudaError_t interp_rows(long long n_rows, int n_src, const double* to, const dou
                         double* out, int rpg, int transposed, cudaStream_t st);
 cudaError_t gather_cols(long long n_groups, int n_in, int n_out, const int* idx, const double* in, double* out,
                         cudaStream_t st);
+cudaError_t interp_leaf_nodes(int dim, long long n_leaves, int p, const double* bounds, const double* ref, double* nodes,
+                              double* wts, cudaStream_t st);
 cudaError_t interp_from_leaves(int dim, long long n_t, int nsrc, const double* tpts, int p, const double* bounds,
                                const double* nodes, const double* wts, const int* rearr, const int* cells,
                                const int* nc, const double* lo, const double* h, const double* f, double* out,
@@ -621,6 +623,17 @@ int hps_gather_cols(long long n_groups, int n_in, int n_out, const int* idx, con
     return HPS_ERR_ARG;
   }
   HPS_CHECK(gather_cols(n_groups, n_in, n_out, idx, in, out, (cudaStream_t)stream));
+  return HPS_OK;
+}
+
+int hps_interp_leaf_nodes(int dim, long long n_leaves, int p, const double* leaf_bounds, const double* ref_nodes,
+                          double* leaf_nodes, double* leaf_weights, void* stream) {
+  if ((dim != 2 && dim != 3) || n_leaves < 0 || p < 2 || !leaf_bounds || !ref_nodes || !leaf_nodes || !leaf_weights) {
+    set_error("hps_interp_leaf_nodes: invalid arguments");
+    return HPS_ERR_ARG;
+  }
+  HPS_CHECK(interp_leaf_nodes(dim, n_leaves, p, leaf_bounds, ref_nodes, leaf_nodes, leaf_weights,
+                              (cudaStream_t)stream));
   return HPS_OK;
 }
 

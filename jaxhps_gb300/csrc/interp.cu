@@ -63,13 +63,24 @@ constexpr int IP_MAXP = 32;
 // descending, as the leaf grid) and wts the matching barycentric weights;
 // cell table (nc[0] x nc[1] (x nc[2])) of leaf indices on the finest cells of
 // the root box [lo, lo + nc h].
-template <int DIM>
+// PLACED: the leaf values are read in raster order through the inverse of
+// rearr, kept in shared memory (ppd <= IP_PLACED points).
+constexpr int IP_PLACED = 4096;
+template <int DIM, bool PLACED>
 __global__ void interp_from_leaves_kernel(long long n_t, int nsrc, const double* __restrict__ tpts, int p, int ppd,
                                           const double* __restrict__ bounds, const double* __restrict__ nodes,
                                           const double* __restrict__ wts, const int* __restrict__ rearr,
                                           const int* __restrict__ cells, int nc0, int nc1, int nc2, double lo0,
                                           double lo1, double lo2, double h0, double h1, double h2,
                                           const double* __restrict__ f, double* out) {
+  __shared__ short place[PLACED ? IP_PLACED : 1];
+  if (PLACED) {
+    for (int c = threadIdx.x; c < ppd; c += blockDim.x) place[c] = 0;
+    __syncthreads();
+    for (int c = threadIdx.x; c < ppd; c += blockDim.x)
+      if ((unsigned)rearr[c] < (unsigned)ppd) place[rearr[c]] = (short)c;
+    __syncthreads();
+  }
   const long long tot = n_t * nsrc;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot; e += (long long)gridDim.x * blockDim.x) {
     const long long t = e / nsrc;
@@ -102,28 +113,87 @@ __global__ void interp_from_leaves_kernel(long long n_t, int nsrc, const double*
           if (in && (leaf < 0 || l < leaf)) leaf = l;
         }
     if (leaf < 0) leaf = 0;
-    // 1D barycentric factors on the leaf's nodes
+    // 1D barycentric factors on the leaf's nodes: 1 / (w d), times 1 / their sum
+    // (one division a node: they are most of the FP64 work, 512 x 512 targets
+    // at p = 16 took 0.56 ms with two, and the tensor sum below without its
+    // inner sums twice the multiply-adds)
     double fac[3][IP_MAXP];
     for (int a = 0; a < DIM; ++a) {
       const double* nd = nodes + (leaf * DIM + a) * p;
       const double* wt = wts + (leaf * DIM + a) * p;
       double nf = 0.0;
-      for (int i = 0; i < p; ++i) nf += 1.0 / (wt[i] * nudge(x[a] - nd[i]));
-      for (int i = 0; i < p; ++i) fac[a][i] = 1.0 / (nudge(x[a] - nd[i]) * wt[i] * nf);
+      for (int i = 0; i < p; ++i) {
+        fac[a][i] = 1.0 / (wt[i] * nudge(x[a] - nd[i]));
+        nf += fac[a][i];
+      }
+      nf = 1.0 / nf;
+      for (int i = 0; i < p; ++i) fac[a][i] *= nf;
     }
     const double* fl = f + leaf * (long long)ppd * nsrc + s;
     double acc = 0.0;
-    for (int c = 0; c < ppd; ++c) {
-      const int m = rearr[c];
-      double wgt;
-      if (DIM == 2)
-        wgt = fac[0][m / p] * fac[1][m % p];
-      else
-        wgt = fac[0][m / (p * p)] * fac[1][(m / p) % p] * fac[2][m % p];
-      acc = fma(wgt, fl[(long long)c * nsrc], acc);
+    if (PLACED) {
+      int m = 0;
+      for (int i = 0; i < p; ++i) {
+        double row = 0.0;
+        for (int j = 0; j < p; ++j) {
+          if (DIM == 2) {
+            row = fma(fac[1][j], fl[(long long)place[m++] * nsrc], row);
+          } else {
+            double line = 0.0;
+            for (int k = 0; k < p; ++k) line = fma(fac[2][k], fl[(long long)place[m++] * nsrc], line);
+            row = fma(fac[1][j], line, row);
+          }
+        }
+        acc = fma(fac[0][i], row, acc);
+      }
+    } else {
+      for (int c = 0; c < ppd; ++c) {
+        const int m = rearr[c];
+        double wgt;
+        if (DIM == 2)
+          wgt = fac[0][m / p] * fac[1][m % p];
+        else
+          wgt = fac[0][m / (p * p)] * fac[1][(m / p) % p] * fac[2][m % p];
+        acc = fma(wgt, fl[(long long)c * nsrc], acc);
+      }
     }
     out[e] = acc;
   }
+}
+
+// Interpolation nodes (affine image of the p reference nodes, 2D: the second
+// axis descending) and barycentric weights prod_{k != j} (x_k - x_j) of every
+// leaf: a thread per node.  The products are rounded one by one in the order
+// of k, as the host tables are.
+__global__ void leaf_nodes_kernel(long long total, int dim, int p, const double* __restrict__ bounds,
+                                  const double* __restrict__ ref, double* nodes, double* wts) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+    const int j = (int)(e % p);
+    const long long la = e / p;
+    const int a = (int)(la % dim);
+    const long long leaf = la / dim;
+    const double lo = bounds[(leaf * dim + a) * 2], hi = bounds[(leaf * dim + a) * 2 + 1];
+    const double half = __dmul_rn(0.5, __dsub_rn(hi, lo)), mid = __dmul_rn(0.5, __dadd_rn(lo, hi));
+    const bool flip = dim == 2 && a == 1;
+    auto node = [&](int k) { return __dadd_rn(__dmul_rn(half, ref[flip ? p - 1 - k : k]), mid); };
+    const double x = node(j);
+    double w = 1.0;
+    for (int k = 0; k < p; ++k)
+      if (k != j) w = __dmul_rn(w, __dsub_rn(node(k), x));
+    nodes[e] = x;
+    wts[e] = w;
+  }
+}
+
+cudaError_t interp_leaf_nodes(int dim, long long n_leaves, int p, const double* bounds, const double* ref, double* nodes,
+                              double* wts, cudaStream_t st) {
+  const long long total = n_leaves * dim * p;
+  if (total <= 0) return cudaSuccess;
+  const long long g = (total + 255) / 256;
+  ProfScope ps(KC_MOVE, st, 16.0 * (double)total);
+  note_launch();
+  leaf_nodes_kernel<<<(int)(g < 16384 ? g : 16384), 256, 0, st>>>(total, dim, p, bounds, ref, nodes, wts);
+  return cudaGetLastError();
 }
 
 cudaError_t interp_rows(long long n_rows, int n_src, const double* to, const double* src, const double* w,
@@ -158,13 +228,17 @@ cudaError_t interp_from_leaves(int dim, long long n_t, int nsrc, const double* t
   if (g > 65535) g = 65535;
   ProfScope ps(KC_MOVE, st, (double)n_t * nsrc * (2.0 * ppd + 8.0 * dim * p));
   note_launch();
+  auto launch = [&](auto kernel) {
+    kernel<<<(int)g, 128, 0, st>>>(n_t, nsrc, tpts, p, ppd, bounds, nodes, wts, rearr, cells, nc[0], nc[1],
+                                   dim == 3 ? nc[2] : 1, lo[0], lo[1], dim == 3 ? lo[2] : 0.0, h[0], h[1],
+                                   dim == 3 ? h[2] : 1.0, f, out);
+  };
   if (dim == 2)
-    interp_from_leaves_kernel<2><<<(int)g, 128, 0, st>>>(n_t, nsrc, tpts, p, ppd, bounds, nodes, wts, rearr, cells,
-                                                        nc[0], nc[1], 1, lo[0], lo[1], 0.0, h[0], h[1], 1.0, f, out);
+    launch(interp_from_leaves_kernel<2, true>);
+  else if (ppd <= IP_PLACED)
+    launch(interp_from_leaves_kernel<3, true>);
   else
-    interp_from_leaves_kernel<3><<<(int)g, 128, 0, st>>>(n_t, nsrc, tpts, p, ppd, bounds, nodes, wts, rearr, cells,
-                                                        nc[0], nc[1], nc[2], lo[0], lo[1], lo[2], h[0], h[1], h[2],
-                                                        f, out);
+    launch(interp_from_leaves_kernel<3, false>);
   return cudaGetLastError();
 }
 

@@ -112,3 +112,50 @@ def test_domain_interp_to_interior_points_polynomial(cuda):
     assert np.allclose(out3.numpy(), g(dom3.interior_points), atol=1e-11)
     with pytest.raises(NotImplementedError):
         dom.interp_to_boundary_points(None, None, None)
+
+
+@pytest.mark.parametrize("dim,p", [(2, 4), (2, 16), (2, 32), (3, 5), (3, 17)])
+def test_interp_leaf_nodes_and_raster_sum(cuda, dim, p):
+    """Device nodes and weights against the host tables (the same roundings),
+    and the interpolated values on both sides of the size up to which the leaf
+    values are read in raster order (p^3 = 4913 is above it): polynomials of
+    degree < p, targets inside the leaves, bound p^dim x 2^-50 of the data."""
+    rng = np.random.default_rng(dim * 100 + p)
+    if dim == 2:
+        bounds = _adaptive_bounds_2D()
+    else:
+        top = uniform_leaf_bounds_3D((0.0, 1.0, 0.0, 1.0, 0.0, 1.0), 1)
+        bounds = np.concatenate([uniform_leaf_bounds_3D(tuple(top[0]), 1), top[1:]])
+    nl = bounds.shape[0]
+    nodes, wts = ip._leaf_nodes(bounds, p, dim)
+    tb, tref = (torch.as_tensor(a, device=cuda) for a in (bounds, ip.chebyshev_points(p)))
+    tn = torch.empty((nl, dim, p), dtype=torch.float64, device=cuda)
+    tw = torch.empty_like(tn)
+    ip.nat.check(ip.nat.lib().hps_interp_leaf_nodes(dim, nl, p, tb.data_ptr(), tref.data_ptr(), tn.data_ptr(),
+                                                    tw.data_ptr(), ip.nat.stream_ptr()), "hps_interp_leaf_nodes")
+    assert np.array_equal(tn.cpu().numpy(), nodes)
+    assert np.abs(tw.cpu().numpy() / wts - 1).max() < p * 2.0 ** -52
+    pts = (bounds_to_cheby_points_2D if dim == 2 else bounds_to_cheby_points_3D)(bounds, p)
+    coef = rng.standard_normal((dim, min(p, 6)))
+    poly = lambda x: np.prod([np.polyval(coef[a], x[..., a]) for a in range(dim)], axis=0)   # noqa: E731
+    lo, hi = bounds[:, 0::2].min(0), bounds[:, 1::2].max(0)
+    ax = [lo[a] + (hi[a] - lo[a]) * (np.arange(n) + 0.37) / n for a, n in zip(range(dim), (6, 5, 7))]
+    fn = ip.interp_from_hps_2D if dim == 2 else ip.interp_from_hps_3D
+    f = poly(pts)
+    vals, tp = fn(bounds, p, f, *ax)
+    assert np.abs(vals.cpu().numpy().reshape(-1) - poly(tp).reshape(-1)).max() < p ** dim * 2.0 ** -50 * np.abs(f).max()
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_complex_and_several_sources_take_the_same_targets(cuda, dim):
+    p = 5
+    bounds = (_adaptive_bounds_2D() if dim == 2 else uniform_leaf_bounds_3D((0.0, 1.0, 0.0, 1.0, 0.0, 1.0), 1))
+    rng = np.random.default_rng(dim)
+    f = rng.standard_normal((bounds.shape[0], p ** dim, 2))
+    lo, hi = bounds[:, 0::2].min(0), bounds[:, 1::2].max(0)
+    ax = [np.linspace(lo[a], hi[a], n) for a, n in zip(range(dim), (4, 6, 3))]
+    fn = ip.interp_from_hps_2D if dim == 2 else ip.interp_from_hps_3D
+    both, tp = fn(bounds, p, f, *ax)
+    z, _ = fn(bounds, p, f[..., 0] + 1j * f[..., 1], *ax)
+    assert np.array_equal(tp, np.stack(np.meshgrid(*ax), axis=dim))
+    assert torch.equal(z.real, both[..., 0]) and torch.equal(z.imag, both[..., 1])
