@@ -82,6 +82,26 @@ cudaError_t gemm_c128_tc(int M, int N, int K, double alpha, const c128* A, long 
                          long long ldb, long long sB, double beta, const c128* C, long long ldc, long long sC, c128* D,
                          long long ldd, long long sD, int batch, cudaStream_t st,
                          const int* skip = nullptr);
+// Products of operands split into FP16 digits ahead of them (gemm_digits.cu),
+// batches of real (M x N x K) products; complex ones by their real views: A's
+// rows of (re, im), N and K doubled, B (K / 2 x N / 2) complex (`cplx`).
+// digit_rows / digit_cols write the leading `digits` (8, 6 or 4) of A and B
+// and the largest high words of their rows (batch, M) or columns (batch, N) to
+// `top`; with `round` (4 digits) B becomes what they hold.  digit_product:
+// D = (neg ? -1 : 1) A B + C from the digits t + u < max(da, db), for (da, db) =
+// (8, 8), (8, 4), (6, 6) or (4, 4), to 2^-60, 2^-60, 2^-47 and 2^-31 of the
+// largest product of a row's and a column's entries; NaN where a row of A or a
+// column of B holds an infinity or a NaN, zeros where all are below 2^-958.  C may alias D.  Leading dimensions and strides in doubles;
+// `skip` as above.
+size_t digit_rows_bytes(int M, int K, int digits);
+size_t digit_cols_bytes(int N, int K, int digits);
+cudaError_t digit_rows(int digits, int M, int K, const double* X, long long ldx, long long sX, int* top, void* out,
+                       int batch, const int* skip, cudaStream_t st);
+cudaError_t digit_cols(int digits, bool cplx, bool round, int N, int K, double* X, long long ldx, long long sX, int* top,
+                       void* out, int batch, const int* skip, cudaStream_t st);
+cudaError_t digit_product(int da, int db, int M, int N, int K, bool cplx, bool neg, const void* A, const int* ta,
+                          const void* B, const int* tb, const double* C, long long ldc, long long sC, double* D,
+                          long long ldd, long long sD, int batch, const int* skip, cudaStream_t st);
 // Device addresses of the tensor-core kernels' failure flag and wait limit.
 cudaError_t tc_wait_state(int** err, const long long** limit);
 int gemm_tc_error();

@@ -5,13 +5,19 @@
 //   R  = I - A X0,  X1 = X0 + X0 (R + R^2 + R^3)
 //   R  = I - A X1,  X  = X1 + X1 R                where the first R was not small
 //
-// The products with A and with X run on the digit kernel (gemm_f64_tc.cu,
-// FP64 and better), the powers of R, corrections of R, in single precision:
-// they leave an error of about |R|^2 2^-21, so a matrix whose R has row sums
-// of at most 5e-5 is done after the first step (leaves: 2e-6 per entry, row
-// sums 2e-5) and left out of the second; the others (interface and impedance
-// matrices, up to 1e-2) have |R| of at most 1e-8 there, and R^2 is left.  The
-// result carries the rounding of R (1e-16) and no elimination's growth.
+// The products with A and with X run on the digit kernels (gemm_f64_tc.cu,
+// FP64 and better, or gemm_digits.cu with the digits that a step needs), the
+// powers of R, corrections of R, in single precision: they leave an error of
+// about |R|^2 2^-21, so a matrix whose R has row sums of at most 5e-5 is done
+// after the first step (leaves: 2e-6 per entry, row sums 2e-5) and left out of
+// the second; the others (interface and impedance matrices, up to 1e-2) have
+// |R| of at most 1e-8 there, and R^2 is left.  The result carries the rounding
+// of R (1e-16) and no elimination's growth.
+// The digits each step needs: A always 8 (62 bits); X0 is rounded to 4 (32
+// bits, it has 24 good ones) and is from then on that matrix, so that its
+// residual is exact with 26 of the 36 digit products; X0 (R + R^2 + R^3) with 6
+// is good to 2^-47 |R|, below the single-precision powers; X1 keeps 8 in its
+// residual; X1 R with 4 is good to 2^-31 |R|, 5e-18.
 //
 // Why: elimination is a chain of n dependent pivots.  Its panels are bound by
 // the FP64 pipe (two multiply-adds per SM and clock) for many matrices and by
@@ -130,7 +136,33 @@ cudaError_t digits_gemm(int n, double alpha, const T* A, long long lda, long lon
 
 size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Matrices at a time: 4.5 FP64 copies of each, about 2 GB (one matrix always).
+// Whether the products run on operands split ahead of them (gemm_digits.cu)
+// with the digits each step needs, rather than on gemm_f64_tc.cu with all of
+// them: the passes that split cost some 20 us and 50 bytes a number, and pay
+// from products of about 1 GFLOP with rows of 192 numbers on.  Measured, the
+// two first products with their splits, whole against split: 432^3 x 3 120 and
+// 115 us, 224^3 x 16 75 and 100, 1000^3 244 and 170, 224^3 x 256 800 and 690,
+// complex 112^3 x 256 416 and 420, 512^3 x 64 1,620 and 1,080.
+template <class T>
+bool splits(int n, int batch) {
+  const double f = sizeof(T) == 16 ? 2.0 : 1.0;
+  return n * f >= 192.0 && 2.0 * n * (n * f) * (n * f) * batch >= 1e9;
+}
+
+// Bytes of the digits of one matrix: of A's rows (kept), of the second
+// operand's columns, and of the rows of X (four digits and six).
+struct DigitBytes {
+  size_t a, b, x;
+};
+template <class T>
+DigitBytes digit_bytes(int n) {
+  const int f = sizeof(T) == 16 ? 2 : 1;
+  return {digit_rows_bytes(n, n * f, 8), digit_cols_bytes(n * f, n * f, 8), digit_rows_bytes(n, n * f, 6)};
+}
+
+// Matrices at a time: about 2 GB of copies (one matrix always), and the digits
+// of as many; with half of it the single-precision panels of 157 complex
+// matrices of 256 were a third slower than those of 512.
 int chunk_of(size_t es, int n, int batch) {
   const size_t per = 4 * es * (size_t)n * n, most = (size_t)2 << 30;
   const size_t c = most / per;
@@ -160,6 +192,20 @@ cudaError_t run(int n, const T* A, long long lda, long long sA, T* X, long long 
   int* skip = (int*)take(sizeof(int) * (size_t)cap);
   const size_t lowb = inverse_workspace_bytes(low_dt, n, cap);
   void* lows = take(lowb);
+  constexpr bool CPLX = DTypeOf<T>::value == C128;
+  const int f = CPLX ? 2 : 1, nr = n * f;   // the real views: n x nr times nr x nr
+  const bool split = splits<T>(n, batch);
+  unsigned char *da = nullptr, *db = nullptr, *dx = nullptr;
+  int *ta = nullptr, *tb = nullptr, *tx = nullptr;
+  if (split) {
+    const DigitBytes d = digit_bytes<T>(n);
+    da = take(d.a * cap);
+    db = take(d.b * cap);
+    dx = take(d.x * cap);
+    ta = (int*)take(sizeof(int) * (size_t)n * cap);
+    tb = (int*)take(sizeof(int) * (size_t)nr * cap);
+    tx = (int*)take(sizeof(int) * (size_t)n * cap);
+  }
   if ((size_t)(w - base) > bytes) return cudaErrorInvalidValue;
   const L one_ = one<L>(), zero_ = zero<L>();
   const int gr = (n + RF_NT / 32 - 1) / (RF_NT / 32);   // CTAs for the rows of one matrix
@@ -181,8 +227,24 @@ cudaError_t run(int n, const T* A, long long lda, long long sA, T* X, long long 
                               INV_TENSOR_MEMORY | INV_BLOCK_RECURSIVE));
     note_launch();
     raise_kernel<T, L><<<gt, RF_NT, 0, st>>>(total, l0, P);
+    // D = X + X Y (contiguous X, Y) from the leading `digits` of both
+    auto correct = [&](int digits, T* Xp, T* Y, T* D, long long ldd, long long sD, const int* sk) {
+      RF_TRY(digit_rows(digits, n, nr, (const double*)Xp, nr, f * nn, tx, dx, nb, sk, st));
+      RF_TRY(digit_cols(digits, CPLX, false, nr, nr, (double*)Y, nr, f * nn, tb, db, nb, sk, st));
+      return digit_product(digits, digits, n, nr, nr, CPLX, false, dx, tx, db, tb, (const double*)Xp, nr, f * nn,
+                           (double*)D, f * ldd, f * sD, nb, sk, st);
+    };
+    // R = -A X
+    auto residual = [&](int digits, T* Xp, const int* sk) {
+      RF_TRY(digit_cols(digits, CPLX, digits == 4, nr, nr, (double*)Xp, nr, f * nn, tb, db, nb, sk, st));
+      return digit_product(8, digits, n, nr, nr, CPLX, true, da, ta, db, tb, nullptr, 0, 0, (double*)R, nr, f * nn, nb, sk,
+                           st);
+    };
+    if (split)
+      RF_TRY(digit_rows(8, n, nr, (const double*)Ab, f * lda, f * sA, ta, da, nb, nullptr, st));
     // first step: l0 = R, l1 = R + R^2, then l0 = R (R + R^2); P holds X0, Q gets X1
-    RF_TRY(digits_gemm<T>(n, -1.0, Ab, lda, sA, P, nn, nullptr, R, n, nn, nb, st, nullptr));
+    RF_TRY(split ? residual(4, P, nullptr)
+                 : digits_gemm<T>(n, -1.0, Ab, lda, sA, P, nn, nullptr, R, n, nn, nb, st, nullptr));
     note_launch();
     residual_kernel<T, L><<<dim3(gr, nb), RF_NT, 0, st>>>(n, R, l0, top, nullptr);
     note_launch();
@@ -191,13 +253,15 @@ cudaError_t run(int n, const T* A, long long lda, long long sA, T* X, long long 
     RF_TRY(gemm_batched<L>(n, n, n, one_, l0, n, nn, l1, n, nn, zero_, nullptr, 0, 0, l2, n, nn, nb, st));
     note_launch();
     add_powers_kernel<T, L><<<gt, RF_NT, 0, st>>>(total, R, l2);
-    RF_TRY(digits_gemm<T>(n, 1.0, P, n, nn, R, nn, P, Q, n, nn, nb, st, nullptr));
+    RF_TRY(split ? correct(6, P, R, Q, n, nn, nullptr)
+                 : digits_gemm<T>(n, 1.0, P, n, nn, R, nn, P, Q, n, nn, nb, st, nullptr));
     // second step, for the matrices that need it
     T* Xb = X + (long long)b0 * sX;
-    RF_TRY(digits_gemm<T>(n, -1.0, Ab, lda, sA, Q, nn, nullptr, R, n, nn, nb, st, skip));
+    RF_TRY(split ? residual(8, Q, skip) : digits_gemm<T>(n, -1.0, Ab, lda, sA, Q, nn, nullptr, R, n, nn, nb, st, skip));
     note_launch();
     residual_kernel<T, L><<<dim3(gr, nb), RF_NT, 0, st>>>(n, R, (L*)nullptr, top, skip);
-    RF_TRY(digits_gemm<T>(n, 1.0, Q, n, nn, R, nn, Q, Xb, ldx, sX, nb, st, skip));
+    RF_TRY(split ? correct(4, Q, R, Xb, ldx, sX, skip)
+                 : digits_gemm<T>(n, 1.0, Q, n, nn, R, nn, Q, Xb, ldx, sX, nb, st, skip));
     note_launch();
     keep_kernel<T><<<dim3(gx, nb), RF_NT, 0, st>>>(n, Q, Xb, ldx, sX, skip);
     note_launch();
@@ -213,10 +277,23 @@ bool inverse_refined_takes(int dtype, int n) {
   return (dtype == F64 || dtype == C128) && n > 64 && f64_products_on_tensor_cores();
 }
 
+template <class T>
+static size_t workspace_bytes(int n, int batch) {
+  const size_t es = sizeof(T), nn = (size_t)n * n;
+  const int cap = chunk_of(sizeof(T), n, batch), low_dt = es == 8 ? F32 : C64;
+  size_t s = 3 * al256(es * nn * cap) + 3 * al256(es / 2 * nn * cap) + 3 * al256(sizeof(int) * (size_t)cap) +
+             al256(inverse_workspace_bytes(low_dt, n, cap)) + 512;
+  if (splits<T>(n, batch)) {
+    const DigitBytes d = digit_bytes<T>(n);
+    const size_t nr = (size_t)n * (es / 8);
+    s += al256(d.a * cap) + al256(d.b * cap) + al256(d.x * cap) + 2 * al256(sizeof(int) * n * cap) +
+         al256(sizeof(int) * nr * cap);
+  }
+  return s;
+}
+
 size_t inverse_refined_workspace_bytes(int dtype, int n, int batch) {
-  const size_t es = dtype_size(dtype), nn = (size_t)n * n;
-  const int cap = chunk_of(es, n, batch), low_dt = dtype == F64 ? F32 : C64;
-  return 3 * al256(es * nn * cap) + 3 * al256(es / 2 * nn * cap) + 3 * al256(sizeof(int) * (size_t)cap) + al256(inverse_workspace_bytes(low_dt, n, cap)) + 512;
+  return dtype == F64 ? workspace_bytes<double>(n, batch) : workspace_bytes<c128>(n, batch);
 }
 
 template <class T>

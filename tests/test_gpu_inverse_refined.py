@@ -116,3 +116,26 @@ def test_status_words_of_the_c_entry(cuda, refined):
     assert info.tolist() == ([-2, 0, 0, 0] if refined else [0, 0, 0, 0])
     a.dtype |= 0x200                      # an unknown flag is an unknown type
     assert L.hps_local_solve_dtn(C.byref(a), nat.stream_ptr()) != 0
+
+
+@pytest.mark.parametrize("p,q,L,iti,d", [(16, 14, 4, False, 2), (17, 15, 4, False, 2), (12, 10, 1, False, 3),
+                                         (13, 11, 3, True, 2), (14, 12, 2, True, 2)])
+def test_products_of_split_operands(cuda, monkeypatch, p, q, L, iti, d):
+    """Stages whose inverses have their operands split ahead of the products
+    (rows of at least 192 numbers, 1 GFLOP a product): n = 196, 225, 1000 with a
+    merge of 1200, complex 169 and 196.  The bound is that of
+    test_stages_agree_with_the_elimination; a leaf with a NaN is handed back
+    and leaves the others alone."""
+    pde = _pde(p, q, L, 1.5, iti, d)
+    ref = _stages(pde, False, monkeypatch)
+    got = _stages(pde, True, monkeypatch)
+    for a, b in zip(got, ref):
+        assert float((a - b).abs().max()) <= 1e-11 * float(b.abs().max())
+    if iti or d == 3:
+        return
+    c = 1.5 * (1 + 0.2 * np.exp(-(pde.domain.interior_points ** 2).sum(-1)))
+    c[3, 4 * p - 4 + 40] = np.nan   # an interior point: the equation is not set at the boundary ones
+    Y = st.local_solve_stage_uniform_2D_DtN(_pde(p, q, L, c))[0]
+    assert bool(torch.isnan(Y[3]).any())
+    keep = [i for i in range(Y.shape[0]) if i != 3]
+    assert float((Y[keep] - ref[0][keep]).abs().max()) <= 1e-11 * float(ref[0].abs().max())
