@@ -374,6 +374,58 @@ static size_t merge_ws(const hps_merge_args* a, Carver* cv) {
   return cv->used + 256;
 }
 
+// The rectangles of C (c_form) or B as groups, one per exterior range with the
+// interface ranges as its segments: the products of a whole merge are then one
+// launch, each with its full K (3D: 72 products of one face each took 20 to 36
+// us apiece, bound by a single tile's latency, and read and wrote S and T_out
+// three times).  64 leaves of 8^2, whole build and solve: 3.2 -> 1.8 ms, 8 x 8
+// leaves of 10^3 27.8 -> 22.1 ms, no size found where the single products are
+// faster.  0 where the ranges are not the same or disjoint, or too many.
+static int rect_groups(const hps_merge_args* a, bool c_form, int other, GemmGroup* g) {
+  const int n = c_form ? a->n_c_rects : a->n_b_rects;
+  const int* r = c_form ? a->c_rects : a->b_rects;
+  int ng = 0;
+  for (int k = 0; k < n; ++k) {
+    const int* q = r + 5 * k;
+    const int i0 = c_form ? q[0] : q[2], li = c_form ? q[1] : q[3], e0 = c_form ? q[2] : q[0], le = c_form ? q[3] : q[1];
+    int j = 0;
+    for (; j < ng; ++j) {
+      const int f0 = c_form ? g[j].n0 : g[j].m0, lf = c_form ? g[j].n : g[j].m;
+      if (f0 == e0 && lf == le) break;
+      if (e0 < f0 + lf && f0 < e0 + le) return 0;
+    }
+    if (j == ng) {
+      if (ng == GEMM_GROUPS) return 0;
+      GemmGroup& x = g[ng++];
+      x.segs = 0;
+      (c_form ? x.n0 : x.m0) = e0;
+      (c_form ? x.n : x.m) = le;
+      (c_form ? x.m0 : x.n0) = 0;
+      (c_form ? x.m : x.n) = other;
+    }
+    GemmGroup& x = g[j];
+    // ranges side by side are one segment
+    if (x.segs > 0 && x.k0[x.segs - 1] + x.len[x.segs - 1] == i0) {
+      x.len[x.segs - 1] += li;
+      continue;
+    }
+    if (x.segs == GEMM_SEGS) return 0;
+    x.k0[x.segs] = i0;
+    x.len[x.segs++] = li;
+  }
+  return ng;
+}
+
+template <class T>
+static cudaError_t run_groups(const GemmGroup* g, int ng, double alpha, const T* A, long long lda, long long sA, const T* B,
+                              long long ldb, long long sB, bool add, T* D, long long ldd, long long sD, int batch,
+                              cudaStream_t st) {
+  if constexpr (DTypeOf<T>::value == F64 || DTypeOf<T>::value == C128)
+    return gemm_groups<T>(g, ng, alpha, A, lda, sA, B, ldb, sB, 1.0, add ? D : nullptr, ldd, sD, D, ldd, sD, batch, st);
+  else
+    return cudaErrorNotSupported;
+}
+
 template <class T>
 static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   const int nm = a->n_merges, ni = a->n_int, ne = a->n_ext, ns = a->nsrc;
@@ -433,8 +485,13 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   T* S = (T*)a->S;
   const long long sDD = (long long)ni * ni, sC = (long long)ni * ne, sB = (long long)ne * ni, sT = (long long)ne * ne;
   const bool rects = a->n_c_rects > 0 && a->n_b_rects > 0;
+  GemmGroup groups[GEMM_GROUPS];
+  const bool digits = (DTypeOf<T>::value == F64 || DTypeOf<T>::value == C128) && f64_products_on_tensor_cores();
   // S = -D^-1 C
-  if (rects) {
+  int ng = rects && digits ? rect_groups(a, true, ni, groups) : 0;
+  if (ng) {
+    HPS_CHECK(run_groups<T>(groups, ng, -1.0, D, ni, sDD, C, ne, sC, false, S, ne, sC, nm, st));
+  } else if (rects) {
     for (int r = 0; r < a->n_c_rects; ++r) {
       const int* q = a->c_rects + 5 * r;   // i0, n_i, e0, n_e, first
       HPS_CHECK(gemm_batched<T>(ni, q[3], q[1], mone, D + q[0], ni, sDD, C + (long long)q[0] * ne + q[2], ne, sC,
@@ -446,7 +503,10 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   // T_out = A + B S
   if (a->T_out) {
     T* To = (T*)a->T_out;
-    if (rects) {
+    ng = rects && digits ? rect_groups(a, false, ne, groups) : 0;
+    if (ng) {
+      HPS_CHECK(run_groups<T>(groups, ng, 1.0, B, ni, sB, S, ne, sC, true, To, ne, sT, nm, st));
+    } else if (rects) {
       for (int r = 0; r < a->n_b_rects; ++r) {
         const int* q = a->b_rects + 5 * r;   // e0, n_e, i0, n_i, first
         HPS_CHECK(gemm_batched<T>(q[1], ne, q[3], one_, B + (long long)q[0] * ni + q[2], ni, sB,
@@ -462,7 +522,12 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
     T* ho = (T*)a->h_out;
     const long long sg = (long long)ni * ns, sh = (long long)ne * ns;
     HPS_CHECK(gemm_batched<T>(ni, ns, ni, mone, D, ni, sDD, dh, ns, sg, zero_, nullptr, 0, 0, gt, ns, sg, nm, st));
-    if (rects) {
+    ng = rects && (ns <= 8 || digits) ? rect_groups(a, false, ns, groups) : 0;
+    if (ng && ns <= 8) {
+      HPS_CHECK(skinny_groups<T>(groups, ng, ne, ns, B, ni, sB, gt, ns, sg, ho, ns, sh, nm, st));
+    } else if (ng) {
+      HPS_CHECK(run_groups<T>(groups, ng, 1.0, B, ni, sB, gt, ns, sg, true, ho, ns, sh, nm, st));
+    } else if (rects) {
       for (int r = 0; r < a->n_b_rects; ++r) {
         const int* q = a->b_rects + 5 * r;
         HPS_CHECK(gemm_batched<T>(q[1], ns, q[3], one_, B + (long long)q[0] * ni + q[2], ni, sB,
@@ -476,7 +541,10 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   // B D^-1
   if (a->BD_inv) {
     T* BD = (T*)a->BD_inv;
-    if (rects) {
+    ng = rects && digits ? rect_groups(a, false, ni, groups) : 0;
+    if (ng) {
+      HPS_CHECK(run_groups<T>(groups, ng, 1.0, B, ni, sB, D, ni, sDD, false, BD, ni, sB, nm, st));
+    } else if (rects) {
       for (int r = 0; r < a->n_b_rects; ++r) {
         const int* q = a->b_rects + 5 * r;
         T* o = BD + (long long)q[0] * ni;

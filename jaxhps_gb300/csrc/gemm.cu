@@ -505,6 +505,91 @@ static cudaError_t launch_skinny(int M, int N, int K, T alpha, const T* A, long 
   return cudaGetLastError();
 }
 
+// D += A B with N <= 8 columns for the rows of every group, K running over the
+// group's segments: one launch for a merge's block rows, where a launch per
+// block (72 of 4 to 6 us in 3D) is bound by its latency.
+struct SkinnyGroups {
+  int n;
+  GemmGroup g[GEMM_GROUPS];
+};
+
+template <class T, int NB>
+__global__ void __launch_bounds__(SK_WARPS * 32)
+skinny_groups_kernel(const __grid_constant__ SkinnyGroups gs, int M, int N, const T* __restrict__ A, long long lda,
+                     long long sA, const T* __restrict__ B, long long ldb, long long sB, T* D, long long ldd,
+                     long long sD) {
+  const int lane = threadIdx.x & 31;
+  const int row = blockIdx.x * SK_WARPS + (threadIdx.x >> 5);
+  if (row >= M) return;  // uniform across the warp
+  int i = 0;
+  while (i < gs.n && !(row >= gs.g[i].m0 && row < gs.g[i].m0 + gs.g[i].m)) ++i;
+  if (i == gs.n) return;
+  const long long bz = blockIdx.y;
+  const T* a = A + bz * sA + (long long)row * lda;
+  T acc[NB];
+#pragma unroll
+  for (int n = 0; n < NB; ++n) acc[n] = zero<T>();
+  for (int s = 0; s < gs.g[i].segs; ++s) {
+    const int k1 = gs.g[i].k0[s] + gs.g[i].len[s];
+    for (int k = gs.g[i].k0[s] + lane; k < k1; k += 32) {
+      const T av = a[k];
+      const T* br = B + bz * sB + (long long)k * ldb;
+#pragma unroll
+      for (int n = 0; n < NB; ++n)
+        if (n < N) acc[n] = fma_(av, br[n], acc[n]);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < NB; ++n)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[n] = add(acc[n], shfl_xor_(acc[n], o));
+  if (lane < N) {
+    T v = acc[0];
+#pragma unroll
+    for (int n = 1; n < NB; ++n)
+      if (lane == n) v = acc[n];
+    T* d = D + bz * sD + (long long)row * ldd + lane;
+    *d = add(*d, v);
+  }
+}
+
+template <class T>
+cudaError_t skinny_groups(const GemmGroup* groups, int n, int M, int N, const T* A, long long lda, long long sA,
+                          const T* B, long long ldb, long long sB, T* D, long long ldd, long long sD, int batch,
+                          cudaStream_t st) {
+  if (n < 1 || n > GEMM_GROUPS || N < 1 || N > 8) return cudaErrorInvalidValue;
+  SkinnyGroups gs;
+  gs.n = n;
+  double flop = 0.0;
+  for (int i = 0; i < n; ++i) {
+    gs.g[i] = groups[i];
+    for (int s = 0; s < groups[i].segs; ++s) flop += 2.0 * groups[i].m * (double)groups[i].len[s] * N * batch;
+  }
+  ProfScope ps(KC_GEMM, st, flop * (DTypeOf<T>::value == C64 || DTypeOf<T>::value == C128 ? 4.0 : 1.0));
+  for (int b0 = 0; b0 < batch; b0 += 65535) {
+    const int nb = batch - b0 < 65535 ? batch - b0 : 65535;
+    auto go = [&](auto kernel) {
+      note_launch();
+      kernel<<<dim3((M + SK_WARPS - 1) / SK_WARPS, nb), SK_WARPS * 32, 0, st>>>(
+          gs, M, N, A + b0 * sA, lda, sA, B + b0 * sB, ldb, sB, D + b0 * sD, ldd, sD);
+    };
+    if (N == 1)
+      go(skinny_groups_kernel<T, 1>);
+    else if (N <= 2)
+      go(skinny_groups_kernel<T, 2>);
+    else
+      go(skinny_groups_kernel<T, 8>);
+  }
+  return cudaGetLastError();
+}
+#define HPS_SKINNY_GROUPS(T)                                                                                      \
+  template cudaError_t skinny_groups<T>(const GemmGroup*, int, int, int, const T*, long long, long long, const T*, \
+                                        long long, long long, T*, long long, long long, int, cudaStream_t);
+HPS_SKINNY_GROUPS(float)
+HPS_SKINNY_GROUPS(double)
+HPS_SKINNY_GROUPS(c64)
+HPS_SKINNY_GROUPS(c128)
+
 // Which products run on the tensor cores (gemm_tc.cu, gemm_f64_tc.cu): 0 none,
 // 1 the shapes where they were measured faster (default), 2 every product,
 // 3 none and the FP32 8x8 tiles with 4-byte shared loads (gemm_kernel) in

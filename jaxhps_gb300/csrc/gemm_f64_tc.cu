@@ -86,21 +86,47 @@ struct OzArgs {
   const long long* limit;
 };
 
+// Products of a batch whose operands are blocks of larger matrices (hps_internal.h),
+// with the first of the group's tiles.
+template <bool GROUP>
+struct OzGroups {
+  int n, tiles;
+  GemmGroup g[GEMM_GROUPS];
+  int t0[GEMM_GROUPS];
+};
+template <>
+struct OzGroups<false> {};
+
+// One tile: its matrix of the batch, its first row and column (inside the
+// group), and the group.
+struct OzTile {
+  long long b;
+  int m0, n0, g;
+};
+
 // One entry of D whose row of A or column of B holds an infinity or a NaN:
 // the multiply-add chain of gemm_kernel.
 template <bool CPLX>
-__device__ __noinline__ double plain_entry(const OzArgs& p, const double* A, const double* B, int m, int n) {
-  const double* a = A + (long long)m * p.lda;
+__device__ __noinline__ double plain_entry(const OzArgs& p, const double* A, const double* B, int m, int n,
+                                           const GemmGroup* g) {
+  const int segs = g ? g->segs : 1;
+  const double* a0 = A + (long long)m * p.lda;
   if constexpr (CPLX) {
-    const c128* ac = reinterpret_cast<const c128*>(a);
     c128 s = zero<c128>();
-    for (int k = 0; k < p.K / 2; ++k)
-      s = fma_(ac[k], *reinterpret_cast<const c128*>(B + k * p.ldb + (n & ~1)), s);
+    for (int i = 0; i < segs; ++i) {
+      const int k0 = g ? g->k0[i] : 0, K = g ? g->len[i] : p.K / 2;
+      const c128* a = reinterpret_cast<const c128*>(a0) + k0;
+      for (int k = 0; k < K; ++k)
+        s = fma_(a[k], *reinterpret_cast<const c128*>(B + (long long)(k0 + k) * p.ldb + (n & ~1)), s);
+    }
     s = mul(c128{p.alpha, 0.0}, s);
     return (n & 1) ? s.y : s.x;
   } else {
     double s = 0.0;
-    for (int k = 0; k < p.K; ++k) s = fma(a[k], B[k * p.ldb + n], s);
+    for (int i = 0; i < segs; ++i) {
+      const int k0 = g ? g->k0[i] : 0, K = g ? g->len[i] : p.K;
+      for (int k = 0; k < K; ++k) s = fma(a0[k0 + k], B[(long long)(k0 + k) * p.ldb + n], s);
+    }
     return p.alpha * s;
   }
 }
@@ -125,8 +151,10 @@ __device__ __noinline__ double plain_entry(const OzArgs& p, const double* A, con
 // Every wait is bounded: after one that runs out a warp goes through its loop
 // without waiting (so that the named barrier is met by all) and the CTA frees
 // its tensor memory.
-template <int BN, bool CPLX, bool SKIP>
-__global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
+// GROUP: the products of all groups at once, K running through a group's
+// segments one after another (each one's last stage filled up with zeros).
+template <int BN, bool CPLX, bool SKIP, bool GROUP>
+__global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const __grid_constant__ OzGroups<GROUP> gs) {
   using Cfg = OzCfg<BN>;
   constexpr int NS = Cfg::NS, NR = Cfg::NR, CW = Cfg::CW, KB = Cfg::KB;
   extern __shared__ unsigned char oz_raw[];
@@ -164,9 +192,55 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tmem_s;
+  constexpr int F = CPLX ? 2 : 1;
   const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + OZ_BM - 1) / OZ_BM;
-  const long long per_b = (long long)tiles_m * tiles_n, n_units = per_b * p.batch;
-  const int nk = (p.K + OZ_BK - 1) / OZ_BK;
+  const int per_b = [&] {
+    if constexpr (GROUP) return gs.tiles;
+    else return tiles_m * tiles_n;
+  }();
+  const long long n_units = (long long)per_b * p.batch;
+  auto tile_of = [&](long long u) {
+    OzTile t;
+    t.b = u / per_b;
+    const int r = (int)(u - t.b * per_b);
+    if constexpr (GROUP) {
+      int g = 0;
+      while (g + 1 < gs.n && r >= gs.t0[g + 1]) ++g;
+      const int tn = (F * gs.g[g].n + BN - 1) / BN, i = r - gs.t0[g];
+      t.g = g, t.m0 = (i / tn) * OZ_BM, t.n0 = (i % tn) * BN;
+    } else {
+      t.g = 0, t.m0 = (r / tiles_n) * OZ_BM, t.n0 = (r % tiles_n) * BN;
+    }
+    return t;
+  };
+  const int nk_all = (p.K + OZ_BK - 1) / OZ_BK;
+  auto stages_of = [&](long long u) {
+    if constexpr (GROUP) {
+      const GemmGroup& g = gs.g[tile_of(u).g];
+      int k = 0;
+      for (int i = 0; i < g.segs; ++i) k += (F * g.len[i] + OZ_BK - 1) / OZ_BK;
+      return k;
+    } else {
+      return nk_all;
+    }
+  };
+  // sizes of a tile's product (real), and where its blocks begin (in doubles)
+  auto rows_of = [&](const OzTile& t) {
+    if constexpr (GROUP) return gs.g[t.g].m;
+    else return p.M;
+  };
+  auto cols_of = [&](const OzTile& t) {
+    if constexpr (GROUP) return F * gs.g[t.g].n;
+    else return p.N;
+  };
+  auto row0_of = [&](const OzTile& t) {
+    if constexpr (GROUP) return gs.g[t.g].m0;
+    else return 0;
+  };
+  auto col0_of = [&](const OzTile& t) {
+    if constexpr (GROUP) return F * gs.g[t.g].n0;
+    else return 0;
+  };
   // the first of the CTA's tiles u, u + gridDim.x, ... that is not left out
   auto tile_from = [&](long long u) {
     if constexpr (SKIP)
@@ -187,6 +261,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
     uint32_t s0[CW], s1[CW], s2[CW];
     uint32_t ch = 0, tile = 0;
     for (long long u = u0; u < n_units; u = tile_from(u + gridDim.x), ++tile) {
+      const int nk = stages_of(u);
 #pragma unroll
       for (int j = 0; j < CW; ++j) s0[j] = s1[j] = s2[j] = 0;
       for (int kt = 0; kt < nk; kt += OZ_CHUNK, ++ch) {
@@ -226,17 +301,17 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
       }
       const int eb = tile % OZ_EB;
       wait(&expo[eb], (tile / OZ_EB) & 1);
-      const long long b = u / per_b;
-      const int r = (int)(u % per_b), m0 = (r / tiles_n) * OZ_BM, n0 = (r % tiles_n) * BN;
-      const int row = m0 + q * 32 + lane, c0 = n0 + cg * CW;
-      if (!ok || row >= p.M || c0 >= p.N) continue;
-      const int re = row_e[eb][q * 32 + lane];
-      const double* Cr = p.C ? p.C + b * p.sC + (long long)row * p.ldc + c0 : nullptr;
-      double* Dr = p.D + b * p.sD + (long long)row * p.ldd + c0;
+      const OzTile t = tile_of(u);
+      const long long b = t.b;
+      const int row = t.m0 + q * 32 + lane, c0 = t.n0 + cg * CW, N = cols_of(t);
+      if (!ok || row >= rows_of(t) || c0 >= N) continue;
+      const int re = row_e[eb][q * 32 + lane], r0 = row0_of(t) + row, n0 = col0_of(t) + c0;   // in the matrices
+      const double* Cr = p.C ? p.C + b * p.sC + (long long)r0 * p.ldc + n0 : nullptr;
+      double* Dr = p.D + b * p.sD + (long long)r0 * p.ldd + n0;
       const bool neg = p.alpha == -1.0;
 #pragma unroll
       for (int g = 0; g < CW; g += 4) {
-        if (c0 + g >= p.N) break;
+        if (c0 + g >= N) break;
         double v[4];
         bool odd = re >= 0x7ff;
 #pragma unroll
@@ -260,13 +335,16 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            if ((plain[j] || (CPLX && plain[j ^ 1])) && c0 + g + j < p.N)
-              v[j] = plain_entry<CPLX>(p, p.A + b * p.sA, p.B + b * p.sB, row, c0 + g + j);
+            if ((plain[j] || (CPLX && plain[j ^ 1])) && c0 + g + j < N) {
+              const GemmGroup* gp = nullptr;
+              if constexpr (GROUP) gp = &gs.g[t.g];
+              v[j] = plain_entry<CPLX>(p, p.A + b * p.sA, p.B + b * p.sB, r0, n0 + g + j, gp);
+            }
         } else if (neg) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) v[j] = -v[j];
         }
-        if (c0 + g + 4 <= p.N && p.vec_d) {
+        if (c0 + g + 4 <= N && p.vec_d) {
           if (Cr) {
             const double2 x = *reinterpret_cast<const double2*>(Cr + g), y = *reinterpret_cast<const double2*>(Cr + g + 2);
             v[0] = fma(p.beta, x.x, v[0]);
@@ -279,7 +357,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
         } else {
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            if (c0 + g + j < p.N) Dr[g + j] = Cr ? fma(p.beta, Cr[g + j], v[j]) : v[j];
+            if (c0 + g + j < N) Dr[g + j] = Cr ? fma(p.beta, Cr[g + j], v[j]) : v[j];
         }
       }
     }
@@ -297,28 +375,38 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
     const uint32_t raw_s = smem_u32(raw);
     const int rr = ar & 15;
 
-    // the stage that is copied next: a tile's nk stages twice
+    // the stage that is copied next: a tile's stages twice
     long long lu = u0;
-    int lkt = 0, lslot = 0;
+    int lslot = 0, lpass = 0, lseg = 0, lk = 0, lseg_len = 0;   // step inside the segment (all of K without groups)
+    auto seg_len = [&] {
+      if constexpr (GROUP) return lseg_len;
+      else return p.K;
+    };
     const double *lA = nullptr, *lB = nullptr;   // this lane's first piece of A, the thread's column of B, at the stage's first step
     int lrows = 0;                              // rows of this warp inside A
     bool lb_in = false;
     const int pr = p.vec_a ? lane >> 3 : lane >> 4, pc = p.vec_a ? lane & 7 : lane & 15;   // row and piece of a copy
-    auto tile_ptrs = [&]() {
-      const long long b = lu / per_b;
-      const int r = (int)(lu % per_b), m = (r / tiles_n) * OZ_BM + 16 * cw, n = (r % tiles_n) * BN + bn;
-      lrows = p.M - m - pr;
-      lA = p.A + b * p.sA + (long long)(m + pr) * p.lda + (p.vec_a ? 2 * pc : pc);
-      lb_in = n < p.N;
-      lB = p.B + b * p.sB + (CPLX ? (long long)(bk >> 1) * p.ldb + (n & ~1) : (long long)bk * p.ldb + n);
+    auto segment_ptrs = [&]() {
+      const OzTile t = tile_of(lu);
+      const int m = t.m0 + 16 * cw + pr, n = t.n0 + bn;
+      lrows = rows_of(t) - m;
+      lA = p.A + t.b * p.sA + (long long)(row0_of(t) + m) * p.lda + (p.vec_a ? 2 * pc : pc);
+      lb_in = n < cols_of(t);
+      lB = p.B + t.b * p.sB + (CPLX ? (long long)(bk >> 1) * p.ldb + (n & ~1) : (long long)bk * p.ldb + n) + col0_of(t);
+      lk = 0;
+      if constexpr (GROUP) {
+        lseg_len = F * gs.g[t.g].len[lseg];
+        lA += F * gs.g[t.g].k0[lseg];
+        lB += (long long)gs.g[t.g].k0[lseg] * p.ldb;
+      }
     };
-    if (lu < n_units) tile_ptrs();
+    if (lu < n_units) segment_ptrs();
     const double* safe = p.A;   // an address for copies that read nothing
     auto copy_stage = [&]() {
       if (lu < n_units) {
         const uint32_t dst = raw_s + lslot * Cfg::RAW;
-        const int k0 = (lkt < nk ? lkt : lkt - nk) * OZ_BK;
-        const bool whole = k0 + OZ_BK <= p.K;
+        const int k0 = lk, lK = seg_len();
+        const bool whole = k0 + OZ_BK <= lK;
         if (p.vec_a) {
           const uint32_t d = dst + pr * 128;
           if (whole) {
@@ -327,7 +415,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
               cp_async16(d + i * 512 + ((pc ^ pr ^ (4 * (i & 1))) << 4), 4 * i < lrows ? lA + (long long)(4 * i) * p.lda : safe,
                          4 * i < lrows);
           } else {
-            const int left = p.K - k0 - 2 * pc;   // values of this piece inside the row
+            const int left = lK - k0 - 2 * pc;   // values of this piece inside the row
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const uint32_t x = d + i * 512 + ((pc ^ pr ^ (4 * (i & 1))) << 4);
@@ -338,7 +426,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
             }
           }
         } else {
-          const bool kin = k0 + pc < p.K;
+          const bool kin = k0 + pc < lK;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const bool in = kin && 2 * i < lrows;
@@ -346,7 +434,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
                       in ? lA + (long long)(2 * i) * p.lda : safe, in);
           }
         }
-        const int left = lb_in ? p.K - k0 - bk : 0;
+        const int left = lb_in ? lK - k0 - bk : 0;
 #pragma unroll
         for (int i = 0; i < KB; ++i) {
           const double* src = CPLX ? lB + (long long)(KB > 1 ? i >> 1 : 0) * p.ldb + ((bk + i + bn) & 1) : lB + (long long)i * p.ldb;
@@ -355,12 +443,18 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
         lslot = lslot + 1 == NR ? 0 : lslot + 1;
         lA += OZ_BK;
         lB += (long long)(CPLX ? OZ_BK / 2 : OZ_BK) * p.ldb;
-        ++lkt;
-        if (lkt == nk) tile_ptrs();
-        if (lkt == 2 * nk) {
-          lkt = 0;
-          lu = tile_from(lu + gridDim.x);
-          if (lu < n_units) tile_ptrs();
+        lk += OZ_BK;
+        if (lk >= seg_len()) {
+          bool end = true;
+          if constexpr (GROUP) {
+            end = ++lseg == gs.g[tile_of(lu).g].segs;
+            if (end) lseg = 0;
+          }
+          if (end && ++lpass == 2) {
+            lpass = 0;
+            lu = tile_from(lu + gridDim.x);
+          }
+          if (lu < n_units) segment_ptrs();
         }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
@@ -385,6 +479,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
 
     uint32_t it = 0, tile = 0;
     for (long long u = u0; u < n_units; u = tile_from(u + gridDim.x), ++tile) {
+      const int nk = stages_of(u);
       uint32_t ae, be;
       {
         uint32_t at = 0, al = 0, bt = 0, bl = 0;
@@ -511,6 +606,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
       uint32_t it = 0, ch = 0;
       int s = 0;
       for (long long u = u0; u < n_units; u = tile_from(u + gridDim.x)) {
+        const int nk = stages_of(u);
         for (int kt = 0; kt < nk; ++kt, ++it) {
           const bool first = kt % OZ_CHUNK == 0, last = kt % OZ_CHUNK == OZ_CHUNK - 1 || kt == nk - 1;
           wait(&full[s], (it / NS) & 1);
@@ -564,19 +660,20 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p) {
   }
 }
 
-template <int BN, bool CPLX, bool SKIP>
-cudaError_t launch_oz(OzArgs p, cudaStream_t st) {
+template <int BN, bool CPLX, bool SKIP, bool GROUP = false>
+cudaError_t launch_oz(OzArgs p, cudaStream_t st, const OzGroups<GROUP>& gs = {}) {
   using Cfg = OzCfg<BN>;
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(gemm_oz_kernel<BN, CPLX, SKIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+    e = cudaFuncSetAttribute(gemm_oz_kernel<BN, CPLX, SKIP, GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
   if (e == cudaSuccess) e = tc_wait_state(&p.err, &p.limit);
   if (e != cudaSuccess) return e;
-  const long long units = (long long)p.batch * ((p.M + OZ_BM - 1) / OZ_BM) * ((p.N + BN - 1) / BN);
+  long long units = (long long)p.batch * ((p.M + OZ_BM - 1) / OZ_BM) * ((p.N + BN - 1) / BN);
+  if constexpr (GROUP) units = (long long)p.batch * gs.tiles;
   note_launch();
-  gemm_oz_kernel<BN, CPLX, SKIP><<<(unsigned)(units < sms ? units : sms), OZ_NT, Cfg::SMEM, st>>>(p);
+  gemm_oz_kernel<BN, CPLX, SKIP, GROUP><<<(unsigned)(units < sms ? units : sms), OZ_NT, Cfg::SMEM, st>>>(p, gs);
   return cudaGetLastError();
 }
 
@@ -596,6 +693,45 @@ static cudaError_t gemm_oz(int M, int N, int K, double alpha, const double* A, l
   if (N <= 16) return launch_oz<16, CPLX, false>(p, st);
   return launch_oz<64, CPLX, false>(p, st);
 }
+
+template <class T>
+cudaError_t gemm_groups(const GemmGroup* groups, int n, double alpha, const T* A, long long lda, long long sA, const T* B,
+                        long long ldb, long long sB, double beta, const T* C, long long ldc, long long sC, T* D,
+                        long long ldd, long long sD, int batch, cudaStream_t st) {
+  constexpr bool CPLX = DTypeOf<T>::value == C128;
+  constexpr int F = CPLX ? 2 : 1;
+  if (n < 1 || n > GEMM_GROUPS) return cudaErrorInvalidValue;
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  OzArgs p{0, 0, 0, alpha, beta, (const double*)A, F * lda, F * sA, (const double*)B, F * ldb, F * sB, (const double*)C,
+           F * ldc, F * sC, (double*)D, F * ldd, F * sD, batch, 0, 0, nullptr, nullptr, nullptr};
+  OzGroups<true> gs;
+  gs.n = n;
+  gs.tiles = 0;
+  bool even_k = true, even_n = true;
+  double flop = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const GemmGroup& g = gs.g[i] = groups[i];
+    gs.t0[i] = gs.tiles;
+    gs.tiles += ((g.m + OZ_BM - 1) / OZ_BM) * ((F * g.n + 63) / 64);
+    even_n = even_n && F * g.n0 % 2 == 0;
+    for (int k = 0; k < g.segs; ++k) {
+      even_k = even_k && F * g.k0[k] % 2 == 0;
+      flop += 2.0 * F * F * g.m * (double)g.n * g.len[k] * batch;
+    }
+  }
+  p.vec_a = even_k && al16(A) && p.lda % 2 == 0 && (batch == 1 || p.sA % 2 == 0);
+  p.vec_d = even_n && al16(D) && p.ldd % 2 == 0 && (batch == 1 || p.sD % 2 == 0) &&
+            (!C || (al16(C) && p.ldc % 2 == 0 && (batch == 1 || p.sC % 2 == 0)));
+  ProfScope ps(KC_GEMM, st, flop);
+  return launch_oz<64, CPLX, false, true>(p, st, gs);
+}
+
+template cudaError_t gemm_groups<double>(const GemmGroup*, int, double, const double*, long long, long long,
+                                         const double*, long long, long long, double, const double*, long long, long long,
+                                         double*, long long, long long, int, cudaStream_t);
+template cudaError_t gemm_groups<c128>(const GemmGroup*, int, double, const c128*, long long, long long, const c128*,
+                                       long long, long long, double, const c128*, long long, long long, c128*, long long,
+                                       long long, int, cudaStream_t);
 
 cudaError_t gemm_f64_tc(int M, int N, int K, double alpha, const double* A, long long lda, long long sA,
                         const double* B, long long ldb, long long sB, double beta, const double* C, long long ldc,

@@ -82,6 +82,25 @@ cudaError_t gemm_c128_tc(int M, int N, int K, double alpha, const c128* A, long 
                          long long ldb, long long sB, double beta, const c128* C, long long ldc, long long sC, c128* D,
                          long long ldd, long long sD, int batch, cudaStream_t st,
                          const int* skip = nullptr);
+// Products of blocks of the same matrices in one launch of the digit kernel
+// (gemm_f64_tc.cu): for every group, rows m0 .. m0 + m - 1 and columns n0 ..
+// n0 + n - 1 of D = alpha A B + beta C with K running over the columns of A and
+// rows of B of its segments.  T = double or c128.  The groups' blocks of D do
+// not overlap; D may alias C only.
+constexpr int GEMM_GROUPS = 32, GEMM_SEGS = 4;
+struct GemmGroup {
+  int m0, m, n0, n, segs, k0[GEMM_SEGS], len[GEMM_SEGS];
+};
+template <class T>
+cudaError_t gemm_groups(const GemmGroup* groups, int n, double alpha, const T* A, long long lda, long long sA, const T* B,
+                        long long ldb, long long sB, double beta, const T* C, long long ldc, long long sC, T* D,
+                        long long ldd, long long sD, int batch, cudaStream_t st);
+// D += A B for the rows of the groups (their n0 and n are not used) and N <= 8
+// columns, any type (gemm.cu); M rows in all.
+template <class T>
+cudaError_t skinny_groups(const GemmGroup* groups, int n, int M, int N, const T* A, long long lda, long long sA,
+                          const T* B, long long ldb, long long sB, T* D, long long ldd, long long sD, int batch,
+                          cudaStream_t st);
 // Products of operands split into FP16 digits ahead of them (gemm_digits.cu),
 // batches of real (M x N x K) products; complex ones by their real views: A's
 // rows of (re, im), N and K doubled, B (K / 2 x N / 2) complex (`cplx`).
