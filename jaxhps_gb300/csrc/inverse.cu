@@ -1090,6 +1090,166 @@ gje_panel_cluster_kernel(int n, int k0, int bw, int rows_per, T* Mat, T* U, T* G
   for (int i = tid; i < nr; i += CP_NT) us[r0 + i] = (ul[i] == 2) ? 1 : ul[i];
 }
 
+// The same panel with a row per thread, in registers: n <= pr_rows<T>(), one
+// CTA per matrix.  A column's step shifts the row by one register, x[j - 1] from
+// x[j], so that the pivot column is always x[0] and the loop body is the same
+// for all columns.  Every warp offers its best row (its magnitude and its 32
+// values) before the column's only barrier; each warp then finds the winner
+// among the offers and scales it for itself.
+//
+// gje_panel_kernel keeps the panel in shared memory and moves every number
+// through it twice a column, and its copies in and out of the panel meet 32-way
+// bank conflicts: 4096 complex64 panels of 256 x 32 took 2,120 us (795 here),
+// where the panel's own traffic takes 190; clusters of 16 CTAs (64 matrices of
+// 224) 118 us a panel (41 here), 3.7 a column, most of it their barriers.  What
+// is left is latency: two CTAs an SM (128 registers a thread) issue in 44% of
+// the cycles, waiting for the argument of the maximum, the reciprocal and the
+// barrier of each column, and for the copies in and out.
+// Rows: up to 512 threads with at most 128 registers each, 256 where a number
+// is FP64 (64 and 128 registers a row, and as many in its updates).
+template <class T>
+constexpr int pr_rows() { return sizeof(typename MagOf<T>::type) == 8 ? 256 : 512; }
+template <class T>
+constexpr int pr_chunk() { return 128 / (int)sizeof(T); }            // columns of a copied tile: 128 bytes a row
+template <class T>
+constexpr size_t pr_tile() { return 32 * (pr_chunk<T>() + 1) * sizeof(T); }
+
+// Magnitudes as integers of the same order, 0 for rows that are pivots already.
+__device__ __forceinline__ uint32_t pr_key(float m, bool used) { return used ? 0u : __float_as_uint(m) + 1u; }
+__device__ __forceinline__ unsigned long long pr_key(double m, bool used) {
+  return used ? 0ull : (unsigned long long)__double_as_longlong(m) + 1ull;
+}
+// The first lane with the largest key.
+__device__ __forceinline__ int pr_best(uint32_t& key) {
+  const uint32_t m = __reduce_max_sync(0xffffffffu, key);
+  const int l = __ffs(__ballot_sync(0xffffffffu, key == m)) - 1;
+  key = m;
+  return l;
+}
+__device__ __forceinline__ int pr_best(unsigned long long& key) {
+  const uint32_t hi = (uint32_t)(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const uint32_t lo = hi == mh ? (uint32_t)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
+  const int l = __ffs(__ballot_sync(0xffffffffu, hi == mh && lo == ml)) - 1;
+  key = ((unsigned long long)mh << 32) | ml;
+  return l;
+}
+
+template <class T>
+__global__ void __launch_bounds__(pr_rows<T>())
+gje_panel_reg_kernel(int n, int k0, int bw, T* Mat, T* U, T* G, T* E, int* piv, unsigned char* used, int* info) {
+  using MagT = typename MagOf<T>::type;
+  using Key = decltype(pr_key(MagT(), false));
+  constexpr int W = pr_rows<T>() / 32, CH = pr_chunk<T>();
+  const long long b = blockIdx.x, nn = (long long)n * n;
+  T* M = Mat + b * nn;
+  T* Ub = U + b * (long long)n * BP;
+  extern __shared__ __align__(16) unsigned char pr_raw[];
+  __shared__ __align__(16) T offer[2][W][BP];
+  __shared__ __align__(16) T scaled[W][BP];
+  __shared__ Key offer_key[2][W];
+  __shared__ int offer_row[2][W], Rs[BP];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  T* tile = reinterpret_cast<T*>(pr_raw + warp * pr_tile<T>());
+
+  T x[BP];
+#pragma unroll
+  for (int c0 = 0; c0 < BP; c0 += CH) {
+#pragma unroll
+    for (int e = lane; e < 32 * CH; e += 32) {
+      const int i = warp * 32 + e / CH, c = c0 + e % CH;
+      tile[(e / CH) * (CH + 1) + e % CH] = i < n && c < bw ? M[(long long)i * n + k0 + c] : zero<T>();
+    }
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < CH; ++c) x[c0 + c] = tile[lane * (CH + 1) + c];
+    __syncwarp();
+  }
+  bool taken = tid >= n || used[b * n + tid] != 0;
+  int mine = -1;   // the column this row is the pivot of
+
+  auto propose = [&](int buf) {
+    Key key = pr_key(nan_to_inf(pivmag(x[0])), taken);
+    const int l = pr_best(key);
+    if (lane == l) {
+#pragma unroll
+      for (int j = 0; j < BP; ++j) offer[buf][warp][j] = x[j];
+      offer_key[buf][warp] = key;
+      offer_row[buf][warp] = tid;
+    }
+  };
+  propose(0);
+  __syncthreads();
+  for (int c = 0; c < bw; ++c) {
+    const int buf = c & 1;
+    Key key = lane < nw ? offer_key[buf][lane] : 0;
+    const int w = pr_best(key);
+    const int r = offer_row[buf][w];
+    const bool any = key > 1;   // a magnitude above zero
+    const T raw = offer[buf][w][lane];
+    const T pinv = any ? rcp_(offer[buf][w][0]) : zero<T>();
+    scaled[warp][lane] = mul(raw, pinv);
+    __syncwarp();
+    if (tid == 0) {
+      piv[b * n + k0 + c] = r;
+      Rs[c] = r;
+      if (!any && info && info[b] == 0) info[b] = k0 + c + 1;
+    }
+    const T f = x[0];
+    if (tid == r) {
+#pragma unroll
+      for (int j = 1; j < BP; ++j) x[j - 1] = scaled[warp][j];
+      x[BP - 1] = pinv;
+      taken = true;
+      mine = c;
+    } else {
+#pragma unroll
+      for (int j = 1; j < BP; ++j) x[j - 1] = fms_(f, scaled[warp][j], x[j]);
+      x[BP - 1] = neg(mul(f, pinv));
+    }
+    __syncwarp();
+    if (c + 1 < bw) propose(buf ^ 1);
+    __syncthreads();
+  }
+  for (int c = bw; c < BP; ++c) {   // a narrower panel: back to its columns' places
+    const T f = x[0];
+#pragma unroll
+    for (int j = 1; j < BP; ++j) x[j - 1] = x[j];
+    x[BP - 1] = f;
+  }
+
+  // outputs as gje_panel_kernel's
+  if (mine >= 0) {
+    T* Eb = E + b * (long long)BP * BP + mine * BP;
+#pragma unroll
+    for (int c = 0; c < BP; ++c)
+      if (c < bw) Eb[c] = x[c];
+    used[b * n + tid] = 1;
+  }
+  const uint32_t pivots = __ballot_sync(0xffffffffu, mine >= 0);
+#pragma unroll
+  for (int c0 = 0; c0 < BP; c0 += CH) {
+#pragma unroll
+    for (int c = 0; c < CH; ++c) tile[lane * (CH + 1) + c] = x[c0 + c];
+    __syncwarp();
+#pragma unroll 4
+    for (int e = lane; e < 32 * CH; e += 32) {
+      const int i = warp * 32 + e / CH, c = c0 + e % CH;
+      if (i < n && c < bw) {
+        const T v = tile[(e / CH) * (CH + 1) + e % CH];
+        M[(long long)i * n + k0 + c] = v;
+        Ub[(long long)i * BP + c] = (pivots >> (e / CH)) & 1u ? zero<T>() : v;
+      }
+    }
+    __syncwarp();
+  }
+  T* Gb = G + b * (long long)BP * n;
+  for (int c = warp; c < bw; c += nw) {
+    const T* row = M + (long long)Rs[c] * n;
+#pragma unroll 8
+    for (int j = lane; j < n; j += 32) Gb[(long long)c * n + j] = j >= k0 && j < k0 + bw ? zero<T>() : row[j];
+  }
+}
+
 template <class T>
 __global__ void gje_scatter_rows_kernel(int n, int k0, int bw, T* Mat, const T* H, const int* piv) {
   const long long b = blockIdx.y;
@@ -1694,7 +1854,7 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&coop_ok, cudaDevAttrCooperativeLaunch, dev);
-    if (coop_ok && sms > 0 && batch < sms && n > 64) {
+    if (n > pr_rows<T>() && coop_ok && sms > 0 && batch < sms && n > 64) {
       nct = 2 * sms / batch;
       if (nct > coop_nct_cap(n)) nct = coop_nct_cap(n);
       bool fits = false;
@@ -1778,7 +1938,14 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
   int bwmax = BP;
   int use_smem = 0;
   size_t pan_smem = 0;
-  if (nct == 0) {
+  // Up to a row per thread the panel stays in registers.
+  const bool reg = n <= pr_rows<T>();
+  const size_t reg_smem = (size_t)((n + 31) / 32) * pr_tile<T>();
+  if (reg) {
+    const cudaError_t e = cudaFuncSetAttribute(gje_panel_reg_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(pr_rows<T>() / 32 * pr_tile<T>()));
+    if (e != cudaSuccess) return e;
+  } else if (nct == 0) {
     while (bwmax > 4 && es * (size_t)n * bwmax > 200 * 1024) bwmax /= 2;
     pan_smem = es * (size_t)n * bwmax;
     use_smem = pan_smem <= 200 * 1024;
@@ -1820,6 +1987,9 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
         e = cudaLaunchCooperativeKernel((void*)gje_panel_coop_kernel<T>, dim3(nct, batch), dim3(CP_NT), args,
                                         csmem, st);
       }
+    } else if (reg) {
+      gje_panel_reg_kernel<T><<<batch, ((n + 31) / 32) * 32, reg_smem, st>>>(n, k0, bw, Mat, U, G, E, piv, used, info);
+      e = cudaGetLastError();
     } else {
       const int pnt = n >= PANEL_NT ? PANEL_NT : ((n + 31) / 32) * 32;
       gje_panel_kernel<T><<<batch, pnt, use_smem ? pan_smem : 0, st>>>(n, k0, bw, Mat, Pw, use_smem, U, G, E, piv,

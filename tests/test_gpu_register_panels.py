@@ -1,0 +1,54 @@
+"""The panel of the blocked Gauss-Jordan inverse with a row per thread
+(gje_panel_reg_kernel in csrc/inverse.cu): every type at the smallest and the
+largest n it takes, narrow last panels, partial warps, few and many matrices."""
+
+import numpy as np
+import pytest
+import torch
+
+from jaxhps_gb300 import _native as nat
+
+pytestmark = pytest.mark.gpu
+
+TYPES = {"f32": (torch.float32, np.float32), "f64": (torch.float64, np.float64),
+         "c64": (torch.complex64, np.complex64), "c128": (torch.complex128, np.complex128)}
+
+
+@pytest.mark.parametrize("kind,n,batch", [
+    ("f32", 225, 3), ("f32", 256, 160), ("f32", 481, 1), ("f32", 512, 5), ("f32", 513, 2), ("f64", 65, 2), ("f64", 129, 200),
+    ("f64", 255, 1), ("f64", 256, 7), ("f64", 257, 2), ("c64", 129, 1), ("c64", 256, 170), ("c64", 301, 2), ("c64", 512, 3),
+    ("c64", 513, 1), ("c128", 65, 1), ("c128", 112, 160), ("c128", 256, 3), ("c128", 258, 1)])
+def test_inverse_with_register_panels(cuda, kind, n, batch):
+    """|A X - I| <= 16 n eps |A| |X| in the row-sum norm: the elimination's own
+    bound with a growth of 16, for diagonally dominant matrices with their rows
+    permuted, so that every pivot has to be looked for."""
+    dt, npdt = TYPES[kind]
+    rng = np.random.default_rng(n + batch)
+    A = rng.standard_normal((batch, n, n))
+    if kind[0] == "c":
+        A = A + 1j * rng.standard_normal(A.shape)
+    A = A + 2 * np.sqrt(n) * np.eye(n)
+    A = np.ascontiguousarray(A[:, rng.permutation(n)]).astype(npdt)
+    info = torch.full((batch,), 7, dtype=torch.int32, device=cuda)
+    X = nat.inverse(torch.as_tensor(A, device=cuda), info=info.zero_()).cpu().numpy()
+    assert (info.cpu().numpy() == 0).all()
+    wide = np.complex128 if kind[0] == "c" else np.float64
+    for b in sorted({0, batch // 2, batch - 1}):
+        R = A[b].astype(wide) @ X[b].astype(wide) - np.eye(n)
+        S = (np.abs(A[b]).astype(np.float64) @ np.abs(X[b])).sum(1).max()
+        assert np.abs(R).sum(1).max() <= 16 * n * np.finfo(npdt).eps * S
+
+
+@pytest.mark.parametrize("kind,n", [("f32", 300), ("f64", 200), ("c64", 260), ("c128", 130)])
+def test_register_panels_report_singular_and_spread_nan(cuda, kind, n):
+    dt, npdt = TYPES[kind]
+    A = np.stack([np.eye(n)] * 4)[:, ::-1].copy()
+    A[1, :, 37] = 0.0            # no pivot in the second panel
+    A[2, 5, n - 2] = np.nan
+    A[3] = np.eye(n)[::-1] * 2.0 ** np.arange(-30, 30, 60 / n)[:n, None]
+    info = torch.zeros(4, dtype=torch.int32, device=cuda)
+    X = nat.inverse(torch.as_tensor(A.astype(npdt), device=cuda), info=info).cpu().numpy()
+    inf = info.cpu().numpy()
+    assert inf[0] == 0 and inf[1] == 38 and inf[3] == 0
+    assert np.array_equal(X[0], np.eye(n)[::-1]) and np.isnan(X[2]).any()
+    assert np.allclose(X[3] @ A[3], np.eye(n), atol=4 * np.finfo(npdt).eps)
