@@ -1134,21 +1134,30 @@ __device__ __forceinline__ int pr_best(unsigned long long& key) {
   return l;
 }
 
-template <class T>
-__global__ void __launch_bounds__(pr_rows<T>())
-gje_panel_reg_kernel(int n, int k0, int bw, T* Mat, T* U, T* G, T* E, int* piv, unsigned char* used, int* info) {
+// CLUSTER: the rows of a matrix over the CTAs of a cluster (blockIdx.x, rows_per
+// each; blockIdx.y the matrix).  Every warp sends the magnitude of its offer to
+// all CTAs; after the column's cluster barrier each warp reads the winning row
+// where it was offered.  All CTAs pass the same barriers, so they need no limit.
+template <class T, int MAXT, bool CLUSTER>
+__global__ void __launch_bounds__(MAXT)
+gje_panel_reg_kernel(int n, int k0, int bw, int rows_per, T* Mat, T* U, T* G, T* E, int* piv, unsigned char* used,
+                     int* info) {
+  namespace cg = cooperative_groups;
   using MagT = typename MagOf<T>::type;
   using Key = decltype(pr_key(MagT(), false));
-  constexpr int W = pr_rows<T>() / 32, CH = pr_chunk<T>();
-  const long long b = blockIdx.x, nn = (long long)n * n;
+  constexpr int W = MAXT / 32, CH = pr_chunk<T>(), NC = CLUSTER ? 16 : 1;
+  const int nct = CLUSTER ? gridDim.x : 1, cta = CLUSTER ? blockIdx.x : 0, r0 = cta * rows_per;
+  const int nr = max(0, min(n - r0, rows_per));   // rows of this CTA
+  const long long b = CLUSTER ? blockIdx.y : blockIdx.x, nn = (long long)n * n;
   T* M = Mat + b * nn;
   T* Ub = U + b * (long long)n * BP;
   extern __shared__ __align__(16) unsigned char pr_raw[];
   __shared__ __align__(16) T offer[2][W][BP];
   __shared__ __align__(16) T scaled[W][BP];
-  __shared__ Key offer_key[2][W];
-  __shared__ int offer_row[2][W], Rs[BP];
+  __shared__ Key offer_key[2][NC * W];
+  __shared__ int offer_row[2][NC * W], Rs[BP];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int offers = nct * nw, per = (offers + 31) / 32;   // of them, a lane looks at `per` consecutive ones
   T* tile = reinterpret_cast<T*>(pr_raw + warp * pr_tile<T>());
 
   T x[BP];
@@ -1157,14 +1166,15 @@ gje_panel_reg_kernel(int n, int k0, int bw, T* Mat, T* U, T* G, T* E, int* piv, 
 #pragma unroll
     for (int e = lane; e < 32 * CH; e += 32) {
       const int i = warp * 32 + e / CH, c = c0 + e % CH;
-      tile[(e / CH) * (CH + 1) + e % CH] = i < n && c < bw ? M[(long long)i * n + k0 + c] : zero<T>();
+      tile[(e / CH) * (CH + 1) + e % CH] = i < nr && c < bw ? M[(long long)(r0 + i) * n + k0 + c] : zero<T>();
     }
     __syncwarp();
 #pragma unroll
     for (int c = 0; c < CH; ++c) x[c0 + c] = tile[lane * (CH + 1) + c];
     __syncwarp();
   }
-  bool taken = tid >= n || used[b * n + tid] != 0;
+  const int row = r0 + tid;
+  bool taken = tid >= nr || used[b * n + row] != 0;
   int mine = -1;   // the column this row is the pivot of
 
   auto propose = [&](int buf) {
@@ -1173,29 +1183,52 @@ gje_panel_reg_kernel(int n, int k0, int bw, T* Mat, T* U, T* G, T* E, int* piv, 
     if (lane == l) {
 #pragma unroll
       for (int j = 0; j < BP; ++j) offer[buf][warp][j] = x[j];
+    }
+    const int from = r0 + warp * 32 + l;
+    if constexpr (CLUSTER) {
+      if (lane < nct) {
+        auto cluster = cg::this_cluster();
+        *cluster.map_shared_rank(&offer_key[buf][cta * nw + warp], lane) = key;
+        *cluster.map_shared_rank(&offer_row[buf][cta * nw + warp], lane) = from;
+      }
+    } else if (lane == 0) {
       offer_key[buf][warp] = key;
-      offer_row[buf][warp] = tid;
+      offer_row[buf][warp] = from;
     }
   };
+  auto meet = [&] {
+    if constexpr (CLUSTER) cluster_sync_all();
+    else __syncthreads();
+  };
+  if constexpr (CLUSTER) cluster_sync_all();   // every CTA runs before its memory is written
   propose(0);
-  __syncthreads();
+  meet();
   for (int c = 0; c < bw; ++c) {
     const int buf = c & 1;
-    Key key = lane < nw ? offer_key[buf][lane] : 0;
-    const int w = pr_best(key);
+    Key key = 0;
+    int w = lane * per;
+    if (!CLUSTER || per == 1) {
+      if (lane < offers) key = offer_key[buf][lane];
+    } else {
+      for (int i = lane * per; i < offers && i < (lane + 1) * per; ++i)
+        if (offer_key[buf][i] > key) key = offer_key[buf][i], w = i;
+    }
+    w = __shfl_sync(0xffffffffu, w, pr_best(key));
     const int r = offer_row[buf][w];
     const bool any = key > 1;   // a magnitude above zero
-    const T raw = offer[buf][w][lane];
-    const T pinv = any ? rcp_(offer[buf][w][0]) : zero<T>();
+    const T* won = offer[buf][CLUSTER ? w % nw : w];
+    if constexpr (CLUSTER) won = cg::this_cluster().map_shared_rank(won, w / nw);
+    const T raw = won[lane];
+    const T pinv = any ? rcp_(shfl_T(raw, 0)) : zero<T>();
     scaled[warp][lane] = mul(raw, pinv);
     __syncwarp();
-    if (tid == 0) {
+    if (tid == 0) Rs[c] = r;
+    if (cta == 0 && tid == 0) {
       piv[b * n + k0 + c] = r;
-      Rs[c] = r;
       if (!any && info && info[b] == 0) info[b] = k0 + c + 1;
     }
     const T f = x[0];
-    if (tid == r) {
+    if (row == r && tid < nr) {
 #pragma unroll
       for (int j = 1; j < BP; ++j) x[j - 1] = scaled[warp][j];
       x[BP - 1] = pinv;
@@ -1208,7 +1241,7 @@ gje_panel_reg_kernel(int n, int k0, int bw, T* Mat, T* U, T* G, T* E, int* piv, 
     }
     __syncwarp();
     if (c + 1 < bw) propose(buf ^ 1);
-    __syncthreads();
+    meet();   // the last one: no CTA leaves while its row is read, and Rs is complete
   }
   for (int c = bw; c < BP; ++c) {   // a narrower panel: back to its columns' places
     const T f = x[0];
@@ -1223,7 +1256,7 @@ gje_panel_reg_kernel(int n, int k0, int bw, T* Mat, T* U, T* G, T* E, int* piv, 
 #pragma unroll
     for (int c = 0; c < BP; ++c)
       if (c < bw) Eb[c] = x[c];
-    used[b * n + tid] = 1;
+    used[b * n + row] = 1;
   }
   const uint32_t pivots = __ballot_sync(0xffffffffu, mine >= 0);
 #pragma unroll
@@ -1234,19 +1267,19 @@ gje_panel_reg_kernel(int n, int k0, int bw, T* Mat, T* U, T* G, T* E, int* piv, 
 #pragma unroll 4
     for (int e = lane; e < 32 * CH; e += 32) {
       const int i = warp * 32 + e / CH, c = c0 + e % CH;
-      if (i < n && c < bw) {
+      if (i < nr && c < bw) {
         const T v = tile[(e / CH) * (CH + 1) + e % CH];
-        M[(long long)i * n + k0 + c] = v;
-        Ub[(long long)i * BP + c] = (pivots >> (e / CH)) & 1u ? zero<T>() : v;
+        M[(long long)(r0 + i) * n + k0 + c] = v;
+        Ub[(long long)(r0 + i) * BP + c] = (pivots >> (e / CH)) & 1u ? zero<T>() : v;
       }
     }
     __syncwarp();
   }
   T* Gb = G + b * (long long)BP * n;
-  for (int c = warp; c < bw; c += nw) {
-    const T* row = M + (long long)Rs[c] * n;
+  for (int c = cta * nw + warp; c < bw; c += nct * nw) {
+    const T* m = M + (long long)Rs[c] * n;
 #pragma unroll 8
-    for (int j = lane; j < n; j += 32) Gb[(long long)c * n + j] = j >= k0 && j < k0 + bw ? zero<T>() : row[j];
+    for (int j = lane; j < n; j += 32) Gb[(long long)c * n + j] = j >= k0 && j < k0 + bw ? zero<T>() : m[j];
   }
 }
 
@@ -1846,7 +1879,7 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
   base += L.used * batch;
   unsigned char* syncb = base;
 
-  // Few matrices: split each panel over several CTAs (cooperative launch).
+  // Few matrices of more than 256 rows: split each panel over several CTAs.
   int nct = 0, rows_per = 0;
   size_t csmem = 0;
   {
@@ -1854,7 +1887,7 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&coop_ok, cudaDevAttrCooperativeLaunch, dev);
-    if (n > pr_rows<T>() && coop_ok && sms > 0 && batch < sms && n > 64) {
+    if (coop_ok && sms > 0 && batch < sms && n > 256) {
       nct = 2 * sms / batch;
       if (nct > coop_nct_cap(n)) nct = coop_nct_cap(n);
       bool fits = false;
@@ -1881,8 +1914,44 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
   // CTAs, each holding rows_per rows of the panel in shared memory.
   int ncl = 0, rows_cl = 0;
   size_t clsmem = 0;
+  bool creg = false;   // clusters with a row per thread
+  auto creg_kernel = gje_panel_reg_kernel<T, 128, true>;
   if (nct > 0 && cluster_panels_enabled()) {
+    // A CTA per 128 rows, up to 8: a column's barrier costs about as much as the
+    // 100 row updates it saves.  Complex64, us a panel with 2 / 4 / 8 / 16 CTAs
+    // and before: n = 448 60 / 52 / 55 / 66 and 105 (one CTA 59), 896 79 / 66 /
+    // 58 / 63 and 104, 1792 - / - / 80 / 87 and 109; 224 is best in one CTA (41,
+    // two 52).
+    for (int want : {n <= 1024 ? (n + 127) / 128 : 8, 16}) {
+      const int rp = (n + want - 1) / want, nc = (n + rp - 1) / rp, nth = (rp + 31) / 32 * 32;
+      if (rp > pr_rows<T>() || nc < 2) continue;
+      const auto kern = rp <= 128 ? gje_panel_reg_kernel<T, 128, true> : gje_panel_reg_kernel<T, pr_rows<T>(), true>;
+      const size_t sm = (size_t)(nth / 32) * pr_tile<T>();
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(pr_rows<T>() / 32 * pr_tile<T>()));
+      if (nc > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(nc, batch);
+      cfg.blockDim = dim3(nth);
+      cfg.dynamicSmemBytes = sm;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = nc;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int max_cl = 0;
+      if (cudaOccupancyMaxActiveClusters(&max_cl, kern, &cfg) == cudaSuccess && max_cl >= 1) {
+        creg = true;
+        creg_kernel = kern;
+        ncl = nc;
+        rows_cl = rp;
+        clsmem = sm;
+        break;
+      }
+    }
     for (int want : {16, 8}) {
+      if (creg) break;
       if (want > (coop_nct_cap(n) > 16 ? coop_nct_cap(n) : 16)) continue;
       const int rp = (n + want - 1) / want;
       const int nc = (n + rp - 1) / rp;
@@ -1939,10 +2008,10 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
   int use_smem = 0;
   size_t pan_smem = 0;
   // Up to a row per thread the panel stays in registers.
-  const bool reg = n <= pr_rows<T>();
+  const bool reg = nct == 0 && n <= pr_rows<T>();
   const size_t reg_smem = (size_t)((n + 31) / 32) * pr_tile<T>();
   if (reg) {
-    const cudaError_t e = cudaFuncSetAttribute(gje_panel_reg_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const cudaError_t e = cudaFuncSetAttribute(gje_panel_reg_kernel<T, pr_rows<T>(), false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)(pr_rows<T>() / 32 * pr_tile<T>()));
     if (e != cudaSuccess) return e;
   } else if (nct == 0) {
@@ -1970,7 +2039,7 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
       if (ncl > 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(nct, batch);
-        cfg.blockDim = dim3(CP_NT);
+        cfg.blockDim = dim3(creg ? (rows_per + 31) / 32 * 32 : CP_NT);
         cfg.dynamicSmemBytes = csmem;
         cfg.stream = st;
         cudaLaunchAttribute at[1];
@@ -1980,7 +2049,7 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, gje_panel_cluster_kernel<T>, n_, k0_, bw, rp, Mat_, U_, G_, E_, piv_, used_,
+        e = cudaLaunchKernelEx(&cfg, creg ? creg_kernel : gje_panel_cluster_kernel<T>, n_, k0_, bw, rp, Mat_, U_, G_, E_, piv_, used_,
                                info_);
       } else {
         void* args[] = {&n_, &k0_, &bw, &rp, &Mat_, &U_, &G_, &E_, &piv_, &used_, &info_, &sync_, &lay_};
@@ -1988,7 +2057,8 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
                                         csmem, st);
       }
     } else if (reg) {
-      gje_panel_reg_kernel<T><<<batch, ((n + 31) / 32) * 32, reg_smem, st>>>(n, k0, bw, Mat, U, G, E, piv, used, info);
+      gje_panel_reg_kernel<T, pr_rows<T>(), false>
+          <<<batch, ((n + 31) / 32) * 32, reg_smem, st>>>(n, k0, bw, n, Mat, U, G, E, piv, used, info);
       e = cudaGetLastError();
     } else {
       const int pnt = n >= PANEL_NT ? PANEL_NT : ((n + 31) / 32) * 32;

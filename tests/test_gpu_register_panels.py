@@ -17,7 +17,10 @@ TYPES = {"f32": (torch.float32, np.float32), "f64": (torch.float64, np.float64),
 @pytest.mark.parametrize("kind,n,batch", [
     ("f32", 225, 3), ("f32", 256, 160), ("f32", 481, 1), ("f32", 512, 5), ("f32", 513, 2), ("f64", 65, 2), ("f64", 129, 200),
     ("f64", 255, 1), ("f64", 256, 7), ("f64", 257, 2), ("c64", 129, 1), ("c64", 256, 170), ("c64", 301, 2), ("c64", 512, 3),
-    ("c64", 513, 1), ("c128", 65, 1), ("c128", 112, 160), ("c128", 256, 3), ("c128", 258, 1)])
+    ("c64", 513, 1), ("c128", 65, 1), ("c128", 112, 160), ("c128", 256, 3), ("c128", 258, 1),
+    # over a cluster: 2 to 8 CTAs, uneven last CTAs, more than 32 offers, 16 CTAs, and beyond its rows
+    ("c64", 257, 4), ("c64", 385, 2), ("c64", 1025, 1), ("f32", 897, 3), ("f32", 2100, 1), ("f64", 700, 2), ("f64", 2049, 1),
+    ("c128", 1100, 1), ("c128", 400, 40), ("f32", 4500, 1)])
 def test_inverse_with_register_panels(cuda, kind, n, batch):
     """|A X - I| <= 16 n eps |A| |X| in the row-sum norm: the elimination's own
     bound with a growth of 16, for diagonally dominant matrices with their rows
