@@ -433,6 +433,144 @@ static cudaError_t launch_gemm_cfg(int M, int N, int K, T alpha, const T* A, lon
 }
 
 // ---------------------------------------------------------------------------
+// Complex64 products in 128 x 64 tiles of 8 x 4 numbers a thread, K in slices
+// of 8: 128 multiply-adds for 96 bytes of 16-byte shared loads, where the 4 x 4
+// tiles of gemm_kernel load 64 bytes (8 at a time) for 64.  The rank-32 updates
+// of the blocked inverse (K = 32) also read C, which is brought to L2 while the
+// product runs: 4096 x (256 x 256 x 32) 1,637 -> 1,413 us (49 TFLOP/s of the
+// FP32 pipe's 74) and with C 2,250 -> 1,864; 4096 x (200 x 56 x 256) 2,980 ->
+// 2,440.  Two multiply-adds an instruction (fma.f32x2) were slower: 1,925 and
+// 2,170.  Sums run over k in gemm_kernel's order: the same results.
+// ---------------------------------------------------------------------------
+constexpr int CG_M = 128, CG_N = 64, CG_K = 8, CG_NT = 256;
+
+__global__ void __launch_bounds__(CG_NT, 2)
+gemm_c64_kernel(int M, int N, int K, c64 alpha, const c64* __restrict__ A, long long lda, long long sA,
+                const c64* __restrict__ B, long long ldb, long long sB, c64 beta, const c64* C, long long ldc,
+                long long sC, c64* D, long long ldd, long long sD, int use_c, int vec) {
+  __shared__ __align__(16) c64 As[2][CG_K][CG_M + 2];
+  __shared__ __align__(16) c64 Bs[2][CG_K][CG_N];
+  const long long bz = blockIdx.z;
+  A += bz * sA;
+  B += bz * sB;
+  D += bz * sD;
+  if (use_c) C += bz * sC;
+  const int m0 = blockIdx.y * CG_M, n0 = blockIdx.x * CG_N;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = (warp >> 2) * 64 + (lane >> 2) * 2, wn = (warp & 3) * 16 + (lane & 3) * 2;   // first row and column
+
+  if (use_c) {   // the tile of C on its way to L2 while the product runs
+    for (int e = tid; e < CG_M * (CG_N / 16); e += CG_NT) {
+      const int m = m0 + e / (CG_N / 16), n = n0 + e % (CG_N / 16) * 16;
+      if (m < M && n < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (long long)m * ldc + n));
+    }
+  }
+  c64 ra[4], rb[2];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const int e = tid + l * CG_NT, m = m0 + e / CG_K, k = k0 + e % CG_K;
+      ra[l] = m < M && k < K ? A[(long long)m * lda + k] : zero<c64>();
+    }
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+      const int e = tid + l * CG_NT, k = k0 + e / CG_N, n = n0 + e % CG_N;
+      rb[l] = k < K && n < N ? B[(long long)k * ldb + n] : zero<c64>();
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const int e = tid + l * CG_NT;
+      As[buf][e % CG_K][e / CG_K] = ra[l];
+    }
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+      const int e = tid + l * CG_NT;
+      Bs[buf][e / CG_N][e % CG_N] = rb[l];
+    }
+  };
+  c64 acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = zero<c64>();
+  const int ktiles = (K + CG_K - 1) / CG_K;
+  if (ktiles > 0) {
+    load(0);
+    store(0);
+    __syncthreads();
+  }
+  for (int kt = 0; kt < ktiles; ++kt) {
+    const int buf = kt & 1;
+    if (kt + 1 < ktiles) load((kt + 1) * CG_K);
+#pragma unroll
+    for (int kk = 0; kk < CG_K; ++kk) {
+      c64 a[8], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(&As[buf][kk][wm + 16 * i]);
+        a[2 * i] = c64{v.x, v.y}, a[2 * i + 1] = c64{v.z, v.w};
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float4 v = *reinterpret_cast<const float4*>(&Bs[buf][kk][wn + 8 * j]);
+        b[2 * j] = c64{v.x, v.y}, b[2 * j + 1] = c64{v.z, v.w};
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fma_(a[i], b[j], acc[i][j]);
+    }
+    if (kt + 1 < ktiles) {
+      store(buf ^ 1);
+      __syncthreads();
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int m = m0 + wm + 16 * (i >> 1) + (i & 1);
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+      const int n = n0 + wn + 4 * j;
+      if (n >= N) continue;
+      c64 v = mul(alpha, acc[i][j]), w = mul(alpha, acc[i][j + 1]);
+      const c64* c = C + (long long)m * ldc + n;
+      c64* d = D + (long long)m * ldd + n;
+      if (vec && n + 1 < N) {
+        if (use_c) {
+          const float4 x = *reinterpret_cast<const float4*>(c);
+          v = fma_(beta, c64{x.x, x.y}, v);
+          w = fma_(beta, c64{x.z, x.w}, w);
+        }
+        *reinterpret_cast<float4*>(d) = make_float4(v.x, v.y, w.x, w.y);
+      } else {
+        d[0] = use_c ? fma_(beta, c[0], v) : v;
+        if (n + 1 < N) d[1] = use_c ? fma_(beta, c[1], w) : w;
+      }
+    }
+  }
+}
+
+static cudaError_t launch_gemm_c64(int M, int N, int K, c64 alpha, const c64* A, long long lda, long long sA,
+                                   const c64* B, long long ldb, long long sB, c64 beta, const c64* C, long long ldc,
+                                   long long sC, c64* D, long long ldd, long long sD, int batch, cudaStream_t st) {
+  const int use_c = C != nullptr;
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  const int vec = al16(D) && ldd % 2 == 0 && sD % 2 == 0 && (!use_c || (al16(C) && ldc % 2 == 0 && sC % 2 == 0));
+  for (int b0 = 0; b0 < batch; b0 += 65535) {
+    const int nb = batch - b0 < 65535 ? batch - b0 : 65535;
+    ProfScope ps(KC_GEMM, st, 8.0 * M * (double)N * K * nb);
+    note_launch();
+    gemm_c64_kernel<<<dim3((N + CG_N - 1) / CG_N, (M + CG_M - 1) / CG_M, nb), CG_NT, 0, st>>>(
+        M, N, K, alpha, A + b0 * sA, lda, sA, B + b0 * sB, ldb, sB, beta, use_c ? C + b0 * sC : nullptr, ldc, sC,
+        D + b0 * sD, ldd, sD, use_c, vec);
+  }
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
 // Skinny products (N <= 8 columns: one or a few right-hand sides).  A tiled
 // kernel would spend most of a 64-wide N tile on padding; here one warp owns
 // one row of A, its lanes stride over K (coalesced reads of A, the dominant
@@ -860,6 +998,12 @@ cudaError_t gemm_batched(int M, int N, int K, T alpha, const T* A, long long lda
     }
     return launch_gemm_cfg<T, 64, 64, 8, 4, 4>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc,
                                                sC, D, ldd, sD, batch, st);
+  }
+  if constexpr (std::is_same<T, c64>::value) {
+    // tiles filled to two fifths at least (65 x 33 is faster in 64 x 64 ones), a tile per SM
+    const long long t = (long long)((M + 127) / 128) * ((N + 63) / 64);
+    if (M > 64 && N > 32 && t * batch >= 152 && t * (128 * 64) <= 5ll * M * N / 2)
+      return launch_gemm_c64(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
   }
   if (sizeof(T) == 16 && M <= 32 && N <= 32)
     return launch_gemm_cfg<T, 32, 32, 8, 2, 2>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc,

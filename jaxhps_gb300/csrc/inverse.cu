@@ -445,7 +445,8 @@ static GjeWs gje_layout(size_t es, int n) {
   return w;
 }
 
-// Copies A into the tableau, clears the used flags and sets piv and rinv to
+// Copies A into the tableau (a warp per row: with an index division per number
+// 4096 complex64 matrices of 256 took 1,600 us), clears the used flags and sets piv and rinv to
 // the identity permutation: a panel that gives up after a barrier timeout
 // leaves its piv entries unwritten, and the later kernels index rows and
 // columns through piv / rinv, which therefore always hold indices below n.
@@ -453,11 +454,12 @@ template <class T>
 __global__ void gje_copy_in_kernel(int n, const T* __restrict__ A, long long lda, long long sA, T* Mat,
                                    unsigned char* used, int* piv, int* rinv) {
   const long long b = blockIdx.y;
-  const long long nn = (long long)n * n;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long i = e / n, j = e % n;
-    Mat[b * nn + e] = A[b * sA + i * lda + j];
+  const int lane = threadIdx.x & 31;
+  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += gridDim.x * 8) {
+    const T* a = A + b * sA + (long long)i * lda;
+    T* m = Mat + (b * n + i) * (long long)n;
+#pragma unroll 4
+    for (int j = lane; j < n; j += 32) m[j] = a[j];
   }
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -1296,6 +1298,41 @@ __global__ void gje_scatter_rows_kernel(int n, int k0, int bw, T* Mat, const T* 
   }
 }
 
+// Pivot rows outside the panel (FP32 types): Mat[piv[k0 + c]] = E G, 32 x 64 numbers a CTA,
+// eight of a column per thread.  As a product of 64 x 64 tiles into H and a
+// kernel that moved H's rows, 4096 complex64 panels of 32 x 256 took 390 + 173
+// us, here 251 (reading G and writing the rows: 80).
+template <class T>
+__global__ void __launch_bounds__(256)
+gje_rows_kernel(int n, int k0, int bw, T* Mat, const T* __restrict__ E, const T* __restrict__ G,
+                const int* __restrict__ piv) {
+  __shared__ __align__(16) T Es[BP][BP];   // [k][row]
+  __shared__ T Gs[BP][64];
+  const long long b = blockIdx.y;
+  const int tid = threadIdx.x, col = tid & 63, row = (tid >> 6) * 8, j = blockIdx.x * 64 + col;
+  E += b * BP * BP;
+  G += b * (long long)BP * n;
+#pragma unroll
+  for (int e = tid; e < BP * BP; e += 256)
+    Es[e % BP][e / BP] = e / BP < bw && e % BP < bw ? E[e] : zero<T>();
+#pragma unroll
+  for (int k = tid >> 6; k < BP; k += 4) Gs[k][col] = k < bw && j < n ? G[(long long)k * n + j] : zero<T>();
+  __syncthreads();
+  if (j >= n || (j >= k0 && j < k0 + bw)) return;
+  T acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = zero<T>();
+#pragma unroll 8
+  for (int k = 0; k < bw; ++k) {
+    const T g = Gs[k][col];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = fma_(Es[k][row + i], g, acc[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (row + i < bw) Mat[(b * n + piv[b * n + k0 + row + i]) * (long long)n + j] = acc[i];
+}
+
 __global__ void gje_rinv_kernel(int n, const int* piv, int* rinv) {
   const long long b = blockIdx.y;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
@@ -1306,12 +1343,13 @@ template <class T>
 __global__ void gje_permute_out_kernel(int n, const T* Mat, const int* piv, const int* rinv, T* X,
                                        long long ldx, long long sX) {
   const long long b = blockIdx.y;
-  const long long nn = (long long)n * n;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(e / n), j = (int)(e % n);
-    X[b * sX + (long long)k * ldx + j] =
-        Mat[b * nn + (long long)piv[b * n + k] * n + rinv[b * n + j]];
+  const int lane = threadIdx.x & 31;
+  const int* rj = rinv + b * n;
+  for (int k = blockIdx.x * 8 + (threadIdx.x >> 5); k < n; k += gridDim.x * 8) {
+    const T* m = Mat + (b * n + piv[b * n + k]) * (long long)n;
+    T* x = X + b * sX + (long long)k * ldx;
+#pragma unroll 4
+    for (int j = lane; j < n; j += 32) x[j] = m[rj[j]];
   }
 }
 
@@ -1995,8 +2033,7 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
   const long long nn = (long long)n * n;
   for (int b0 = 0; b0 < batch; b0 += 65535) {
     const int nb = (batch - b0) < 65535 ? (batch - b0) : 65535;
-    int gx = (int)((nn + 255) / 256);
-    if (gx > 1024) gx = 1024;
+    const int gx = (n + 7) / 8;
     note_launch();
     gje_copy_in_kernel<T><<<dim3(gx, nb), 256, 0, st>>>(n, A + (long long)b0 * sA, lda, sA,
                                                         Mat + (long long)b0 * nn, used + (long long)b0 * n,
@@ -2067,20 +2104,27 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
-    // H = E G
-    e = gemm_batched<T>(bw, n, bw, one_, E, BP, BP * BP, G, n, (long long)BP * n, zero<T>(), nullptr, 0,
-                        0, H, n, (long long)BP * n, batch, st);
-    if (e != cudaSuccess) return e;
+    // FP64: H = E G as a product (its digits are faster than the FP64 pipe), then into the pivot rows
+    constexpr bool wide = sizeof(typename MagOf<T>::type) == 8;
+    if constexpr (wide) {
+      e = gemm_batched<T>(bw, n, bw, one_, E, BP, BP * BP, G, n, (long long)BP * n, zero<T>(), nullptr, 0, 0, H, n,
+                          (long long)BP * n, batch, st);
+      if (e != cudaSuccess) return e;
+    }
     // Mat += U G
     e = gemm_batched<T>(n, n, bw, one_, U, BP, (long long)n * BP, G, n, (long long)BP * n, one_, Mat, n,
                         nn, Mat, n, nn, batch, st);
     if (e != cudaSuccess) return e;
     for (int b0 = 0; b0 < batch; b0 += 65535) {
       const int nb = (batch - b0) < 65535 ? (batch - b0) : 65535;
-      int gx = (bw * n + 255) / 256;
       note_launch();
-      gje_scatter_rows_kernel<T><<<dim3(gx, nb), 256, 0, st>>>(
-          n, k0, bw, Mat + (long long)b0 * nn, H + (long long)b0 * BP * n, piv + (long long)b0 * n);
+      if constexpr (wide)
+        gje_scatter_rows_kernel<T><<<dim3((bw * n + 255) / 256, nb), 256, 0, st>>>(
+            n, k0, bw, Mat + (long long)b0 * nn, H + (long long)b0 * BP * n, piv + (long long)b0 * n);
+      else
+        gje_rows_kernel<T><<<dim3((n + 63) / 64, nb), 256, 0, st>>>(n, k0, bw, Mat + (long long)b0 * nn,
+                                                                    E + (long long)b0 * BP * BP,
+                                                                    G + (long long)b0 * BP * n, piv + (long long)b0 * n);
     }
   }
   for (int b0 = 0; b0 < batch; b0 += 65535) {
@@ -2088,8 +2132,7 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
     note_launch();
     gje_rinv_kernel<<<dim3((n + 255) / 256, nb), 256, 0, st>>>(n, piv + (long long)b0 * n,
                                                                rinv + (long long)b0 * n);
-    int gx = (int)((nn + 255) / 256);
-    if (gx > 2048) gx = 2048;
+    const int gx = (n + 7) / 8;
     note_launch();
     gje_permute_out_kernel<T><<<dim3(gx, nb), 256, 0, st>>>(
         n, Mat + (long long)b0 * nn, piv + (long long)b0 * n, rinv + (long long)b0 * n,
