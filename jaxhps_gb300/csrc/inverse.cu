@@ -1820,6 +1820,122 @@ cudaError_t inverse_batched(int n, const T* A, long long lda, long long sA, T* X
   return inverse_batched_flat<T>(n, A, lda, sA, X, ldx, sX, batch, info, ws, ws_bytes, st, tensor_memory);
 }
 
+// FP64 matrices of n <= 64: a thread per row and half of the columns (2 c + g
+// for the warps of half g), in registers.  As in gje_panel_reg_kernel a
+// column's step shifts the rows of the half that owns it by one register.
+//
+// The FP64 pipe (two multiply-adds an SM and clock) bounds this: n^2 / 2 cycles
+// a column for the update.  inv_reg_kernel spends as much again three times
+// over, 512 threads taking the same reciprocal and comparing magnitudes in
+// FP64: here they are compared as integers, one warp takes the reciprocal and
+// the row is scaled once per warp.  4 matrices of 48 249 -> 77 us, 64 of 36
+// 187 -> 55, 1024 of 56 1,825 -> 420.  The same operations on the same
+// numbers: the same results.
+template <int NMAX>
+__global__ void __launch_bounds__((NMAX + 31) / 32 * 64)
+inv_rows_f64_kernel(int n, const double* __restrict__ A, long long lda, long long sA, double* X, long long ldx,
+                    long long sX, int* info) {
+  constexpr int RW = (NMAX + 31) / 32, H = NMAX / 2;   // warps of rows, columns of a half
+  __shared__ double tile[NMAX][NMAX + 1];
+  __shared__ double colv[2][RW * 32], offered[2][2][H], scaled[2 * RW][H], s_pinv[2];
+  __shared__ unsigned long long wkey[2][RW];
+  __shared__ int wrow[2][RW], piv[NMAX], colof[NMAX];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rw = warp % RW, g = warp / RW;
+  const int row = rw * 32 + lane;
+  const long long b = blockIdx.x;
+  for (int e = tid; e < NMAX * NMAX; e += RW * 64) {
+    const int i = e / NMAX, j = e % NMAX;
+    tile[i][j] = i < n && j < n ? A[b * sA + (long long)i * lda + j] : 0.0;
+  }
+  __syncthreads();
+  double x[H];
+#pragma unroll
+  for (int c = 0; c < H; ++c) x[c] = row < NMAX ? tile[row][2 * c + g] : 0.0;
+  bool taken = row >= n;
+  int first_bad = 0;
+  for (int k = 0; k < n; ++k) {
+    const int buf = k & 1;
+    const bool own = g == (k & 1);   // the same for a warp
+    if (own) {
+      colv[buf][row] = x[0];
+      unsigned long long key = pr_key(nan_to_inf(fabs(x[0])), taken);
+      const int l = pr_best(key);
+      if (lane == 0) {
+        wkey[buf][rw] = key;
+        wrow[buf][rw] = rw * 32 + l;
+      }
+    }
+    __syncthreads();
+    unsigned long long key = wkey[buf][0];
+    int r = wrow[buf][0];
+    if (RW > 1 && wkey[buf][RW - 1] > key) key = wkey[buf][RW - 1], r = wrow[buf][RW - 1];
+    const bool any = key > 1;   // a magnitude above zero
+    if (row == r) {
+#pragma unroll
+      for (int c = 0; c < H; ++c) offered[buf][g][c] = x[c];
+    }
+    if (warp == 0) {
+      const double pv = any ? rcp_(colv[buf][r]) : 0.0;
+      if (lane == 0) {
+        s_pinv[buf] = pv;
+        piv[k] = r;
+        colof[r] = k;
+        if (!any && first_bad == 0) first_bad = k + 1;
+      }
+    }
+    __syncthreads();
+    const double pinv = s_pinv[buf], f = colv[buf][row];
+    if (lane < H) scaled[warp][lane] = offered[buf][g][lane] * pinv;
+    __syncwarp();
+    const bool mine = row == r;
+    if (own) {
+#pragma unroll
+      for (int c = 1; c < H; ++c) x[c - 1] = fms_(f, scaled[warp][c], x[c]);
+      x[H - 1] = neg(f * pinv);
+    } else {
+#pragma unroll
+      for (int c = 0; c < H; ++c) x[c] = fms_(f, scaled[warp][c], x[c]);
+    }
+    if (mine) {
+      taken = true;
+      if (own) {
+#pragma unroll
+        for (int c = 1; c < H; ++c) x[c - 1] = scaled[warp][c];
+        x[H - 1] = pinv;
+      } else {
+#pragma unroll
+        for (int c = 0; c < H; ++c) x[c] = scaled[warp][c];
+      }
+    }
+    __syncwarp();
+  }
+  for (int c = (n - g + 1) / 2; c < H; ++c) {   // back to the columns' places
+    const double f = x[0];
+#pragma unroll
+    for (int j = 1; j < H; ++j) x[j - 1] = x[j];
+    x[H - 1] = f;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < H; ++c)
+    if (row < NMAX) tile[row][2 * c + g] = x[c];
+  __syncthreads();
+  for (int e = tid; e < n * NMAX; e += RW * 64) {
+    const int i = e / NMAX, j = e % NMAX;
+    if (j < n) X[b * sX + (long long)i * ldx + j] = tile[piv[i]][colof[j]];
+  }
+  if (tid == 0 && info) info[b] = first_bad;
+}
+
+template <int NMAX>
+static cudaError_t launch_rows_f64(int n, const double* A, long long lda, long long sA, double* X, long long ldx,
+                                   long long sX, int batch, int* info, cudaStream_t st) {
+  ProfScope ps(KC_INVERSE, st, 2.0 * (double)n * n * n * batch);
+  note_launch();
+  inv_rows_f64_kernel<NMAX><<<batch, (NMAX + 31) / 32 * 64, 0, st>>>(n, A, lda, sA, X, ldx, sX, info);
+  return cudaGetLastError();
+}
+
 template <class T, int NMAX>
 static cudaError_t launch_reg(int n, const T* A, long long lda, long long sA, T* X, long long ldx,
                              long long sX, int batch, int* info, cudaStream_t st) {
@@ -1850,8 +1966,14 @@ cudaError_t inverse_small<float>(int n, const float* A, long long lda, long long
 template <>
 cudaError_t inverse_small<double>(int n, const double* A, long long lda, long long sA, double* X,
                                   long long ldx, long long sX, int batch, int* info, cudaStream_t st) {
-  if (n <= 32) return launch_reg<double, 32>(n, A, lda, sA, X, ldx, sX, batch, info, st);
-  if (n <= 64) return launch_reg<double, 64>(n, A, lda, sA, X, ldx, sX, batch, info, st);
+  // the update is done on all NMAX columns: an instance per 8
+  if (n <= 16) return launch_rows_f64<16>(n, A, lda, sA, X, ldx, sX, batch, info, st);
+  if (n <= 24) return launch_rows_f64<24>(n, A, lda, sA, X, ldx, sX, batch, info, st);
+  if (n <= 32) return launch_rows_f64<32>(n, A, lda, sA, X, ldx, sX, batch, info, st);
+  if (n <= 40) return launch_rows_f64<40>(n, A, lda, sA, X, ldx, sX, batch, info, st);
+  if (n <= 48) return launch_rows_f64<48>(n, A, lda, sA, X, ldx, sX, batch, info, st);
+  if (n <= 56) return launch_rows_f64<56>(n, A, lda, sA, X, ldx, sX, batch, info, st);
+  if (n <= 64) return launch_rows_f64<64>(n, A, lda, sA, X, ldx, sX, batch, info, st);
   return launch_reg<double, 128>(n, A, lda, sA, X, ldx, sX, batch, info, st);
 }
 template <>

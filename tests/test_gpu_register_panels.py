@@ -55,3 +55,23 @@ def test_register_panels_report_singular_and_spread_nan(cuda, kind, n):
     assert inf[0] == 0 and inf[1] == 38 and inf[3] == 0
     assert np.array_equal(X[0], np.eye(n)[::-1]) and np.isnan(X[2]).any()
     assert np.allclose(X[3] @ A[3], np.eye(n), atol=4 * np.finfo(npdt).eps)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 15, 16, 17, 24, 25, 31, 32, 33, 40, 41, 48, 49, 56, 57, 63, 64])
+def test_small_fp64_inverse_by_rows(cuda, n):
+    """inv_rows_f64_kernel at the edges of its instances, in place, strided, and
+    with a zero column and a NaN in one matrix each; bound as above."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((5, n, n + 3)) + 2 * np.sqrt(n) * np.eye(n, n + 3)
+    A = np.ascontiguousarray(A[:, rng.permutation(n)])
+    A[3, :, n // 2] = 0.0
+    A[4, 0, n - 1] = np.nan
+    t = torch.as_tensor(A, device=cuda)[..., :n]
+    info = torch.zeros(5, dtype=torch.int32, device=cuda)
+    X = nat.inverse(t, out=t, info=info).cpu().numpy()
+    inf = info.cpu().numpy()
+    assert (inf[:3] == 0).all() and inf[3] == n // 2 + 1 and np.isnan(X[4]).any()
+    for b in range(3):
+        R = A[b, :, :n] @ X[b] - np.eye(n)
+        S = (np.abs(A[b, :, :n]) @ np.abs(X[b])).sum(1).max()
+        assert np.abs(R).sum(1).max() <= 16 * n * 2.0 ** -52 * S
