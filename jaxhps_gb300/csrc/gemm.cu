@@ -25,6 +25,24 @@
 
 namespace hps {
 
+// A BM x BN tile of C on its way to L2 while the product runs: read after it,
+// its latency was a third of a rank-32 update's time (4096 x (256 x 256 x 32)
+// complex64, beyond the product alone 633 us without and 450 with this).
+// use_c: 1 with a C, and 2 where it is larger than what L2 is likely to hold
+// (64 x (64 x 1536 x 64) and smaller lose up to 2 us to the requests).
+template <class T>
+static int use_c_flags(const T* C, int M, int N, int batch) {
+  return C == nullptr ? 0 : (double)M * N * batch * sizeof(T) >= 64e6 ? 3 : 1;
+}
+template <class T, int BM, int BN, int NT>
+__device__ __forceinline__ void prefetch_tile(const T* C, long long ldc, int m0, int n0, int M, int N, int tid) {
+  constexpr int L = 128 / (int)sizeof(T), PL = (BN + L - 1) / L;   // numbers a line, lines a row
+  for (int e = tid; e < BM * PL; e += NT) {
+    const int m = m0 + e / PL, n = n0 + e % PL * L;
+    if (m < M && n < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (long long)m * ldc + n));
+  }
+}
+
 template <class T, int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_kernel(int M, int N, int K, T alpha, const T* __restrict__ A, long long lda, long long sA,
@@ -49,6 +67,7 @@ gemm_kernel(int M, int N, int K, T alpha, const T* __restrict__ A, long long lda
   const int tx = tid % NTX;
   const int ty = tid / NTX;
 
+  if (use_c & 2) prefetch_tile<T, BM, BN, NT>(C, ldc, m0, n0, M, N, tid);
   T ra[LA], rb[LB];
   auto load_tiles = [&](int k0) {
 #pragma unroll
@@ -189,6 +208,7 @@ gemm_f32_v4_kernel(int M, int N, int K, float alpha, const float* __restrict__ A
   const int tx = tid % NTX;
   const int ty = tid / NTX;
 
+  if (!SPLIT && (use_c & 2)) prefetch_tile<float, BM, BN, NT>(C, ldc, m0, n0, M, N, tid);
   float4 ra[A4], rb[B4];
   auto load_tiles = [&](int k0) {
 #pragma unroll
@@ -351,7 +371,7 @@ static cudaError_t launch_gemm_f32_v4(int M, int N, int K, float alpha, const fl
                                       const float* B, long long ldb, long long sB, float beta, const float* C,
                                       long long ldc, long long sC, float* D, long long ldd, long long sD, int batch,
                                       cudaStream_t st) {
-  const int use_c = (C != nullptr);
+  const int use_c = use_c_flags(C, M, N, batch);
   constexpr int NT = (BM / 8) * (BN / 8);
   // float4 rows: leading dimensions and batch strides multiples of 4 floats,
   // base addresses 16-byte aligned (then every row start and k or n offset
@@ -417,7 +437,7 @@ static cudaError_t launch_gemm_cfg(int M, int N, int K, T alpha, const T* A, lon
                                    const T* B, long long ldb, long long sB, T beta, const T* C,
                                    long long ldc, long long sC, T* D, long long ldd, long long sD,
                                    int batch, cudaStream_t st) {
-  const int use_c = (C != nullptr);
+  const int use_c = use_c_flags(C, M, N, batch);
   constexpr int NT = (BM / TM) * (BN / TN);
   for (int b0 = 0; b0 < batch; b0 += 65535) {
     int nb = batch - b0 < 65535 ? batch - b0 : 65535;
@@ -459,12 +479,7 @@ gemm_c64_kernel(int M, int N, int K, c64 alpha, const c64* __restrict__ A, long 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = (warp >> 2) * 64 + (lane >> 2) * 2, wn = (warp & 3) * 16 + (lane & 3) * 2;   // first row and column
 
-  if (use_c) {   // the tile of C on its way to L2 while the product runs
-    for (int e = tid; e < CG_M * (CG_N / 16); e += CG_NT) {
-      const int m = m0 + e / (CG_N / 16), n = n0 + e % (CG_N / 16) * 16;
-      if (m < M && n < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (long long)m * ldc + n));
-    }
-  }
+  if (use_c & 2) prefetch_tile<c64, CG_M, CG_N, CG_NT>(C, ldc, m0, n0, M, N, tid);
   c64 ra[4], rb[2];
   auto load = [&](int k0) {
 #pragma unroll
@@ -556,7 +571,7 @@ gemm_c64_kernel(int M, int N, int K, c64 alpha, const c64* __restrict__ A, long 
 static cudaError_t launch_gemm_c64(int M, int N, int K, c64 alpha, const c64* A, long long lda, long long sA,
                                    const c64* B, long long ldb, long long sB, c64 beta, const c64* C, long long ldc,
                                    long long sC, c64* D, long long ldd, long long sD, int batch, cudaStream_t st) {
-  const int use_c = C != nullptr;
+  const int use_c = use_c_flags(C, M, N, batch);
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   const int vec = al16(D) && ldd % 2 == 0 && sD % 2 == 0 && (!use_c || (al16(C) && ldc % 2 == 0 && sC % 2 == 0));
   for (int b0 = 0; b0 < batch; b0 += 65535) {
@@ -574,8 +589,14 @@ static cudaError_t launch_gemm_c64(int M, int N, int K, c64 alpha, const c64* A,
 // Skinny products (N <= 8 columns: one or a few right-hand sides).  A tiled
 // kernel would spend most of a 64-wide N tile on padding; here one warp owns
 // one row of A, its lanes stride over K (coalesced reads of A, the dominant
-// traffic) and the N partial sums are reduced with shuffles.  The kernel is
-// bound by reading A once.
+// traffic) and the N partial sums are reduced with shuffles.  With many rows a
+// warp takes R of them: the loads of R rows are in flight together, and its
+// R N partial sums are reduced by halves, each exchange leaving a lane half as
+// many (9 additions for 8 sums where every lane adding up all takes 40: with
+// FP64's two a clock that was more work than the product).  The additions are
+// those of the same pairs: the same results.  FP64, us with one row and with R:
+// 4096 x (196 x 1 x 196) 660 and 405, 512 x (512 x 1 x 512) 345 and 261, 4096 x
+// (256 x 1 x 56) 574 and 250; FP32 207 and 129, 96 and 85, 149 and 72.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float shfl_xor_(float v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
 __device__ __forceinline__ double shfl_xor_(double v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
@@ -588,40 +609,65 @@ __device__ __forceinline__ c128 shfl_xor_(c128 v, int m) {
 
 constexpr int SK_WARPS = 8;
 
-template <class T, int NB>
+// Sums of V values (a power of two) over a warp: lane l returns the sum of value
+// l / (32 / V).
+template <class T, int V>
+__device__ __forceinline__ T reduce_halves(T (&v)[V], int lane) {
+#pragma unroll
+  for (int o = 16, n = V; o > 0; o >>= 1) {
+    if (n > 1) {
+      n >>= 1;
+      const bool up = lane & o;
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i)
+        if (i < n) {
+          const T keep = up ? v[i + n] : v[i], give = up ? v[i] : v[i + n];
+          v[i] = add(keep, shfl_xor_(give, o));
+        }
+    } else {
+      v[0] = add(v[0], shfl_xor_(v[0], o));
+    }
+  }
+  return v[0];
+}
+
+template <class T, int NB, int R>
 __global__ void __launch_bounds__(SK_WARPS * 32)
 gemm_skinny_kernel(int M, int N, int K, T alpha, const T* __restrict__ A, long long lda, long long sA,
                    const T* __restrict__ B, long long ldb, long long sB, T beta, const T* C, long long ldc,
                    long long sC, T* D, long long ldd, long long sD, int use_c) {
+  constexpr int V = R * NB;
   const int lane = threadIdx.x & 31;
-  const int row = blockIdx.x * SK_WARPS + (threadIdx.x >> 5);
-  if (row >= M) return;  // uniform across the warp
+  const int row0 = (blockIdx.x * SK_WARPS + (threadIdx.x >> 5)) * R;
+  if (row0 >= M) return;  // uniform across the warp
   const long long bz = blockIdx.y;
-  const T* a = A + bz * sA + (long long)row * lda;
   const T* b = B + bz * sB;
-  T acc[NB];
+  const T* a[R];
 #pragma unroll
-  for (int n = 0; n < NB; ++n) acc[n] = zero<T>();
+  for (int r = 0; r < R; ++r) a[r] = A + bz * sA + (long long)min(row0 + r, M - 1) * lda;
+  T acc[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) acc[i] = zero<T>();
 #pragma unroll 4
   for (int k = lane; k < K; k += 32) {
-    const T av = a[k];
+    T av[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) av[r] = a[r][k];
     const T* br = b + (long long)k * ldb;
 #pragma unroll
     for (int n = 0; n < NB; ++n)
-      if (n < N) acc[n] = fma_(av, br[n], acc[n]);
+      if (n < N) {
+        const T bv = br[n];
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r * NB + n] = fma_(av[r], bv, acc[r * NB + n]);
+      }
   }
-#pragma unroll
-  for (int n = 0; n < NB; ++n)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc[n] = add(acc[n], shfl_xor_(acc[n], o));
-  if (lane < N) {
-    T v = acc[0];
-#pragma unroll
-    for (int n = 1; n < NB; ++n)
-      if (lane == n) v = acc[n];
+  const T v = reduce_halves<T, V>(acc, lane);
+  const int i = lane / (32 / V), row = row0 + i / NB, n = i % NB;
+  if (lane % (32 / V) == 0 && n < N && row < M) {
     T out = mul(alpha, v);
-    if (use_c) out = fma_(beta, C[bz * sC + (long long)row * ldc + lane], out);
-    D[bz * sD + (long long)row * ldd + lane] = out;
+    if (use_c) out = fma_(beta, C[bz * sC + (long long)row * ldc + n], out);
+    D[bz * sD + (long long)row * ldd + n] = out;
   }
 }
 
@@ -630,15 +676,24 @@ static cudaError_t launch_skinny(int M, int N, int K, T alpha, const T* A, long 
                                  long long ldb, long long sB, T beta, const T* C, long long ldc, long long sC, T* D,
                                  long long ldd, long long sD, int batch, cudaStream_t st) {
   const int use_c = (C != nullptr);
+  constexpr int R = NB < 4 ? 4 / NB : 1;
+  // R rows a warp where that leaves 16 warps an SM
+  const bool many = R > 1 && M >= R && (long long)M * batch >= (long long)R * 16 * 152;
   for (int b0 = 0; b0 < batch; b0 += 65535) {
     const int nb = batch - b0 < 65535 ? batch - b0 : 65535;
-    dim3 grid((M + SK_WARPS - 1) / SK_WARPS, nb);
+    const int rows = SK_WARPS * (many ? R : 1);
     const double cplx = (sizeof(T) == 16 || (sizeof(T) == 8 && DTypeOf<T>::value == C64)) ? 4.0 : 1.0;
     ProfScope ps(KC_GEMM, st, 2.0 * cplx * M * (double)N * K * nb);
-    note_launch();
-    gemm_skinny_kernel<T, NB><<<grid, SK_WARPS * 32, 0, st>>>(
-        M, N, K, alpha, A + b0 * sA, lda, sA, B + b0 * sB, ldb, sB, beta, use_c ? C + b0 * sC : nullptr, ldc, sC,
-        D + b0 * sD, ldd, sD, use_c);
+    auto go = [&](auto kernel) {
+      note_launch();
+      kernel<<<dim3((M + rows - 1) / rows, nb), SK_WARPS * 32, 0, st>>>(
+          M, N, K, alpha, A + b0 * sA, lda, sA, B + b0 * sB, ldb, sB, beta, use_c ? C + b0 * sC : nullptr, ldc, sC,
+          D + b0 * sD, ldd, sD, use_c);
+    };
+    if (many)
+      go(gemm_skinny_kernel<T, NB, R>);
+    else
+      go(gemm_skinny_kernel<T, NB, 1>);
   }
   return cudaGetLastError();
 }
@@ -877,11 +932,10 @@ bool f64_products_on_tensor_cores() {
 // outputs or more (112 x 112 x 4 x 256 50 against 75 us, x 16 23 against 20).  Products
 // with N <= 8 columns read A once either way and their FP64 time grows with N,
 // so both times are estimated, in us: a round of 128-row tiles on 152 SMs
-// takes 0.077 per step of K; the one-row-per-warp kernel 4.2e-6 (N = 1) to
-// 28e-6 (N = 8) per element of A (complex: 11.7e-6 to 74e-6).  Measured at
-// M = K = 196: N = 1 0.67 (FP64) against 0.93 ms, N = 2 1.20 against 0.92, N = 8
-// 4.4 against 0.94 (batch 4096); M = 1792, K = 3584, N = 8, one matrix: 0.13
-// against 0.28 ms.
+// takes 0.077 per step of K; the row-per-warp kernel 2.6e-6 (N = 1) to 18.6e-6
+// (N = 8) per element of A (complex: 9.1e-6 to 66e-6).  Measured at M = K = 196,
+// batch 4096: N = 1 0.41 (FP64) against 0.92 ms, N = 2 0.80 against 0.92, N = 8
+// 2.9 against 0.94; M = 3584, K = 1792, N = 8, one matrix: 0.094 against 0.149.
 static bool f64_on_tensor_cores(int M, int N, int K, int batch, bool cplx) {
   if (K <= 0 || !f64_products_on_tensor_cores()) return false;
   if (gemm_policy() == 2) return true;
@@ -890,8 +944,8 @@ static bool f64_on_tensor_cores(int M, int N, int K, int batch, bool cplx) {
   const double tiles = (double)((M + 127) / 128) * batch;
   const double rounds = (double)(((long long)tiles + 151) / 152);
   const double tc = 15.0 + rounds * K * (cplx ? 0.154 : 0.077);
-  const double per = cplx ? (N == 1 ? 11.7e-6 : N == 2 ? 20.7e-6 : N <= 4 ? 38e-6 : 74e-6)
-                          : (N == 1 ? 4.2e-6 : N == 2 ? 7.6e-6 : N <= 4 ? 14.5e-6 : 28e-6);
+  const double per = cplx ? (N == 1 ? 9.1e-6 : N == 2 ? 17.4e-6 : N <= 4 ? 34.8e-6 : 66e-6)
+                          : (N == 1 ? 2.6e-6 : N == 2 ? 5.1e-6 : N <= 4 ? 10.2e-6 : 18.6e-6);
   return tc < 10.0 + per * M * (double)K * batch;
 }
 
