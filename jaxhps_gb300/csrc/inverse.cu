@@ -1463,201 +1463,140 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
 // ---------------------------------------------------------------------------
 // Block Gauss-Jordan inversion of one FP32 matrix per CTA, n <= 128, for the
 // interface blocks the recursive inversion ends at (and the n <= 128 merge
-// interfaces).  The matrix lives in registers (thread (ty, tx) of a 16 x 32
-// grid owns rows ty + 16 a, columns tx + 32 c); each of the n / 16 steps
-// publishes the 16-wide column and row blocks to shared memory, one warp
-// inverts the 16 x 16 diagonal block in registers (Gauss-Jordan with partial
-// pivoting inside the block, a column of [M_kk | I] per lane), the CTA forms
-// the new row block R = P M_k. and every thread updates its elements as an
-// outer product:
+// interfaces).  The matrix lives in registers: warp w holds the rows 8 w .. 8 w
+// + 7, lane l the columns 4 l .. 4 l + 3, so that a step's operands are 16-byte
+// loads (the columns' one, the rows' two for the whole warp) and the warps and
+// lanes of a 16-wide block are whole ones.  Each of the n / 16 steps publishes
+// the column and row blocks to shared memory, one warp inverts the 16 x 16
+// diagonal block (Gauss-Jordan with partial pivoting inside the block, a row
+// per lane, shifted by one register per pivot), the CTA forms the new row
+// block R = P M_k. and every thread updates its elements as an outer product:
 //     M_ij -= M_ik R_kj,  M_kj = R_kj,  M_ik = -M_ik P,  M_kk = P.
 // Pivots are searched within the 16 x 16 blocks only (as in the recursion
-// above); a zero pivot sets info to its column (1-based).  Six barriers per
-// 16 columns where the per-column kernels need one or two per column.
+// above); a zero pivot sets info to its column (1-based).
+// Bound by the chain of pivots and four barriers a step: one matrix of 112
+// takes 47 us (128: 55).  With rows and columns dealt out 16 and 32 apart (8 + 4 loads
+// of four bytes for 32 multiply-adds) and the diagonal block's columns in the
+// lanes (the pivot searched by a tree over 16 registers, 16 shuffles of its
+// factors): 86 us, 10,100 cycles a step for the diagonal block, 9,700 for the
+// update, 2,600 for R and 1,500 to publish.
 // ---------------------------------------------------------------------------
-constexpr int B16_NT = 512, B16_TY = 16, B16_TX = 32, B16_B = 16, B16_NMAX = 128;
-constexpr int B16_RM = B16_NMAX / B16_TY, B16_RN = B16_NMAX / B16_TX;   // 8 x 4 elements per thread
+constexpr int B16_NT = 512, B16_B = 16, B16_NMAX = 128;
 
 __global__ void __launch_bounds__(B16_NT, 1)
 inv_block16_kernel(int n, const float* __restrict__ A, long long lda, long long sA, float* X, long long ldx,
                    long long sX, int* info) {
-  __shared__ float Cb[B16_NMAX][B16_B + 1];   // the step's column block (old values)
-  __shared__ float Rk[B16_B][B16_NMAX + 1];   // the step's row block, then R = P M_k.
-  __shared__ float Pk[B16_B][B16_B + 1];      // inverse of the diagonal block
-  __shared__ float Ag[1][B16_B][2 * B16_B + 1];   // [M_kk | I] after elimination
-  __shared__ int rowof_s[B16_B];
+  __shared__ __align__(16) float Cb[B16_B][B16_NMAX];   // the step's column block (old values), transposed
+  __shared__ __align__(16) float Rk[B16_B][B16_NMAX];   // the step's row block
+  __shared__ __align__(16) float Rn[B16_B][B16_NMAX];   // R = P M_k., P in the block's own columns
+  __shared__ float Pk[B16_B][B16_B + 1];                // inverse of the diagonal block
   __shared__ int s_info;
   const long long bb = blockIdx.x;
   const float* Ab = A + bb * sA;
-  const int tid = threadIdx.x, ty = tid / B16_TX, tx = tid % B16_TX, lane = tid & 31, warp = tid >> 5;
-  float m[B16_RM][B16_RN];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, i0 = 8 * warp, j0 = 4 * lane;
+  float m[8][4];
 #pragma unroll
-  for (int a = 0; a < B16_RM; ++a)
+  for (int a = 0; a < 8; ++a)
 #pragma unroll
-    for (int c = 0; c < B16_RN; ++c) {
-      const int i = ty + B16_TY * a, j = tx + B16_TX * c;
-      m[a][c] = (i < n && j < n) ? Ab[(long long)i * lda + j] : 0.f;
-    }
+    for (int c = 0; c < 4; ++c) m[a][c] = (i0 + a < n && j0 + c < n) ? Ab[(long long)(i0 + a) * lda + j0 + c] : 0.f;
   if (tid == 0) s_info = 0;
   for (int k0 = 0; k0 < n; k0 += B16_B) {
     const int bs = min(B16_B, n - k0);
+    const bool rows_in = (i0 ^ k0) < B16_B, cols_in = (j0 ^ k0) < B16_B;   // of the block (all 8, all 4)
     // (1) publish the column block and the row block
+    if (cols_in) {
 #pragma unroll
-    for (int a = 0; a < B16_RM; ++a)
-#pragma unroll
-      for (int c = 0; c < B16_RN; ++c) {
-        const int i = ty + B16_TY * a, j = tx + B16_TX * c;
-        if (i < n && j >= k0 && j < k0 + bs) Cb[i][j - k0] = m[a][c];
-        if (j < n && i >= k0 && i < k0 + bs) Rk[i - k0][j] = m[a][c];
+      for (int c = 0; c < 4; ++c) {
+        float4* d = reinterpret_cast<float4*>(&Cb[j0 - k0 + c][i0]);
+        d[0] = make_float4(m[0][c], m[1][c], m[2][c], m[3][c]);
+        d[1] = make_float4(m[4][c], m[5][c], m[6][c], m[7][c]);
       }
+    }
+    if (rows_in) {
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+        *reinterpret_cast<float4*>(&Rk[i0 - k0 + a][j0]) = make_float4(m[a][0], m[a][1], m[a][2], m[a][3]);
+    }
     __syncthreads();
-    // (2) the diagonal block by Gauss-Jordan on [M_kk | I] in warp 0: lane c
-    // holds column c of the 16 x 32 tableau in registers.  Per pivot, lane k
-    // scans its column for the largest unused row (the lowest such row on
-    // ties, a NaN taken as the largest) and every lane takes the pivot, the
-    // column-k factors and the pivot's reciprocal from lane k by shuffles,
-    // then eliminates its own column: no block barrier inside the 16 pivots.
+    // (2) the diagonal block by Gauss-Jordan in warp 0, lane r holding row r
+    // (a unit row beyond the matrix); the pivot is the largest of the rows not
+    // used yet, the lowest on ties, a NaN taken as the largest
     if (warp == 0) {
-      float t[B16_B];
+      float x[B16_B];
 #pragma unroll
-      for (int r = 0; r < B16_B; ++r) {
-        if (lane < B16_B) t[r] = (r < bs && lane < bs) ? Cb[k0 + r][lane] : (r == lane ? 1.f : 0.f);
-        else t[r] = (lane - B16_B == r) ? 1.f : 0.f;
-      }
-      unsigned used = 0;
+      for (int c = 0; c < B16_B; ++c)
+        x[c] = lane < bs && c < bs ? Cb[c][k0 + (lane & 15)] : (c == lane ? 1.f : 0.f);
       unsigned long long rows = 0;   // pivot row of step k in bits 4k .. 4k+3
-      int first_zero = -1;
+      int first_zero = -1, mine = -1;
 #pragma unroll 1
       for (int k = 0; k < B16_B; ++k) {
-        // largest unused |t| of the column, the lowest row on ties, as a
-        // tree (each merge keeps its lower half unless the upper is larger)
-        float bv[B16_B];
-        int bi[B16_B];
+        uint32_t key = pr_key(nan_to_inf(fabsf(x[0])), mine >= 0 || lane >= B16_B);
+        const int who = pr_best(key);
+        const float p = __shfl_sync(0xffffffffu, x[0], who), f = x[0];
+        const float pinv = key > 1u ? __frcp_rn(p) : 0.f;
 #pragma unroll
-        for (int r = 0; r < B16_B; ++r) {
-          float v = ((used >> r) & 1u) ? -1.f : fabsf(t[r]);
-          if (v != v) v = INFINITY;   // a NaN pivot is taken (and poisons the result) rather than skipped
-          bv[r] = v;
-          bi[r] = r;
+        for (int c = 1; c < B16_B; ++c) {
+          const float pv = __shfl_sync(0xffffffffu, x[c], who) * pinv;
+          x[c - 1] = lane == who ? pv : fmaf(-f, pv, x[c]);
         }
-#pragma unroll
-        for (int w = 1; w < B16_B; w <<= 1)
-#pragma unroll
-          for (int r = 0; r < B16_B; r += 2 * w)
-            if (bv[r + w] > bv[r]) {
-              bv[r] = bv[r + w];
-              bi[r] = bi[r + w];
-            }
-        const float best = __shfl_sync(0xffffffffu, bv[0], k);
-        const int who = __shfl_sync(0xffffffffu, bi[0], k);
-        float f[B16_B];
-#pragma unroll
-        for (int r = 0; r < B16_B; ++r) f[r] = __shfl_sync(0xffffffffu, t[r], k);
-        // t[who] and f[who] by a multiplexer tree on the bits of who
-        float mt[B16_B / 2], mf[B16_B / 2];
-#pragma unroll
-        for (int r = 0; r < B16_B / 2; ++r) {
-          mt[r] = (who & 1) ? t[2 * r + 1] : t[2 * r];
-          mf[r] = (who & 1) ? f[2 * r + 1] : f[2 * r];
-        }
-#pragma unroll
-        for (int w = 2, bit = 2; w <= B16_B / 2; w <<= 1, bit <<= 1)
-#pragma unroll
-          for (int r = 0; r < B16_B / 2; r += w) {
-            mt[r] = (who & bit) ? mt[r + w / 2] : mt[r];
-            mf[r] = (who & bit) ? mf[r + w / 2] : mf[r];
-          }
-        const float prow = mt[0], fk = mf[0];   // this column's entry in the pivot row; column k's
-        const float pinv = (best > 0.f) ? __frcp_rn(fk) : 0.f;
-        const float pv = prow * pinv;
-#pragma unroll
-        for (int r = 0; r < B16_B; ++r) t[r] = (r == who) ? pv : fmaf(-f[r], pv, t[r]);
-        used |= 1u << who;
+        x[B16_B - 1] = lane == who ? pinv : -(f * pinv);
+        if (lane == who) mine = k;
         rows |= (unsigned long long)who << (4 * k);
-        if (first_zero < 0 && !(best > 0.f) && k < bs) first_zero = k;
+        if (first_zero < 0 && key <= 1u && k < bs) first_zero = k;
       }
-      if (lane < B16_B) rowof_s[lane] = (int)((rows >> (4 * lane)) & 15ull);
       if (lane == 0 && first_zero >= 0 && s_info == 0) s_info = k0 + first_zero + 1;
+      // row r was the pivot of column `mine`: it holds row `mine` of the
+      // inverse, whose column piv(c) is x[c]
+      if (lane < B16_B)
 #pragma unroll
-      for (int r = 0; r < B16_B; ++r) Ag[0][r][lane] = t[r];
+        for (int c = 0; c < B16_B; ++c) Pk[mine][(int)((rows >> (4 * c)) & 15ull)] = x[c];
     }
     __syncthreads();
+    // (3) row `warp` of R = P M_k., and of P in the block's columns
     {
-      // the pivot row of column k holds row k of the inverse
-      const int r = tid >> 5, c = tid & 31;
-      if (r < bs && c < bs) Pk[r][c] = Ag[0][rowof_s[r]][B16_B + c];
-    }
-    __syncthreads();
-    // (3) R = P M_k. into registers of the threads that own those columns:
-    // thread (ty, tx) forms R[ty][j] for its columns j (bs <= 16 rows)
-    float r_new[B16_RN];
-    {
-      float prow[B16_B];
+      float r[4] = {0.f, 0.f, 0.f, 0.f};
+      if (warp < bs) {
 #pragma unroll
-      for (int d = 0; d < B16_B; ++d) prow[d] = (ty < bs && d < bs) ? Pk[ty][d] : 0.f;
-#pragma unroll
-      for (int c = 0; c < B16_RN; ++c) {
-        const int j = tx + B16_TX * c;
-        float acc = 0.f;
-        if (ty < bs && j < n) {
-#pragma unroll
-          for (int d = 0; d < B16_B; ++d)
-            if (d < bs) acc = fmaf(prow[d], Rk[d][j], acc);
+        for (int d = 0; d < B16_B; ++d) {
+          if (d >= bs) break;
+          const float pd = Pk[warp][d];
+          const float4 v = *reinterpret_cast<const float4*>(&Rk[d][j0]);
+          r[0] = fmaf(pd, v.x, r[0]);
+          r[1] = fmaf(pd, v.y, r[1]);
+          r[2] = fmaf(pd, v.z, r[2]);
+          r[3] = fmaf(pd, v.w, r[3]);
         }
-        r_new[c] = acc;
+        if (cols_in) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) r[c] = j0 + c < n ? Pk[warp][j0 - k0 + c] : 0.f;
+        }
       }
+      *reinterpret_cast<float4*>(&Rn[warp][j0]) = make_float4(r[0], r[1], r[2], r[3]);
     }
     __syncthreads();
+    // (4) rows of the block are R's; every other element is an outer-product
+    // update from the snapshots: M_ij = [j outside the block] M_ij - sum_d C_id R_dj
+    if (rows_in) {
 #pragma unroll
-    for (int c = 0; c < B16_RN; ++c) {
-      const int j = tx + B16_TX * c;
-      if (ty < bs && j < n) Rk[ty][j] = r_new[c];
-    }
-    __syncthreads();
-    // (4) every element as an outer-product update from the snapshots in
-    // shared memory: per d, the 8 column-block values of this thread's rows
-    // and the 4 values of the new row block (or of P, in the block's own
-    // columns) of its columns, each loaded once:
-    //     rows outside the block:  M_ij = [j outside] M_ij - sum_d C_id R'_dj
-    //     rows inside the block:   M_ij = R'_(i-k0) j
-    // with R' = R outside the block's columns and P inside them.
-#pragma unroll
-    for (int a = 0; a < B16_RM; ++a) {
-      const int i = ty + B16_TY * a;
-      const bool ib = i >= k0 && i < k0 + bs;
-#pragma unroll
-      for (int c = 0; c < B16_RN; ++c) {
-        const int j = tx + B16_TX * c;
-        if (ib || (j >= k0 && j < k0 + bs)) m[a][c] = 0.f;
+      for (int a = 0; a < 8; ++a) {
+        const float4 v = *reinterpret_cast<const float4*>(&Rn[i0 - k0 + a][j0]);
+        m[a][0] = v.x, m[a][1] = v.y, m[a][2] = v.z, m[a][3] = v.w;
       }
-    }
+    } else if (i0 < n) {
+      if (cols_in) {
 #pragma unroll
-    for (int d = 0; d < B16_B; ++d) {
-      if (d >= bs) break;
-      float cv[B16_RM], rv[B16_RN];
-#pragma unroll
-      for (int a = 0; a < B16_RM; ++a) {
-        const int i = ty + B16_TY * a;
-        cv[a] = (i < n && !(i >= k0 && i < k0 + bs)) ? Cb[i][d] : 0.f;
+        for (int a = 0; a < 8; ++a) m[a][0] = m[a][1] = m[a][2] = m[a][3] = 0.f;
       }
 #pragma unroll
-      for (int c = 0; c < B16_RN; ++c) {
-        const int j = tx + B16_TX * c;
-        rv[c] = (j >= n) ? 0.f : (j >= k0 && j < k0 + bs) ? Pk[d][j - k0] : Rk[d][j];
-      }
+      for (int d = 0; d < B16_B; ++d) {
+        if (d >= bs) break;
+        const float4 v = *reinterpret_cast<const float4*>(&Rn[d][j0]);
+        const float4 u0 = *reinterpret_cast<const float4*>(&Cb[d][i0]), u1 = *reinterpret_cast<const float4*>(&Cb[d][i0 + 4]);
+        const float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w}, w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int a = 0; a < B16_RM; ++a)
+        for (int a = 0; a < 8; ++a)
 #pragma unroll
-        for (int c = 0; c < B16_RN; ++c) m[a][c] = fmaf(-cv[a], rv[c], m[a][c]);
-    }
-#pragma unroll
-    for (int a = 0; a < B16_RM; ++a) {
-      const int i = ty + B16_TY * a;
-      if (!(i >= k0 && i < k0 + bs)) continue;
-#pragma unroll
-      for (int c = 0; c < B16_RN; ++c) {
-        const int j = tx + B16_TX * c;
-        if (j < n) m[a][c] = (j >= k0 && j < k0 + bs) ? Pk[i - k0][j - k0] : Rk[i - k0][j];
+          for (int c = 0; c < 4; ++c) m[a][c] = fmaf(-u[a], w[c], m[a][c]);
       }
     }
     __syncthreads();   // the next step overwrites Cb, Rk and Pk
@@ -1665,12 +1604,10 @@ inv_block16_kernel(int n, const float* __restrict__ A, long long lda, long long 
   if (tid == 0 && info) info[bb] = s_info;
   float* Xb = X + bb * sX;
 #pragma unroll
-  for (int a = 0; a < B16_RM; ++a)
+  for (int a = 0; a < 8; ++a)
 #pragma unroll
-    for (int c = 0; c < B16_RN; ++c) {
-      const int i = ty + B16_TY * a, j = tx + B16_TX * c;
-      if (i < n && j < n) Xb[(long long)i * ldx + j] = m[a][c];
-    }
+    for (int c = 0; c < 4; ++c)
+      if (i0 + a < n && j0 + c < n) Xb[(long long)(i0 + a) * ldx + j0 + c] = m[a][c];
 }
 
 static cudaError_t launch_block16(int n, const float* A, long long lda, long long sA, float* X, long long ldx,
