@@ -423,7 +423,7 @@ static cudaError_t run_groups(const GemmGroup* g, int ng, double alpha, const T*
   if constexpr (DTypeOf<T>::value == F64 || DTypeOf<T>::value == C128)
     return gemm_groups<T>(g, ng, alpha, A, lda, sA, B, ldb, sB, 1.0, add ? D : nullptr, ldd, sD, D, ldd, sD, batch, st);
   else
-    return cudaErrorNotSupported;
+    return gemm_groups_simt<T>(g, ng, make_scalar<T>(alpha, 0.0), A, lda, sA, B, ldb, sB, add, D, ldd, sD, batch, st);
 }
 
 template <class T>
@@ -486,9 +486,16 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   const long long sDD = (long long)ni * ni, sC = (long long)ni * ne, sB = (long long)ne * ni, sT = (long long)ne * ne;
   const bool rects = a->n_c_rects > 0 && a->n_b_rects > 0;
   GemmGroup groups[GEMM_GROUPS];
-  const bool digits = (DTypeOf<T>::value == F64 || DTypeOf<T>::value == C128) && f64_products_on_tensor_cores();
+  // FP64: on the digit kernel, or not at all.  FP32: where no block is long
+  // enough for the tensor cores' products (from 128 on), which are faster there.
+  bool grouped = f64_products_on_tensor_cores();
+  if (DTypeOf<T>::value == F32 || DTypeOf<T>::value == C64) {
+    grouped = !gemm_variant_forced();
+    for (int k = 0; rects_on && k < a->n_c_rects; ++k) grouped = grouped && a->c_rects[5 * k + 1] < 128;
+    for (int k = 0; rects_on && k < a->n_b_rects; ++k) grouped = grouped && a->b_rects[5 * k + 3] < 128;
+  }
   // S = -D^-1 C
-  int ng = rects && digits ? rect_groups(a, true, ni, groups) : 0;
+  int ng = rects && grouped ? rect_groups(a, true, ni, groups) : 0;
   if (ng) {
     HPS_CHECK(run_groups<T>(groups, ng, -1.0, D, ni, sDD, C, ne, sC, false, S, ne, sC, nm, st));
   } else if (rects) {
@@ -503,7 +510,7 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   // T_out = A + B S
   if (a->T_out) {
     T* To = (T*)a->T_out;
-    ng = rects && digits ? rect_groups(a, false, ne, groups) : 0;
+    ng = rects && grouped ? rect_groups(a, false, ne, groups) : 0;
     if (ng) {
       HPS_CHECK(run_groups<T>(groups, ng, 1.0, B, ni, sB, S, ne, sC, true, To, ne, sT, nm, st));
     } else if (rects) {
@@ -522,7 +529,7 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
     T* ho = (T*)a->h_out;
     const long long sg = (long long)ni * ns, sh = (long long)ne * ns;
     HPS_CHECK(gemm_batched<T>(ni, ns, ni, mone, D, ni, sDD, dh, ns, sg, zero_, nullptr, 0, 0, gt, ns, sg, nm, st));
-    ng = rects && (ns <= 8 || digits) ? rect_groups(a, false, ns, groups) : 0;
+    ng = rects && (ns <= 8 || grouped) ? rect_groups(a, false, ns, groups) : 0;
     if (ng && ns <= 8) {
       HPS_CHECK(skinny_groups<T>(groups, ng, ne, ns, B, ni, sB, gt, ns, sg, ho, ns, sh, nm, st));
     } else if (ng) {
@@ -541,7 +548,7 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   // B D^-1
   if (a->BD_inv) {
     T* BD = (T*)a->BD_inv;
-    ng = rects && digits ? rect_groups(a, false, ni, groups) : 0;
+    ng = rects && grouped ? rect_groups(a, false, ni, groups) : 0;
     if (ng) {
       HPS_CHECK(run_groups<T>(groups, ng, 1.0, B, ni, sB, D, ni, sDD, false, BD, ni, sB, nm, st));
     } else if (rects) {

@@ -783,6 +783,145 @@ HPS_SKINNY_GROUPS(double)
 HPS_SKINNY_GROUPS(c64)
 HPS_SKINNY_GROUPS(c128)
 
+// The groups' products in FP32 and complex64 (D = alpha A B, + D with `add`): a
+// CTA per tile of any group, K running through the group's segments in slices
+// of 16.  A block of its own per launch (4 to 17 us, 60 launches in a 2D merge
+// of five levels) left most SMs idle.
+struct SimtGroups {
+  int n, tiles;
+  GemmGroup g[GEMM_GROUPS];
+  int t0[GEMM_GROUPS];
+};
+
+template <class T, int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+gemm_groups_kernel(const __grid_constant__ SimtGroups gs, T alpha, const T* __restrict__ A, long long lda, long long sA,
+                   const T* __restrict__ B, long long ldb, long long sB, T* D, long long ldd, long long sD, int add_d) {
+  constexpr int BK = 16, NTX = BN / TN, NT = (BM / TM) * NTX, LA = BM * BK / NT, LB = BK * BN / NT;
+  __shared__ T As[2][BK][BM + 1];
+  __shared__ T Bs[2][BK][BN];
+  int gi = 0;
+  while (gi + 1 < gs.n && (int)blockIdx.x >= gs.t0[gi + 1]) ++gi;
+  const GemmGroup& g = gs.g[gi];
+  const int tn = (g.n + BN - 1) / BN, t = blockIdx.x - gs.t0[gi], m0 = t / tn * BM, n0 = t % tn * BN;
+  const long long bz = blockIdx.y;
+  A += bz * sA + (long long)(g.m0 + m0) * lda;
+  B += bz * sB + g.n0 + n0;
+  D += bz * sD + (long long)(g.m0 + m0) * ldd + g.n0 + n0;
+  const int M = g.m - m0, N = g.n - n0, tid = threadIdx.x, tx = tid % NTX, ty = tid / NTX;
+  T ra[LA], rb[LB];
+  auto load = [&](int seg, int k0) {   // slice k0 of a segment
+    const int off = g.k0[seg] + k0, left = g.len[seg] - k0;
+#pragma unroll
+    for (int l = 0; l < LA; ++l) {
+      const int e = tid + l * NT, r = e / BK, c = e % BK;
+      ra[l] = r < M && c < left ? A[(long long)r * lda + off + c] : zero<T>();
+    }
+#pragma unroll
+    for (int l = 0; l < LB; ++l) {
+      const int e = tid + l * NT, r = e / BN, c = e % BN;
+      rb[l] = r < left && c < N ? B[(long long)(off + r) * ldb + c] : zero<T>();
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int l = 0; l < LA; ++l) {
+      const int e = tid + l * NT;
+      As[buf][e % BK][e / BK] = ra[l];
+    }
+#pragma unroll
+    for (int l = 0; l < LB; ++l) {
+      const int e = tid + l * NT;
+      Bs[buf][e / BN][e % BN] = rb[l];
+    }
+  };
+  T acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = zero<T>();
+  int seg = 0, k0 = 0, buf = 0;
+  load(0, 0);
+  store(0);
+  __syncthreads();
+  while (true) {
+    k0 += BK;
+    if (k0 >= g.len[seg]) ++seg, k0 = 0;
+    const bool more = seg < g.segs;
+    if (more) load(seg, k0);
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      T a[TM], b[TN];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = As[buf][k][ty + i * (BM / TM)];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) b[j] = Bs[buf][k][tx + j * NTX];
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fma_(a[i], b[j], acc[i][j]);
+    }
+    if (!more) break;
+    buf ^= 1;
+    store(buf);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = ty + i * (BM / TM);
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int n = tx + j * NTX;
+      if (n >= N) continue;
+      T* d = D + (long long)m * ldd + n;
+      const T v = mul(alpha, acc[i][j]);
+      *d = add_d ? add(*d, v) : v;
+    }
+  }
+}
+
+template <class T>
+cudaError_t gemm_groups_simt(const GemmGroup* groups, int n, T alpha, const T* A, long long lda, long long sA, const T* B,
+                             long long ldb, long long sB, bool add_d, T* D, long long ldd, long long sD, int batch,
+                             cudaStream_t st) {
+  if (n < 1 || n > GEMM_GROUPS) return cudaErrorInvalidValue;
+  SimtGroups gs;
+  gs.n = n;
+  gs.tiles = 0;
+  int mm = 0, mn = 0;
+  for (int i = 0; i < n; ++i) mm = groups[i].m > mm ? groups[i].m : mm, mn = groups[i].n > mn ? groups[i].n : mn;
+  // blocks of up to 32 rows or columns: half as high or wide a tile
+  const int bm = mm <= 32 ? 32 : 64, bn = bm == 64 && mn <= 32 ? 32 : 64;
+  double flop = 0.0;
+  for (int i = 0; i < n; ++i) {
+    gs.g[i] = groups[i];
+    gs.t0[i] = gs.tiles;
+    gs.tiles += ((groups[i].m + bm - 1) / bm) * ((groups[i].n + bn - 1) / bn);
+    for (int k = 0; k < groups[i].segs; ++k) flop += 2.0 * groups[i].m * (double)groups[i].n * groups[i].len[k] * batch;
+  }
+  ProfScope ps(KC_GEMM, st, flop * (DTypeOf<T>::value == C64 ? 4.0 : 1.0));
+  for (int b0 = 0; b0 < batch; b0 += 65535) {
+    const int nb = batch - b0 < 65535 ? batch - b0 : 65535;
+    auto go = [&](auto kernel) {
+      note_launch();
+      kernel<<<dim3(gs.tiles, nb), 256, 0, st>>>(gs, alpha, A + b0 * sA, lda, sA, B + b0 * sB, ldb, sB, D + b0 * sD, ldd, sD,
+                                                 (int)add_d);
+    };
+    if (bm == 32)
+      go(gemm_groups_kernel<T, 32, 64, 2, 4>);
+    else if (bn == 32)
+      go(gemm_groups_kernel<T, 64, 32, 4, 2>);
+    else
+      go(gemm_groups_kernel<T, 64, 64, 4, 4>);
+  }
+  return cudaGetLastError();
+}
+template cudaError_t gemm_groups_simt<float>(const GemmGroup*, int, float, const float*, long long, long long, const float*,
+                                             long long, long long, bool, float*, long long, long long, int, cudaStream_t);
+template cudaError_t gemm_groups_simt<c64>(const GemmGroup*, int, c64, const c64*, long long, long long, const c64*,
+                                           long long, long long, bool, c64*, long long, long long, int, cudaStream_t);
+
 // Which products run on the tensor cores (gemm_tc.cu, gemm_f64_tc.cu): 0 none,
 // 1 the shapes where they were measured faster (default), 2 every product,
 // 3 none and the FP32 8x8 tiles with 4-byte shared loads (gemm_kernel) in
@@ -849,6 +988,8 @@ void gemm_tune_clear() {
   g_tune.clear();
   g_tune_size.store(0);
 }
+
+bool gemm_variant_forced() { return g_force_variant.load() >= 0; }
 
 int gemm_force_variant(int variant) {
   if (variant >= GV_COUNT) return -2;

@@ -95,6 +95,11 @@ template <class T>
 cudaError_t gemm_groups(const GemmGroup* groups, int n, double alpha, const T* A, long long lda, long long sA, const T* B,
                         long long ldb, long long sB, double beta, const T* C, long long ldc, long long sC, T* D,
                         long long ldd, long long sD, int batch, cudaStream_t st);
+// The same for T = float or c64 in multiply-adds (gemm.cu), D = alpha A B (+ D).
+template <class T>
+cudaError_t gemm_groups_simt(const GemmGroup* groups, int n, T alpha, const T* A, long long lda, long long sA, const T* B,
+                             long long ldb, long long sB, bool add_d, T* D, long long ldd, long long sD, int batch,
+                             cudaStream_t st);
 // D += A B for the rows of the groups (their n0 and n are not used) and N <= 8
 // columns, any type (gemm.cu); M rows in all.
 template <class T>
@@ -146,6 +151,7 @@ int set_inverse_tc_policy(int policy);
 int gemm_tune_set(int M, int N, int K, int batch, int variant);
 void gemm_tune_clear();
 int gemm_force_variant(int variant);
+bool gemm_variant_forced();
 long long gemm_shapes(int mode, long long* out, long long cap);
 // Whether that policy lets FP64 products use the tensor cores.
 bool f64_products_on_tensor_cores();

@@ -69,3 +69,31 @@ def test_grouped_rows_of_right_hand_sides(cuda, monkeypatch, dtype, ns):
     eps = torch.finfo(dtype).eps
     for a, b in zip(*out):
         assert float((a - b).abs().max()) <= 8 * maps.n_int * eps * float(b.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.complex64])
+@pytest.mark.parametrize("kind,q,nm", [("2d", 2, 3), ("2d", 7, 300), ("2d", 14, 2), ("2d", 33, 2), ("2d", 64, 1), ("2d", 127, 1),
+                                       ("2d", 128, 1), ("3d", 3, 5), ("3d", 5, 2), ("3d", 11, 1)])
+def test_grouped_fp32_products_match_the_dense_ones(cuda, monkeypatch, dtype, kind, q, nm):
+    """gemm_groups_kernel's three tiles, partial slices of 16 and segments side by
+    side, and blocks of 128 that stay with the single products.  The same D^-1
+    either way; S and T_out differ by the order of K <= 4 q (3D 12 q^2) terms:
+    K eps of the largest entry, 4 for the sums of magnitudes over it."""
+    iti = dtype.is_complex
+    if iti and kind == "3d":
+        pytest.skip("impedance merges are two-dimensional")
+    maps = oct_merge_maps_dtn(q * q) if kind == "3d" else quad_merge_maps_iti(q) if iti else quad_merge_maps_dtn(q)
+    rng = np.random.default_rng(q)
+    shape = (nm * maps.nch, maps.nb, maps.nb)
+    T = rng.standard_normal(shape) / maps.nb
+    T = 0.3 * (T + 1j * rng.standard_normal(shape) / maps.nb) if iti else T + 4.0 * np.eye(maps.nb)
+    T = torch.as_tensor(T, device=cuda).to(dtype)
+    out = []
+    for rects in (True, False):
+        monkeypatch.setattr(st, "_RECTS", rects)
+        r = st.merge_level_dtn(T, None, maps, keep_D_inv=True, keep_BD_inv=True, iti=iti)
+        out.append((r[0], r[2], r[4], r[5]))
+    assert torch.equal(out[0][2], out[1][2])
+    eps = torch.finfo(dtype).eps
+    for a, b in zip(*out):
+        assert float((a - b).abs().max()) <= 4 * maps.n_int * eps * float(b.abs().max())
