@@ -490,7 +490,7 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   // enough for the tensor cores' products (from 128 on), which are faster there.
   bool grouped = f64_products_on_tensor_cores();
   if (DTypeOf<T>::value == F32 || DTypeOf<T>::value == C64) {
-    grouped = !gemm_variant_forced();
+    grouped = gemm_simt_blocks();
     for (int k = 0; rects_on && k < a->n_c_rects; ++k) grouped = grouped && a->c_rects[5 * k + 1] < 128;
     for (int k = 0; rects_on && k < a->n_b_rects; ++k) grouped = grouped && a->b_rects[5 * k + 3] < 128;
   }

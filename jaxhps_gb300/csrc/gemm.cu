@@ -989,7 +989,7 @@ void gemm_tune_clear() {
   g_tune_size.store(0);
 }
 
-bool gemm_variant_forced() { return g_force_variant.load() >= 0; }
+bool gemm_simt_blocks() { return g_force_variant.load() < 0 && gemm_policy() != 2; }
 
 int gemm_force_variant(int variant) {
   if (variant >= GV_COUNT) return -2;

@@ -151,7 +151,9 @@ int set_inverse_tc_policy(int policy);
 int gemm_tune_set(int M, int N, int K, int batch, int variant);
 void gemm_tune_clear();
 int gemm_force_variant(int variant);
-bool gemm_variant_forced();
+// Whether FP32 products may be grouped on the SIMT tiles: no variant forced, no
+// policy that sends every product to the tensor cores.
+bool gemm_simt_blocks();
 long long gemm_shapes(int mode, long long* out, long long cap);
 // Whether that policy lets FP64 products use the tensor cores.
 bool f64_products_on_tensor_cores();
