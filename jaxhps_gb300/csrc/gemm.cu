@@ -1068,7 +1068,7 @@ bool f64_products_on_tensor_cores() {
 
 // FP64 and complex128 products: digits on the tensor cores (gemm_f64_tc.cu)
 // against the FP64 pipe.  From K = 16 on the digits win at every size measured
-// (one 16^3 product 18 against 26 us, 4096 of 196 x 56 x 196 in 1.34 against
+// (one 16^3 product 18 against 26 us, 4096 of 196 x 56 x 196 in 1.42 against
 // 21.6 ms, 224^3 x 1024 in 1.45 against 24.2 ms), below it with a million
 // outputs or more (112 x 112 x 4 x 256 50 against 75 us, x 16 23 against 20).  Products
 // with N <= 8 columns read A once either way and their FP64 time grows with N,

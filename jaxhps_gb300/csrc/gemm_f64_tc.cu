@@ -20,12 +20,15 @@
 // factors meet small ones keeps the bound K 2^-56 max|a_i| max|b_j| only:
 // callers bring rows of such operands to one scale first (leaf_dtn_impl).
 //
-// Measured (FP64 chain before, digits): 4096 x (196 x 56 x 196) 21.6 -> 1.34 ms
-// (13.2 TFLOP/s), 512 x (512 x 384 x 512) 82.7 -> 4.5 ms (22.7), 1792^3 10.7
-// -> 0.56 ms, complex 1024 x (256 x 56 x 256) 27.6 -> 1.54 ms, 4096 x (196 x 8 x
-// 196) 4.4 -> 0.94 ms.  The tensor pipe is busy 40% of the large product's
-// time: the conversion (about 24 integer operations an element on the
-// half-rate ALU, A once per 64 columns) bounds it.
+// Measured (FP64 chain before, digits): 4096 x (196 x 56 x 196) 21.6 -> 1.42 ms
+// (12.4 TFLOP/s), 512 x (512 x 384 x 512) 82.7 -> 4.8 ms (21.4), 1792^3 10.7
+// -> 0.60 ms, complex 1024 x (256 x 56 x 256) 27.6 -> 1.58 ms, 4096 x (196 x 8 x
+// 196) 4.4 -> 0.94 ms.  Of the 50,000 cycles of a 196 x 56 x 196 tile the
+// converting warps spend 20,000 converting (about 24 integer operations an
+// element on the half-rate ALU, A once per 64 columns) and 18,000 issuing the
+// copies of their operands; with K = 64 and less the reading warps bound it:
+// 14,700 cycles a tile to round its sums and write D, 7,700 to read the
+// accumulators.  (A bulk copy per row of an operand: five times slower.)
 #include "hps_common.cuh"
 #include "hps_internal.h"
 #include "digits.cuh"

@@ -115,7 +115,7 @@ __global__ void interp_from_leaves_kernel(long long n_t, int nsrc, const double*
     if (leaf < 0) leaf = 0;
     // 1D barycentric factors on the leaf's nodes: 1 / (w d), times 1 / their sum
     // (one division a node: they are most of the FP64 work, 512 x 512 targets
-    // at p = 16 took 0.56 ms with two, and the tensor sum below without its
+    // at p = 16 took 0.56 ms with two, 0.32 now; and the tensor sum below without its
     // inner sums twice the multiply-adds)
     double fac[3][IP_MAXP];
     for (int a = 0; a < DIM; ++a) {

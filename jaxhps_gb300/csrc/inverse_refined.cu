@@ -21,7 +21,7 @@
 //
 // Why: elimination is a chain of n dependent pivots.  Its panels are bound by
 // the FP64 pipe (two multiply-adds per SM and clock) for many matrices and by
-// the pivot exchange for few (6.6 us a column on a 16-CTA cluster), and its
+// the pivot exchange for few (3.3 us a column on a cluster), and its
 // rank-32 updates read and write the whole matrix n / 32 times; the products
 // of size n do not wait for one another's columns.
 // A matrix whose second residual is not small (or whose single-precision
