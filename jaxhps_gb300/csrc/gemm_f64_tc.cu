@@ -20,15 +20,16 @@
 // factors meet small ones keeps the bound K 2^-56 max|a_i| max|b_j| only:
 // callers bring rows of such operands to one scale first (leaf_dtn_impl).
 //
-// Measured (FP64 chain before, digits): 4096 x (196 x 56 x 196) 21.6 -> 1.42 ms
-// (12.4 TFLOP/s), 512 x (512 x 384 x 512) 82.7 -> 4.8 ms (21.4), 1792^3 10.7
-// -> 0.60 ms, complex 1024 x (256 x 56 x 256) 27.6 -> 1.58 ms, 4096 x (196 x 8 x
-// 196) 4.4 -> 0.94 ms.  Of the 50,000 cycles of a 196 x 56 x 196 tile the
-// converting warps spend 20,000 converting (about 24 integer operations an
-// element on the half-rate ALU, A once per 64 columns) and 18,000 issuing the
-// copies of their operands; with K = 64 and less the reading warps bound it:
-// 14,700 cycles a tile to round its sums and write D, 7,700 to read the
-// accumulators.  (A bulk copy per row of an operand: five times slower.)
+// Measured (FP64 chain before, digits): 4096 x (196 x 56 x 196) 21.6 -> 1.22 ms
+// (14.5 TFLOP/s), 512 x (512 x 384 x 512) 82.7 -> 4.2 ms (24.5), 1792^3 10.7
+// -> 0.54 ms, complex 1024 x (256 x 56 x 256) 27.6 -> 1.45 ms, 4096 x (196 x 8 x
+// 196) 4.4 -> 0.86 ms (1.42, 4.8, 0.60, 1.58 and 0.94 without tensor maps).  The
+// conversion bounds long products (about 24 integer operations an element on
+// the half-rate ALU, A once per 64 columns: 20,000 cycles of a 196 x 56 x 196
+// tile); with K = 64 and less the reading warps do: 14,700 cycles a tile to
+// round its sums and write D, 7,700 to read the accumulators.
+#include <cuda.h>
+
 #include "hps_common.cuh"
 #include "hps_internal.h"
 #include "digits.cuh"
@@ -51,18 +52,25 @@ constexpr int OZ_NT = (OZ_MW + 4) * 32;
 constexpr int OZ_EB = 8;                 // tiles whose exponents are kept (up to NS + 3 are in use)
 constexpr int OZ_APL = OZ_BM * 32;       // bytes of one digit plane of A
 
-template <int BN>
+template <int BN, bool TMA = false>
 struct OzCfg {
   static constexpr int BPL = BN * 32;                       // bytes of one digit plane of B
   static constexpr int STAGE = OZ_SL * (OZ_APL + BPL);      // digits of 16 steps of K
   static constexpr int RAW = (OZ_BM + BN) * OZ_BK * 8;      // the same as FP64
-  static constexpr int NS = 3;                              // digit stages
-  static constexpr int NR = (BN <= 16) ? 5 : 3;             // FP64 stages (NR - 1 in flight)
+  static constexpr int NS = (TMA && BN > 16) ? 2 : 3;       // digit stages
+  static constexpr int NR = (TMA || BN <= 16) ? 5 : 3;      // FP64 stages (NR - 1 in flight)
   static constexpr size_t SMEM = (size_t)NS * STAGE + (size_t)NR * RAW + 1024;
   static constexpr int COLS = OZ_SL * BN;                   // TMEM columns: one block of BN per weight
   static constexpr int CW = BN / 2;                         // output columns per reading thread
   static constexpr int KB = BN * OZ_BK / OZ_CT;             // B values per converting thread and stage
 };
+
+__device__ __forceinline__ void load_box(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
 
 // Asynchronous copies of 16 or 8 bytes; `in` false writes zeros and reads nothing.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in) {
@@ -99,6 +107,15 @@ struct OzGroups {
 };
 template <>
 struct OzGroups<false> {};
+
+// Tensor maps of A and B as FP32 pairs, and whether each has a batch.
+template <bool TMA>
+struct OzMaps {
+  CUtensorMap a, b;
+  int a_batched, b_batched;
+};
+template <>
+struct OzMaps<false> {};
 
 // One tile: its matrix of the batch, its first row and column (inside the
 // group), and the group.
@@ -156,13 +173,19 @@ __device__ __noinline__ double plain_entry(const OzArgs& p, const double* A, con
 // its tensor memory.
 // GROUP: the products of all groups at once, K running through a group's
 // segments one after another (each one's last stage filled up with zeros).
-template <int BN, bool CPLX, bool SKIP, bool GROUP>
-__global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const __grid_constant__ OzGroups<GROUP> gs) {
-  using Cfg = OzCfg<BN>;
+// TMA: warp 17 brings the FP64 stages, a box of A (128 rows of 16, 128-byte
+// swizzled) and one of B each (`rfull`, `rempty`; 16-byte aligned rows and
+// matrices).  With each converting warp issuing its own cp.async of 16 and 8
+// bytes, those took 700 cycles of every step, 18,000 of the 50,000 of a 196 x
+// 56 x 196 tile; a bulk copy per row takes 9,000 a step.
+template <int BN, bool CPLX, bool SKIP, bool GROUP, bool TMA>
+__global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const __grid_constant__ OzGroups<GROUP> gs, const __grid_constant__ OzMaps<TMA> maps) {
+  using Cfg = OzCfg<BN, TMA>;
+  static_assert(!(TMA && GROUP), "segments end where their neighbours begin");
   constexpr int NS = Cfg::NS, NR = Cfg::NR, CW = Cfg::CW, KB = Cfg::KB;
   extern __shared__ unsigned char oz_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(oz_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t full[NS], empty[NS], accf[2], acce[2], expo[OZ_EB];
+  __shared__ uint64_t full[NS], empty[NS], accf[2], acce[2], expo[OZ_EB], rfull[NR], rempty[NR];
   __shared__ uint32_t committed[NS], acc_committed[2];
   __shared__ short row_e[OZ_EB][OZ_BM], col_e[OZ_EB][BN];
   __shared__ uint2 col_part[2][OZ_CT];
@@ -182,6 +205,10 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const
       acc_committed[i] = 0;
     }
     for (int i = 0; i < OZ_EB; ++i) mbar_init(&expo[i], OZ_CW);
+    for (int i = 0; i < NR; ++i) {
+      mbar_init(&rfull[i], 1);
+      mbar_init(&rempty[i], OZ_CW);
+    }
     fail_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -366,7 +393,8 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const
     }
   } else if (warp < OZ_MW) {
     // ---------------- FP64 -> exponents, digit planes ----------------
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+    if constexpr (TMA) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
     const int ct = tid - OZ_DW * 32, cw = ct >> 5;
     const int ar = ct >> 1, ah = ct & 1;                // A: one row, steps 8 ah .. 8 ah + 7
     const int bn = ct % BN, bk = (ct / BN) * KB;        // B: one column, KB steps
@@ -403,7 +431,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const
         lB += (long long)gs.g[t.g].k0[lseg] * p.ldb;
       }
     };
-    if (lu < n_units) segment_ptrs();
+    if (!TMA && lu < n_units) segment_ptrs();
     const double* safe = p.A;   // an address for copies that read nothing
     auto copy_stage = [&]() {
       if (lu < n_units) {
@@ -462,17 +490,50 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    if constexpr (!TMA) {
 #pragma unroll
-    for (int i = 0; i < NR - 1; ++i) copy_stage();
+      for (int i = 0; i < NR - 1; ++i) copy_stage();
+    }
     int slot = 0;
+    uint32_t round = 0;   // of the ring (TMA)
     // the next FP64 stage, and the copy into the slot read before it
-    auto next_raw = [&]() {
+    auto next_raw = [&]() -> const unsigned char* {
+      if constexpr (TMA) {
+        wait(&rfull[slot], round & 1);
+        return smem + NS * Cfg::STAGE + slot * Cfg::RAW;
+      }
       asm volatile("cp.async.wait_group %0;" ::"n"(NR - 2) : "memory");
       __syncwarp();   // the warp's copies are visible to all of its lanes, and all have read the slot refilled next
       const unsigned char* rw = raw + slot * Cfg::RAW;
       slot = slot + 1 == NR ? 0 : slot + 1;
       copy_stage();
       return rw;
+    };
+    // this warp has read the stage
+    auto raw_done = [&]() {
+      if constexpr (TMA) {
+        // the lanes' loads, which may still be on their way, before the next box's
+        // write (without this fence a few rows and columns per thousand short
+        // tiles took their exponents from the box after)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&rempty[slot]);
+        if (++slot == NR) slot = 0, ++round;
+      }
+    };
+    // two of the thread's values of A and one of B
+    auto raw_a = [&](const unsigned char* rw, int i) {
+      const unsigned char* r = TMA ? rw + ar * 128 : rw + rr * 128;   // (ar mod 8 = rr mod 8)
+      return *reinterpret_cast<const uint4*>(r + (((4 * ah + i) ^ (rr & 7)) << 4));
+    };
+    auto raw_b = [&](const unsigned char* rw, int i) {
+      if constexpr (TMA) {
+        const int k = bk + i;
+        const unsigned char* b = rw + OZ_BM * 128;
+        return CPLX ? *reinterpret_cast<const uint2*>(b + (k >> 1) * (BN * 8) + ((bn & ~1) + ((k + bn) & 1)) * 8)
+                    : *reinterpret_cast<const uint2*>(b + k * (BN * 8) + bn * 8);
+      }
+      return *reinterpret_cast<const uint2*>(rw + 16 * 128 + i * 256 + lane * 8);
     };
     // 0x7ff for a row or column that cannot be scaled (infinities, NaN, or nothing but tiny values)
     auto code = [](uint32_t top, uint32_t low) {
@@ -490,16 +551,17 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const
           const unsigned char* rw = next_raw();
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const uint4 v = *reinterpret_cast<const uint4*>(rw + rr * 128 + (((4 * ah + i) ^ (rr & 7)) << 4));
+            const uint4 v = raw_a(rw, i);
             at = max(at, max(v.y & 0x7fffffffu, v.w & 0x7fffffffu));
             al |= v.x | v.z;
           }
 #pragma unroll
           for (int i = 0; i < KB; ++i) {
-            const uint2 v = *reinterpret_cast<const uint2*>(rw + 16 * 128 + i * 256 + lane * 8);
+            const uint2 v = raw_b(rw, i);
             bt = max(bt, v.y & 0x7fffffffu);
             bl |= v.x;
           }
+          raw_done();
         }
         at = max(at, __shfl_xor_sync(0xffffffffu, at, 1));
         al |= __shfl_xor_sync(0xffffffffu, al, 1);
@@ -532,7 +594,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const
           uint32_t x[16], one[4], off[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const uint4 v = *reinterpret_cast<const uint4*>(rw + rr * 128 + (((4 * ah + i) ^ (rr & 7)) << 4));
+            const uint4 v = raw_a(rw, i);
             x[4 * i] = v.x, x[4 * i + 1] = v.y, x[4 * i + 2] = v.z, x[4 * i + 3] = v.w;
           }
 #pragma unroll
@@ -563,10 +625,11 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const
           uint32_t one[PB], off[PB];
 #pragma unroll
           for (int i = 0; i < KB; ++i) {
-            x[i] = *reinterpret_cast<const uint2*>(rw + 16 * 128 + i * 256 + lane * 8);
+            x[i] = raw_b(rw, i);
             // real view of a complex column: rows 2k, 2k + 1 are (re, -im) or (im, re)
             if (CPLX && ((bk + i) & 1) && !(bn & 1)) x[i].y ^= 0x80000000u;
           }
+          raw_done();
           if constexpr (KB == 1) x[1] = x[0];
 #pragma unroll
           for (int i = 0; i < PB; ++i) sign_pair(x[2 * i].y, x[2 * i + 1].y, one[i], off[i]);
@@ -604,7 +667,38 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
     // ---------------- MMA issuer ----------------
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    if constexpr (TMA) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    if constexpr (TMA) {
+      if (warp == OZ_MW + 1) {
+        // ---------------- copies ----------------
+        constexpr uint32_t BYTES = OZ_BM * 128 + (CPLX ? OZ_BK / 2 : OZ_BK) * BN * 8;
+        int s = 0;
+        uint32_t it = 0;
+        for (long long u = u0; u < n_units && ok; u = tile_from(u + gridDim.x)) {
+          const OzTile t = tile_of(u);
+          const int za = maps.a_batched ? (int)t.b : 0, zb = maps.b_batched ? (int)t.b : 0;
+          for (int k = 0; k < 2 * nk_all; ++k, ++it) {
+            const int k0 = (k < nk_all ? k : k - nk_all) * OZ_BK;
+            if (it >= NR) wait(&rempty[s], (it / NR - 1) & 1);
+            if (!ok) break;
+            if (lane == 0) {
+              const uint32_t dst = smem_u32(smem + NS * Cfg::STAGE + s * Cfg::RAW);
+              asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&rfull[s])), "r"(BYTES)
+                           : "memory");
+              load_box(dst, &maps.a, 2 * k0, t.m0, za, &rfull[s]);
+              load_box(dst + OZ_BM * 128, &maps.b, 2 * t.n0, CPLX ? k0 / 2 : k0, zb, &rfull[s]);
+            }
+            __syncwarp();
+            s = s + 1 == NR ? 0 : s + 1;
+          }
+        }
+        if (!ok) {   // a second bounded chance for the copies in flight
+          for (int i = 0; i < NR; ++i)
+            if (it > (uint32_t)i) tc::mbar_wait(&rfull[i], ((it - 1 - i) / NR) & 1, limit);
+        }
+      }
+    }
     if (warp == OZ_MW) {
       uint32_t it = 0, ch = 0;
       int s = 0;
@@ -663,20 +757,20 @@ __global__ void __launch_bounds__(OZ_NT, 1) gemm_oz_kernel(const OzArgs p, const
   }
 }
 
-template <int BN, bool CPLX, bool SKIP, bool GROUP = false>
-cudaError_t launch_oz(OzArgs p, cudaStream_t st, const OzGroups<GROUP>& gs = {}) {
-  using Cfg = OzCfg<BN>;
+template <int BN, bool CPLX, bool SKIP, bool GROUP = false, bool TMA = false>
+cudaError_t launch_oz(OzArgs p, cudaStream_t st, const OzGroups<GROUP>& gs = {}, const OzMaps<TMA>& maps = {}) {
+  using Cfg = OzCfg<BN, TMA>;
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(gemm_oz_kernel<BN, CPLX, SKIP, GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+    e = cudaFuncSetAttribute(gemm_oz_kernel<BN, CPLX, SKIP, GROUP, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
   if (e == cudaSuccess) e = tc_wait_state(&p.err, &p.limit);
   if (e != cudaSuccess) return e;
   long long units = (long long)p.batch * ((p.M + OZ_BM - 1) / OZ_BM) * ((p.N + BN - 1) / BN);
   if constexpr (GROUP) units = (long long)p.batch * gs.tiles;
   note_launch();
-  gemm_oz_kernel<BN, CPLX, SKIP, GROUP><<<(unsigned)(units < sms ? units : sms), OZ_NT, Cfg::SMEM, st>>>(p, gs);
+  gemm_oz_kernel<BN, CPLX, SKIP, GROUP, TMA><<<(unsigned)(units < sms ? units : sms), OZ_NT, Cfg::SMEM, st>>>(p, gs, maps);
   return cudaGetLastError();
 }
 
@@ -693,6 +787,23 @@ static cudaError_t gemm_oz(int M, int N, int K, double alpha, const double* A, l
             (!C || (al16(C) && ldc % 2 == 0 && (batch == 1 || sC % 2 == 0)));
   ProfScope ps(KC_GEMM, st, 2.0 * M * (double)N * K * batch * (CPLX ? 2.0 : 1.0));
   if (skip) return launch_oz<64, CPLX, true>(p, st);
+  // A tile per SM and more: the two tensor maps cost the host some 2 us a launch,
+  // which the few tiles of a smaller product do not win back (256 leaves of 13^2
+  // took 3.81 ms with maps everywhere, 3.78 without any).
+  const long long tiles = (long long)batch * ((M + OZ_BM - 1) / OZ_BM) * ((N + 63) / 64);
+  if (tiles >= 152 && p.vec_a && al16(B) && ldb % 2 == 0 && (batch == 1 || sB % 2 == 0)) {
+    // FP64 numbers as FP32 pairs; boxes reach over the edges into zeros
+    OzMaps<true> m;
+    m.a_batched = batch > 1 && sA != 0;
+    m.b_batched = batch > 1 && sB != 0;
+    const int bn = N <= 16 ? 16 : 64;
+    if (tma_map_f32(&m.a, reinterpret_cast<const float*>(A), 2ll * K, M, m.a_batched ? batch : 1, 2 * lda, 2 * sA, 2 * OZ_BK,
+                    OZ_BM, true) &&
+        tma_map_f32(&m.b, reinterpret_cast<const float*>(B), 2ll * N, CPLX ? K / 2 : K, m.b_batched ? batch : 1, 2 * ldb, 2 * sB,
+                    2 * bn, CPLX ? OZ_BK / 2 : OZ_BK, false))
+      return bn == 16 ? launch_oz<16, CPLX, false, false, true>(p, st, {}, m)
+                      : launch_oz<64, CPLX, false, false, true>(p, st, {}, m);
+  }
   if (N <= 16) return launch_oz<16, CPLX, false>(p, st);
   return launch_oz<64, CPLX, false>(p, st);
 }

@@ -177,3 +177,27 @@ def test_few_columns_either_way(policy, N):
         out.append(D)
     scale = At.abs() @ Bt.abs()
     assert float(((out[0] - out[1]).abs() / scale).max()) <= 196 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("M,N,K,batch,pad", [(196, 196, 4, 256, 0), (196, 196, 16, 256, 0), (196, 196, 32, 256, 0),
+                                             (130, 10, 20, 400, 0), (196, 196, 16, 256, 1), (128, 64, 17, 400, 3)])
+def test_many_short_tiles_with_a_c(policy, M, N, K, batch, pad, cplx):
+    """Several tiles a CTA whose operands wait in the ring while sums are rounded
+    and C is read, every matrix of the batch and several runs: even and odd rows
+    (tensor-map boxes and single copies).  Against torch's FP64 product: K + 2
+    roundings of the sum of the magnitudes on its side, 2^-56 of the row's and
+    column's largest per step here, both below 2 (K + 2) 2^-53 of the bound."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    dt = torch.complex128 if cplx else torch.float64
+    A, B, C = (torch.randn((batch, m, n + pad), dtype=dt, device="cuda", generator=g)[..., :n]
+               for m, n in ((M, K), (K, N), (M, N)))
+    ref = A @ B + C
+    am = A.abs().amax(-1, keepdim=True)
+    bm = B.abs().amax(-2, keepdim=True)
+    tol = 2 * (K + 2) * 2.0 ** -53 * (4 if cplx else 1) * (K * am * bm + C.abs())
+    policy(ALL)
+    for _ in range(3):
+        D = C.clone()
+        nat.gemm(A, B, D, 1.0, 1.0, Cmat=D)
+        assert bool(((D - ref).abs() <= tol).all())
