@@ -246,10 +246,14 @@ def interp_to_hps_2D(leaf_bounds, samples, p: int, from_x, from_y, device=None, 
     samples (n_x, n_y) given on meshgrid(from_x, from_y, indexing='ij')
     (reference interp_to_single_Chebyshev_panel_2D, :228-263, vmapped)."""
     ax = [np.asarray(a.cpu() if isinstance(a, torch.Tensor) else a, dtype=np.float64) for a in (from_x, from_y)]
-    return st._to_host(_to_hps(_leaf_bounds(leaf_bounds), samples, p, ax, device), host_device)
+    out = st._to_host(_to_hps(_leaf_bounds(leaf_bounds), samples, p, ax, device), host_device)
+    nat.raise_on_tc_timeout("interp_to_hps_2D")
+    return out
 
 
 def interp_to_hps_3D(leaf_bounds, samples, p: int, from_x, from_y, from_z, device=None, host_device="cpu"):
     """3D analogue (reference :271-302): samples (n_x, n_y, n_z)."""
     ax = [np.asarray(a.cpu() if isinstance(a, torch.Tensor) else a, dtype=np.float64) for a in (from_x, from_y, from_z)]
-    return st._to_host(_to_hps(_leaf_bounds(leaf_bounds), samples, p, ax, device), host_device)
+    out = st._to_host(_to_hps(_leaf_bounds(leaf_bounds), samples, p, ax, device), host_device)
+    nat.raise_on_tc_timeout("interp_to_hps_3D")
+    return out

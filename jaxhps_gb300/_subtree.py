@@ -6,13 +6,16 @@ leave a small device memory: it merges each subtree to its root, merges the
 roots, and during the solve recomputes every subtree.  A GB300 keeps the
 whole operator set of such problems in HBM, so here the three entry points
 keep their signatures and results but run the ordinary build (all levels in
-HBM, no recomputation); ``subtree_height`` is accepted and ignored.
+HBM, no recomputation); ``subtree_height`` is accepted and ignored.  As
+build_solver and solve do, each checks the leaf inverses' status words and the
+tensor-core products' timeout flag before it returns.
 """
 
 from __future__ import annotations
 
 import torch
 
+from . import _native as nat
 from . import _stages as st
 
 
@@ -31,6 +34,7 @@ def _build(pde_problem, compute_device, return_T):
     else:
         Y, T, v, h = st.local_solve_stage_uniform_2D_DtN(pde_problem, device=compute_device)
         out = st.merge_stage_uniform_2D_DtN(T, h, l=dom.L, device=compute_device, return_T=return_T)
+    st.check_infos([pde_problem._leaf_info], "leaf inverse")
     return Y, v, out
 
 
@@ -50,7 +54,9 @@ def solve_subtree(pde_problem, boundary_data, subtree_height: int = 7, compute_d
     on the problem (_subtree_recomp.py:20-163)."""
     _check(pde_problem)
     Y, v, out = _build(pde_problem, compute_device, False)
-    return _down(pde_problem, boundary_data, out[0], out[1], Y, v, compute_device, host_device)
+    u = _down(pde_problem, boundary_data, out[0], out[1], Y, v, compute_device, host_device)
+    nat.raise_on_tc_timeout("solve_subtree")
+    return u
 
 
 def upward_pass_subtree(pde_problem, subtree_height: int = 7, compute_device=None, host_device="cpu"):
@@ -58,6 +64,7 @@ def upward_pass_subtree(pde_problem, subtree_height: int = 7, compute_device=Non
     top-level Poincare-Steklov matrix (_subtree_recomp.py:395-456)."""
     _check(pde_problem)
     Y, v, out = _build(pde_problem, compute_device, True)
+    nat.raise_on_tc_timeout("upward_pass_subtree")
     pde_problem.S_lst, pde_problem.g_tilde_lst = out[0], out[1]
     pde_problem._subtree_leaf_ops = (Y, v)
     return st._to_host(out[2], host_device)
@@ -71,5 +78,7 @@ def downward_pass_subtree(pde_problem, boundary_data, subtree_height: int = 7, c
     if ops is None:
         raise ValueError("downward_pass_subtree needs upward_pass_subtree first")
     Y, v = ops
-    return _down(pde_problem, boundary_data, pde_problem.S_lst, pde_problem.g_tilde_lst, Y, v, compute_device,
-                 host_device)
+    u = _down(pde_problem, boundary_data, pde_problem.S_lst, pde_problem.g_tilde_lst, Y, v, compute_device,
+              host_device)
+    nat.raise_on_tc_timeout("downward_pass_subtree")
+    return u
