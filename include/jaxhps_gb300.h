@@ -49,10 +49,11 @@ enum { HPS_F64 = 0, HPS_F32 = 1, HPS_C128 = 2, HPS_C64 = 3 };
  * effect but for FP64 and complex128, with info and blocks of n > 64): the
  * stage's inverses are refined from the
  * single-precision inverse instead of eliminated in double.  A matrix on
- * which the refinement does not reach double precision gets info = -2 and the
+ * which the refinement does not reach double precision, or one of whose columns
+ * lies more than 2^9 below the rows it meets, gets info = -2 and the
  * stage's output for it is not valid: call the stage again without the flag.
- * The workspace size differs, ask with the flag set.  No counterpart in the
- * reference. */
+ * The workspace size differs, ask with the flag and info set.  No counterpart in
+ * the reference. */
 #define HPS_INVERSE_REFINED 0x100
 
 /* status codes */

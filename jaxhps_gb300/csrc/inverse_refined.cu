@@ -24,9 +24,9 @@
 // the pivot exchange for few (3.3 us a column on a cluster), and its
 // rank-32 updates read and write the whole matrix n / 32 times; the products
 // of size n do not wait for one another's columns.
-// A matrix whose second residual is not small (or whose single-precision
-// inverse met a zero pivot or an overflow) gets info = INV_NOT_REFINED, and
-// the caller runs the elimination.
+// A matrix whose second residual is not small, whose single-precision inverse
+// met a zero pivot or an overflow, or whose columns are graded (done_kernel)
+// gets info = INV_NOT_REFINED, and the caller runs the elimination.
 #include "hps_common.cuh"
 #include "hps_internal.h"
 
@@ -47,13 +47,44 @@ __device__ __forceinline__ float mag(c64 v) { return fabsf(v.x) + fabsf(v.y); }
 
 constexpr int RF_NT = 256;
 
-// out (contiguous) = A in single precision
+// The larger part's magnitude as the upper word of its bits.
+__device__ __forceinline__ uint32_t top_word(double v) { return (uint32_t)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t top_word(c128 v) { return max(top_word(v.x), top_word(v.y)); }
+
+// out (contiguous) = A in single precision, and the columns' spans: RF_ONE less
+// the binary orders by which a column's largest entry lies below its own row's
+// largest, the best of the rows (0: a column of zeros).  A warp per row, which
+// it reads twice (the second time from L1); a CTA's spans meet in shared memory.
+constexpr int RF_ONE = 64, RF_COLS = 4096;
 template <class T, class L>
-__global__ void __launch_bounds__(RF_NT) lower_kernel(int n, const T* __restrict__ A, long long lda, long long sA, L* out) {
+__global__ void __launch_bounds__(RF_NT) lower_kernel(int n, const T* __restrict__ A, long long lda, long long sA, L* out,
+                                                      int* span) {
+  __shared__ int best[RF_COLS];
   const long long b = blockIdx.y, nn = (long long)n * n;
-  for (long long e = blockIdx.x * (long long)RF_NT + threadIdx.x; e < nn; e += (long long)gridDim.x * RF_NT) {
-    const long long i = e / n;
-    out[b * nn + e] = to_low(A[b * sA + i * lda + (e - i * n)]);
+  const int lane = threadIdx.x & 31, step = gridDim.x * (RF_NT / 32);
+  for (int c0 = 0; c0 < n; c0 += RF_COLS) {
+    const int c1 = min(n, c0 + RF_COLS);
+    for (int j = c0 + threadIdx.x; j < c1; j += RF_NT) best[j - c0] = 0;
+    __syncthreads();
+    for (int i = blockIdx.x * (RF_NT / 32) + (threadIdx.x >> 5); i < n; i += step) {
+      const T* a = A + b * sA + i * lda;
+      uint32_t m = 0;
+#pragma unroll 4
+      for (int j = lane; j < n; j += 32) m = max(m, top_word(a[j]));
+      const int e = (int)(__reduce_max_sync(0xffffffffu, m) >> 20);
+#pragma unroll 4
+      for (int j = c0 + lane; j < c1; j += 32) {
+        const T v = a[j];
+        out[b * nn + (long long)i * n + j] = to_low(v);
+        const uint32_t w = top_word(v);
+        const int s = w ? max(1, RF_ONE + (int)(w >> 20) - e) : 0;
+        if (s > best[j - c0]) atomicMax(&best[j - c0], s);
+      }
+    }
+    __syncthreads();
+    for (int j = c0 + threadIdx.x; j < c1; j += RF_NT)
+      if (best[j - c0] > span[b * n + j]) atomicMax(span + b * n + j, best[j - c0]);
+    __syncthreads();
   }
 }
 
@@ -109,10 +140,22 @@ __global__ void __launch_bounds__(RF_NT) keep_kernel(int n, const T* __restrict_
   }
 }
 
-// After the first residual: the matrices that need no second step.
-__global__ void done_kernel(int batch, const int* __restrict__ low_info, int* top, int* skip) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= batch) return;
+// After the first residual: the matrices that need no second step, and those
+// whose columns are graded.  The products with A cut its entries 2^-62 below
+// their row's largest, which its residual, formed with the same cut entries,
+// cannot show; elimination rounds a column relative to the column.  As long as
+// every column's largest entry lies within 2^9 of its row's largest, the cut
+// stays below 2^-53 of the column (columns of 96 scaled by 2^-k, error of the
+// inverse's rows: 2e-16 at k = 9, elimination 6e-16; 2.5e-15 at 12, 6e-13 at 20,
+// all of them with residuals below 1e-10).
+constexpr int RF_SPAN = 9;
+__global__ void __launch_bounds__(128) done_kernel(int n, const int* __restrict__ span, int* low_info, int* top, int* skip) {
+  const long long b = blockIdx.x;
+  int least = RF_ONE;
+  for (int j = threadIdx.x; j < n; j += 128) least = min(least, span[b * n + j]);
+  const bool graded = __syncthreads_or(least < RF_ONE - RF_SPAN);
+  if (threadIdx.x) return;
+  if (graded) low_info[b] = INV_NOT_REFINED;
   skip[b] = (low_info[b] == 0 && __int_as_float(top[b]) <= 5e-5f) ? 1 : 0;
   if (!skip[b]) top[b] = 0;
 }
@@ -188,7 +231,8 @@ cudaError_t run(int n, const T* A, long long lda, long long sA, T* X, long long 
   L* l1 = (L*)take(sizeof(L) * (size_t)nn * cap);
   L* l2 = (L*)take(sizeof(L) * (size_t)nn * cap);
   int* low_info = (int*)take(sizeof(int) * (size_t)cap);
-  int* top = (int*)take(sizeof(int) * (size_t)cap);
+  int* top = (int*)take(sizeof(int) * (size_t)cap * (n + 1));   // with the columns' spans behind it
+  int* span = top + cap;
   int* skip = (int*)take(sizeof(int) * (size_t)cap);
   const size_t lowb = inverse_workspace_bytes(low_dt, n, cap);
   void* lows = take(lowb);
@@ -209,6 +253,7 @@ cudaError_t run(int n, const T* A, long long lda, long long sA, T* X, long long 
   if ((size_t)(w - base) > bytes) return cudaErrorInvalidValue;
   const L one_ = one<L>(), zero_ = zero<L>();
   const int gr = (n + RF_NT / 32 - 1) / (RF_NT / 32);   // CTAs for the rows of one matrix
+  const int gl = (n + RF_NT / 8 - 1) / (RF_NT / 8);     // four rows a warp
   const int gx = (int)((nn + RF_NT * 4 - 1) / (RF_NT * 4) < 256 ? (nn + RF_NT * 4 - 1) / (RF_NT * 4) : 256);
   cudaError_t e;
 #define RF_TRY(x)                              \
@@ -220,9 +265,9 @@ cudaError_t run(int n, const T* A, long long lda, long long sA, T* X, long long 
     const T* Ab = A + (long long)b0 * sA;
     const long long total = nn * nb;
     const int gt = (int)((total + RF_NT * 4 - 1) / (RF_NT * 4) < 16384 ? (total + RF_NT * 4 - 1) / (RF_NT * 4) : 16384);
-    RF_TRY(cudaMemsetAsync(top, 0, sizeof(int) * (size_t)nb, st));
+    RF_TRY(cudaMemsetAsync(top, 0, sizeof(int) * ((size_t)cap + (size_t)n * nb), st));
     note_launch();
-    lower_kernel<T, L><<<dim3(gx, nb), RF_NT, 0, st>>>(n, Ab, lda, sA, l0);
+    lower_kernel<T, L><<<dim3(gl, nb), RF_NT, 0, st>>>(n, Ab, lda, sA, l0, span);
     RF_TRY(inverse_batched<L>(n, l0, n, nn, l0, n, nn, nb, low_info, lows, lowb, st,
                               INV_TENSOR_MEMORY | INV_BLOCK_RECURSIVE));
     note_launch();
@@ -248,7 +293,7 @@ cudaError_t run(int n, const T* A, long long lda, long long sA, T* X, long long 
     note_launch();
     residual_kernel<T, L><<<dim3(gr, nb), RF_NT, 0, st>>>(n, R, l0, top, nullptr);
     note_launch();
-    done_kernel<<<(nb + 255) / 256, 256, 0, st>>>(nb, low_info, top, skip);
+    done_kernel<<<nb, 128, 0, st>>>(n, span, low_info, top, skip);
     RF_TRY(gemm_batched<L>(n, n, n, one_, l0, n, nn, l0, n, nn, one_, l0, n, nn, l1, n, nn, nb, st));
     RF_TRY(gemm_batched<L>(n, n, n, one_, l0, n, nn, l1, n, nn, zero_, nullptr, 0, 0, l2, n, nn, nb, st));
     note_launch();
@@ -281,7 +326,8 @@ template <class T>
 static size_t workspace_bytes(int n, int batch) {
   const size_t es = sizeof(T), nn = (size_t)n * n;
   const int cap = chunk_of(sizeof(T), n, batch), low_dt = es == 8 ? F32 : C64;
-  size_t s = 3 * al256(es * nn * cap) + 3 * al256(es / 2 * nn * cap) + 3 * al256(sizeof(int) * (size_t)cap) +
+  size_t s = 3 * al256(es * nn * cap) + 3 * al256(es / 2 * nn * cap) + 2 * al256(sizeof(int) * (size_t)cap) +
+             al256(sizeof(int) * (size_t)cap * (n + 1)) +
              al256(inverse_workspace_bytes(low_dt, n, cap)) + 512;
   if (splits<T>(n, batch)) {
     const DigitBytes d = digit_bytes<T>(n);
