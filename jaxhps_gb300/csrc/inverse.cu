@@ -1285,6 +1285,54 @@ gje_panel_reg_kernel(int n, int k0, int bw, int rows_per, T* Mat, T* U, T* G, T*
   }
 }
 
+// FP64 types, ahead of a panel's products on the digit kernels: the pivot rows G
+// are brought to the scale of the largest of them where they lie more than 2^4
+// apart, the columns of U and E that meet them the other way (powers of two:
+// the products are the same).  The digits keep a row's and a column's entries
+// relative to its largest, and U has large entries exactly where a pivot row is
+// small: one row in 16 of 128 larger by 2^30 gave inverses off by 5e-10, by 2^60
+// by 0.4 (3e-14 from multiply-adds and with this; NumPy emulation).  A warp a row,
+// bound by the latency of reading G once; without such rows nothing is written.
+__device__ __forceinline__ uint32_t gje_top(double v) { return (uint32_t)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t gje_top(c128 v) { return max(gje_top(v.x), gje_top(v.y)); }
+__device__ __forceinline__ double gje_scaled(double v, double s) { return v * s; }
+__device__ __forceinline__ c128 gje_scaled(c128 v, double s) { return c128{v.x * s, v.y * s}; }
+
+template <class T>
+__global__ void __launch_bounds__(BP * 32) gje_balance_kernel(int n, int bw, T* U, T* G, T* E) {
+  __shared__ int ex[BP];
+  const long long b = blockIdx.x;
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  T* g = G + (b * BP + k) * (long long)n;
+  uint32_t m = 0;
+  if (k < bw) {
+#pragma unroll 4
+    for (int j = lane; j < n; j += 32) m = max(m, gje_top(g[j]));
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if (lane == 0) ex[k] = (int)(m >> 20);   // 0: a row of zeros stays as it is
+  __syncthreads();
+  const int e = ex[lane], hi = (int)__reduce_max_sync(0xffffffffu, (uint32_t)e);
+  const int lo = (int)__reduce_min_sync(0xffffffffu, (uint32_t)(e ? e : 0x7ff));
+  if (hi - lo <= 4 || hi == 0x7ff) return;   // of one scale; infinities or NaN
+  auto below = [&](int c) { return ex[c] ? min(hi - ex[c], 1000) : 0; };
+  if (k < bw && below(k) > 0) {
+    const double s = __hiloint2double((1023 + below(k)) << 20, 0);
+    for (int j = lane; j < n; j += 32) g[j] = gje_scaled(g[j], s);
+  }
+  if (lane < bw) {
+    const double s = __hiloint2double((1023 - below(lane)) << 20, 0);
+    if (k < bw) {
+      T* x = E + (b * BP + k) * BP + lane;
+      *x = gje_scaled(*x, s);
+    }
+    for (int i = k; i < n; i += BP) {
+      T* x = U + (b * n + i) * BP + lane;
+      *x = gje_scaled(*x, s);
+    }
+  }
+}
+
 template <class T>
 __global__ void gje_scatter_rows_kernel(int n, int k0, int bw, T* Mat, const T* H, const int* piv) {
   const long long b = blockIdx.y;
@@ -2166,6 +2214,11 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
     // FP64: H = E G as a product (its digits are faster than the FP64 pipe), then into the pivot rows
     constexpr bool wide = sizeof(typename MagOf<T>::type) == 8;
     if constexpr (wide) {
+      if (f64_products_on_tensor_cores()) {
+        note_launch();
+        gje_balance_kernel<T><<<batch, BP * 32, 0, st>>>(n, bw, U, G, E);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      }
       e = gemm_batched<T>(bw, n, bw, one_, E, BP, BP * BP, G, n, (long long)BP * n, zero<T>(), nullptr, 0, 0, H, n,
                           (long long)BP * n, batch, st);
       if (e != cudaSuccess) return e;
