@@ -31,6 +31,8 @@ cudaError_t col_scale(int batch, int n, T* X, long long ldx, long long sX, const
 template <class T>
 cudaError_t row_scale(int batch, int rows, int cols, T* X, const double* s, cudaStream_t st);
 template <class T>
+cudaError_t balance_rows(int nm, int n, int ne, int ns, T* D, T* C, T* dh, double* s, cudaStream_t st);
+template <class T>
 cudaError_t perm_gather(int batch, int n, int nr, int nc, const T* M, long long sM, const int* perm, int r0, int c0,
                         T* out, long long sO, cudaStream_t st);
 template <class T>
@@ -371,6 +373,7 @@ static size_t merge_ws(const hps_merge_args* a, Carver* cv) {
   } else {
     cv->take(stage_inverse_bytes(a->dtype, a->n_int, a->n_merges, a->info));
   }
+  if (leaf_rows_scaled(base_dtype(a->dtype))) cv->take(sizeof(double) * nm * a->n_int);   // balance_rows
   return cv->used + 256;
 }
 
@@ -447,6 +450,7 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   }
   const size_t invb = stage_inverse_bytes(a->dtype, nx > 0 ? nx : ni, nm, a->info);
   void* invws = cv.take(invb);
+  double* rscale = leaf_rows_scaled(DTypeOf<T>::value) ? (double*)cv.take(sizeof(double) * (size_t)nm * ni) : nullptr;
   const bool with_h = ns > 0 && a->h_children && a->h_out && a->g_tilde;
   // with the block rectangles, the zero blocks of C (and of B unless B is
   // returned) are never read: the gather leaves them unwritten
@@ -461,6 +465,9 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
                               with_h ? (const T*)a->h_children : nullptr, a->int_c, a->int_l, a->ext_c, a->ext_l,
                               a->loc, D, C, B, (T*)a->T_out, dh, (T*)a->h_out, skip_zero, st));
   const T one_ = one<T>(), zero_ = zero<T>(), mone = make_scalar<T>(-1.0, 0.0);
+  // an impedance merge's rows are an identity's and a contraction's: of one scale
+  const bool balanced = rscale && !iti && f64_products_on_tensor_cores();
+  if (balanced) HPS_CHECK(balance_rows<T>(nm, ni, ne, with_h ? ns : 0, D, C, with_h ? dh : nullptr, rscale, st));
   if (nx > 0) {
     // D = [[I, D12], [D21, I]] in colour order; W = I - D12 D21,
     // D^-1 = [[W^-1, -W^-1 D12], [-D21 W^-1, I + D21 W^-1 D12]]
@@ -545,6 +552,7 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
       HPS_CHECK(gemm_batched<T>(ne, ns, ni, one_, B, ni, sB, gt, ns, sg, one_, ho, ns, sh, ho, ns, sh, nm, st));
     }
   }
+  if (balanced && (a->D_inv || a->BD_inv)) HPS_CHECK(col_scale<T>(nm, ni, D, ni, sDD, rscale, st));
   // B D^-1
   if (a->BD_inv) {
     T* BD = (T*)a->BD_inv;

@@ -268,7 +268,63 @@ __global__ void __launch_bounds__(256) col_scale_kernel(long long rows_total, in
   const long long b = row / n;
   T* x = X + b * sX + (row - b * n) * ldx;
 #pragma unroll 4
-  for (int c = lane; c < n; c += 32) x[c] = scale_by(x[c], s[b * n + c]);
+  for (int c = lane; c < n; c += 32) {
+    const double f = s[b * n + c];
+    if (f != 1.0) x[c] = scale_by(x[c], f);
+  }
+}
+
+// Rows of a merge's D that lie more than 2^4 from its first one are brought to
+// that one's scale, with C's and dh's: s = the factors (powers of two: S and g~
+// are the same, D^-1's columns are to be scaled by s).  The digit products keep
+// a row's and a column's entries relative to its largest, and D^-1's columns are
+// graded the opposite way to C's rows: with one interface row in 16 of 112 larger
+// by 2^12, S was off by 3e-14 of its largest entry, by 2^20 by 7e-12, by 2^40 by
+// 5e-6, now 1e-16 throughout.  Children that are refined differently give such
+// rows (a DtN row goes as 1 / panel size).  Merges whose rows are of one scale
+// are read once and not written.
+template <class T>
+__global__ void __launch_bounds__(256) balance_rows_kernel(long long rows_total, int n, int ne, int ns, T* D, T* C, T* dh,
+                                                           double* s) {
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= rows_total) return;
+  const T *first = D + row / n * n * (long long)n;
+  T* a = D + row * n;
+  decltype(mag_bits(T())) m = 0, m0 = 0;
+#pragma unroll 4
+  for (int c = lane; c < n; c += 32) {
+    m = max(m, mag_bits(a[c]));
+    m0 = max(m0, mag_bits(first[c]));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+  }
+  const double v = bits_value(m), v0 = bits_value(m0);
+  double f = 1.0;
+  if (v > 0.0 && v0 > 0.0 && v <= 1.7e308 && v0 <= 1.7e308) {
+    const int d = ilogb(v0) - ilogb(v);
+    if (d > 4 || d < -4) f = ldexp(1.0, min(max(d, -1000), 1000));
+  }
+  if (lane == 0) s[row] = f;
+  if (f == 1.0) return;
+  for (int c = lane; c < n; c += 32) a[c] = scale_by(a[c], f);
+  T* x = C + row * ne;
+  for (int c = lane; c < ne; c += 32) x[c] = scale_by(x[c], f);
+  if (dh)
+    for (int c = lane; c < ns; c += 32) dh[row * ns + c] = scale_by(dh[row * ns + c], f);
+}
+
+template <class T>
+cudaError_t balance_rows(int nm, int n, int ne, int ns, T* D, T* C, T* dh, double* s, cudaStream_t st) {
+  const long long rows = (long long)nm * n;
+  if (rows <= 0) return cudaSuccess;
+  ProfScope ps(KC_MOVE, st, (double)rows * n * sizeof(T));
+  note_launch();
+  balance_rows_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(rows, n, ne, ns, D, C, dh, s);
+  return cudaGetLastError();
 }
 
 // X[b] (rows x cols, contiguous) with row r scaled by s[b * rows + r].
@@ -754,6 +810,7 @@ cudaError_t convert(long long n, const S* src, D* dst, cudaStream_t st) {
   template cudaError_t row_equilibrate<T>(int, int, T*, long long, long long, double*, cudaStream_t);              \
   template cudaError_t col_scale<T>(int, int, T*, long long, long long, const double*, cudaStream_t);           \
   template cudaError_t row_scale<T>(int, int, int, T*, const double*, cudaStream_t);                            \
+  template cudaError_t balance_rows<T>(int, int, int, int, T*, T*, T*, double*, cudaStream_t);                  \
   template cudaError_t perm_gather<T>(int, int, int, int, const T*, long long, const int*, int, int, T*,       \
                                       long long, cudaStream_t);                                                  \
   template cudaError_t perm_scatter<T>(int, int, int, int, T*, long long, const int*, int, int, const T*,       \
