@@ -56,6 +56,18 @@ enum { HPS_F64 = 0, HPS_F32 = 1, HPS_C128 = 2, HPS_C64 = 3 };
  * the reference. */
 #define HPS_INVERSE_REFINED 0x100
 
+/* May be OR'ed into the dtype of hps_gemm_batched (no effect but for FP64 and
+ * complex128): the product may run on the FP16 tensor cores from 8-bit digits
+ * (csrc/gemm_f64_tc.cu) where that is faster.  An entry of the product is then
+ * within k 2^-56 max|A[i,:]| max|B[:,j]| (complex: four times) and two roundings
+ * of its value, which for operands of one scale is less than what k
+ * multiply-adds round; where every large entry of a row of A meets a small one
+ * of B's column (columns of A graded against the rows of B) it is more.  The
+ * stages' own products run that way: rows of leaf, interface and pivot blocks
+ * whose scales differ are brought to one before.  No counterpart in the
+ * reference. */
+#define HPS_PRODUCT_DIGITS 0x400
+
 /* status codes */
 enum {
   HPS_OK = 0,
@@ -125,7 +137,8 @@ HPS_API int hps_inverse_block_policy(int policy);
 
 /* Which batched products run on the tcgen05 kernels: 0 none (SIMT kernels
  * only), 1 the shapes where they were measured faster (default; HPS_GEMM_TC=0
- * in the environment starts a process at 0), 2 every product (for tests and
+ * in the environment starts a process at 0; FP64 and complex128 calls of
+ * hps_gemm_batched with HPS_PRODUCT_DIGITS only), 2 every product (for tests and
  * measurements; complex ones with real alpha and beta), 3 none and the FP32 8x8 SIMT tiles with 4-byte
  * shared-memory loads instead of the 16-byte-load tiles (for comparisons;
  * identical results).  Returns the previous policy, or -1 for an
@@ -181,7 +194,9 @@ HPS_API int hps_last_error(char* buf, size_t len);
 
 /* D[b] = alpha * A[b] @ B[b] + beta * C[b]  (row-major, m x k times k x n).
  * alpha/beta are host pointers to {re, im}.  C may be NULL (beta ignored)
- * and may alias D.  A batch stride of 0 broadcasts that operand.
+ * and may alias D.  A batch stride of 0 broadcasts that operand.  FP64 and
+ * complex128 products are multiply-adds in FP64 unless HPS_PRODUCT_DIGITS is set
+ * in dtype or hps_gemm_policy is 2.
  * Replaces the `@` / einsum products of get_DtN (_uniform_2D_DtN.py:264-271),
  * _assemble_merge_outputs (merge/_schur_complement.py:222-235) and the down
  * pass (down_pass/_uniform_2D_DtN.py:114-120, :149). */

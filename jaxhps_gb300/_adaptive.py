@@ -403,9 +403,9 @@ def down_pass_adaptive_3D_DtN(pde_problem, boundary_data, device=None, host_devi
         vv = v if v.dim() == 3 else v.unsqueeze(-1)
         if vv.shape[-1] != ns:
             vv = vv.expand(-1, -1, ns)
-        nat.gemm(Y, gl, u, 1.0, 1.0, Cmat=vv.contiguous())
+        nat.gemm(Y, gl, u, 1.0, 1.0, Cmat=vv.contiguous(), digits=True)
     else:
-        nat.gemm(Y, gl, u)
+        nat.gemm(Y, gl, u, digits=True)
     for i, lf in enumerate(leaves):
         lf.data.u = u[i]
     if single and (v is None or v.dim() == 2):

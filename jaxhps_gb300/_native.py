@@ -22,6 +22,7 @@ HPS_F64, HPS_F32, HPS_C128, HPS_C64 = 0, 1, 2, 3
 HPS_CODE_PAD = -(2 ** 31)
 HPS_UP_B_IS_BD_INV, HPS_UP_ITI = 1, 2
 HPS_INVERSE_REFINED = 0x100   # for blocks of n > REFINED_ABOVE
+HPS_PRODUCT_DIGITS = 0x400
 INFO_NOT_REFINED = -2
 REFINED_ABOVE = 64
 
@@ -381,11 +382,13 @@ def release_workspace() -> None:
 # ---------------------------------------------------------------------------
 
 
-def gemm(A, B, out, alpha=1.0, beta=0.0, Cmat=None, batch=None):
+def gemm(A, B, out, alpha=1.0, beta=0.0, Cmat=None, batch=None, digits=False):
     """out[b] = alpha A[b] @ B[b] + beta C[b] for 3D (or broadcast 2D) tensors,
-    all contiguous in their last two dims."""
+    all contiguous in their last two dims.  ``digits`` lets FP64 and complex128
+    products run on the tensor cores, with errors relative to the largest entries
+    of A's rows and B's columns (HPS_PRODUCT_DIGITS in the C ABI)."""
     L = lib()
-    dt = TORCH_TO_HPS[out.dtype]
+    dt = TORCH_TO_HPS[out.dtype] | (HPS_PRODUCT_DIGITS if digits else 0)
 
     def mat(t):
         if t.dim() == 2:

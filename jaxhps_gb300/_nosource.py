@@ -169,14 +169,14 @@ def _up_pass(source, pde_problem, iti: bool, device=None, return_h_last: bool = 
     nl, n_pts, ns = f.shape
     if iti:
         v = torch.empty((nl, n_pts, ns), dtype=dtype, device=dev)
-        nat.gemm(Phi, f[:, n_cb:, :], v)
+        nat.gemm(Phi, f[:, n_cb:, :], v, digits=True)
         Q = st._as_tensor(pde_problem.QH, dtype, dev)
     else:
         v = torch.zeros((nl, n_pts, ns), dtype=dtype, device=dev)
-        nat.gemm(Phi, f[:, n_cb:, :], v[:, n_cb:, :])
+        nat.gemm(Phi, f[:, n_cb:, :], v[:, n_cb:, :], digits=True)
         Q = st._as_tensor(pde_problem.Q, dtype, dev)
     h = torch.empty((nl, Q.shape[0], ns), dtype=dtype, device=dev)
-    nat.gemm(Q, v, h)
+    nat.gemm(Q, v, h, digits=True)
     g_lst = []
     for Dinv, BDinv in zip(pde_problem._D_inv_int, pde_problem._BD_inv_int):
         nc = BDinv.shape[1] // 8

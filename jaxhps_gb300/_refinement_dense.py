@@ -106,8 +106,8 @@ def _refine_leaf_operators(Y, Aii_inv, Aint, P64, Q64, Q_int, n_cb):
     Y0_64 = torch.empty((nl, n_i, ng), dtype=torch.float64, device=dev)
     _f32_to_f64(Y0.contiguous(), Y0_64)
     R = torch.empty((nl, n_i, ng), dtype=torch.float64, device=dev)
-    nat.gemm(Aint[:, :, :n_cb], P64, R, alpha=-1.0)
-    nat.gemm(Aint[:, :, n_cb:], Y0_64, R, alpha=-1.0, beta=1.0, Cmat=R)
+    nat.gemm(Aint[:, :, :n_cb], P64, R, alpha=-1.0, digits=True)
+    nat.gemm(Aint[:, :, n_cb:], Y0_64, R, alpha=-1.0, beta=1.0, Cmat=R, digits=True)
     r32 = torch.empty((nl, n_i, ng), dtype=torch.float32, device=dev)
     _f64_to_f32(R, r32)
     del R
@@ -115,9 +115,9 @@ def _refine_leaf_operators(Y, Aii_inv, Aint, P64, Q64, Q_int, n_cb):
     nat.gemm(Aii_inv, r32, dY)
     nat.gemm(Aii_inv, r32, Y0, 1.0, 1.0, Cmat=Y0)       # Y_int += dY (in place)
     QbP = torch.empty((ng, ng), dtype=torch.float64, device=dev)
-    nat.gemm(Q64[:, :n_cb], P64, QbP)
+    nat.gemm(Q64[:, :n_cb], P64, QbP, digits=True)
     T64 = torch.empty((nl, ng, ng), dtype=torch.float64, device=dev)
-    nat.gemm(Q64[:, n_cb:], Y0_64, T64, 1.0, 1.0, Cmat=QbP)
+    nat.gemm(Q64[:, n_cb:], Y0_64, T64, 1.0, 1.0, Cmat=QbP, digits=True)
     T = torch.empty((nl, ng, ng), dtype=torch.float32, device=dev)
     _f64_to_f32(T64, T)
     nat.gemm(Q_int, dY, T, 1.0, 1.0, Cmat=T)
@@ -192,11 +192,11 @@ def _residual(state: DenseMixedState, u_int, g, ub, r64, r32, flux):
     """FP64 residual at (u_int, g): r64 = f_int - A_int [P g ; u_int],
     flux = Q [P g ; u_int]; r32 = r64 rounded."""
     n_cb = state.n_cb
-    nat.gemm(state.P64, g, ub)
-    nat.gemm(state.Aint[:, :, :n_cb], ub, r64, alpha=-1.0, beta=1.0, Cmat=state.f[:, n_cb:, :])
-    nat.gemm(state.Aint[:, :, n_cb:], u_int, r64, alpha=-1.0, beta=1.0, Cmat=r64)
-    nat.gemm(state.Q64[:, :n_cb], ub, flux)
-    nat.gemm(state.Q64[:, n_cb:], u_int, flux, 1.0, 1.0, Cmat=flux)
+    nat.gemm(state.P64, g, ub, digits=True)
+    nat.gemm(state.Aint[:, :, :n_cb], ub, r64, alpha=-1.0, beta=1.0, Cmat=state.f[:, n_cb:, :], digits=True)
+    nat.gemm(state.Aint[:, :, n_cb:], u_int, r64, alpha=-1.0, beta=1.0, Cmat=r64, digits=True)
+    nat.gemm(state.Q64[:, :n_cb], ub, flux, digits=True)
+    nat.gemm(state.Q64[:, n_cb:], u_int, flux, 1.0, 1.0, Cmat=flux, digits=True)
     _f64_to_f32(r64, r32)
 
 
@@ -268,7 +268,7 @@ def solve_mixed_dense(pde_problem, boundary_data, source=None, host_device="cpu"
         raise_not_converged(state.history, tol, max_iters, "mixed-precision 3D solve")
     nat.raise_on_tc_timeout("mixed-precision 3D solve")
     u = torch.empty((nl, n_pts, ns), dtype=torch.float64, device=dev)
-    nat.gemm(state.P64, g, u[:, :n_cb, :])
+    nat.gemm(state.P64, g, u[:, :n_cb, :], digits=True)
     u[:, n_cb:, :].copy_(u_int)
     if not state.multi:
         u = u[..., 0]

@@ -563,9 +563,9 @@ def _down_pass_generic(boundary_data, S_lst, g_tilde_lst, Y_arr, v_arr, maps_fn,
         if v.shape[-1] != ns:
             v = v.expand(-1, -1, ns)
         v = v.contiguous()
-        nat.gemm(Y_arr, g, u, 1.0, 1.0, Cmat=v)
+        nat.gemm(Y_arr, g, u, 1.0, 1.0, Cmat=v, digits=True)
     else:
-        nat.gemm(Y_arr, g, u)
+        nat.gemm(Y_arr, g, u, digits=True)
     if ns == 1 and not multi_g and (v_arr is None or v_arr.dim() == 2):
         u = u[..., 0]
     return _to_host(u, host_device)

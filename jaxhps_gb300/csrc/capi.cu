@@ -590,13 +590,13 @@ static int down_impl(const hps_down_args* a, cudaStream_t st) {
 }
 
 template <class T>
-static int gemm_entry(int m, int n, int k, const double* alpha, const void* A, long long lda, long long sA,
+static int gemm_entry(bool digits, int m, int n, int k, const double* alpha, const void* A, long long lda, long long sA,
                       const void* B, long long ldb, long long sB, const double* beta, const void* C, long long ldc,
                       long long sC, void* D, long long ldd, long long sD, int batch, void* stream) {
   const T al = make_scalar<T>(alpha ? alpha[0] : 1.0, alpha ? alpha[1] : 0.0);
   const T be = make_scalar<T>(beta ? beta[0] : 0.0, beta ? beta[1] : 0.0);
   HPS_CHECK(gemm_batched<T>(m, n, k, al, (const T*)A, lda, sA, (const T*)B, ldb, sB, be, (const T*)C, ldc, sC,
-                            (T*)D, ldd, sD, batch, (cudaStream_t)stream));
+                            (T*)D, ldd, sD, batch, (cudaStream_t)stream, digits));
   return HPS_OK;
 }
 
@@ -807,7 +807,7 @@ int hps_gemm_batched(int dtype, int m, int n, int k, const double* alpha, const 
     set_error("hps_gemm_batched: invalid arguments");
     return HPS_ERR_ARG;
   }
-  DISPATCH(dtype, gemm_entry, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc, strideC, D, ldd,
+  DISPATCH(dtype & ~HPS_PRODUCT_DIGITS, gemm_entry, (dtype & HPS_PRODUCT_DIGITS) != 0, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc, strideC, D, ldd,
            strideD, batch, stream)
 }
 

@@ -1077,9 +1077,10 @@ bool f64_products_on_tensor_cores() {
 // (N = 8) per element of A (complex: 9.1e-6 to 66e-6).  Measured at M = K = 196,
 // batch 4096: N = 1 0.41 (FP64) against 0.92 ms, N = 2 0.80 against 0.92, N = 8
 // 2.9 against 0.94; M = 3584, K = 1792, N = 8, one matrix: 0.094 against 0.149.
-static bool f64_on_tensor_cores(int M, int N, int K, int batch, bool cplx) {
+static bool f64_on_tensor_cores(int M, int N, int K, int batch, bool cplx, bool digits) {
   if (K <= 0 || !f64_products_on_tensor_cores()) return false;
   if (gemm_policy() == 2) return true;
+  if (!digits) return false;
   if (N > 8) return K >= 16 || (K >= 4 && (double)M * N * batch >= 1 << 20);
   if (K < 32) return false;
   const double tiles = (double)((M + 127) / 128) * batch;
@@ -1093,7 +1094,8 @@ static bool f64_on_tensor_cores(int M, int N, int K, int batch, bool cplx) {
 template <class T>
 cudaError_t gemm_batched(int M, int N, int K, T alpha, const T* A, long long lda, long long sA,
                          const T* B, long long ldb, long long sB, T beta, const T* C, long long ldc,
-                         long long sC, T* D, long long ldd, long long sD, int batch, cudaStream_t st) {
+                         long long sC, T* D, long long ldd, long long sD, int batch, cudaStream_t st,
+                         bool digits) {
   if (M <= 0 || N <= 0 || batch <= 0) return cudaSuccess;
   if constexpr (std::is_same<T, float>::value) {
     if (!(N <= 8 && K >= 32)) {
@@ -1105,11 +1107,11 @@ cudaError_t gemm_batched(int M, int N, int K, T alpha, const T* A, long long lda
     }
   }
   if constexpr (std::is_same<T, double>::value) {
-    if (f64_on_tensor_cores(M, N, K, batch, false))
+    if (f64_on_tensor_cores(M, N, K, batch, false, digits))
       return gemm_f64_tc(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, D, ldd, sD, batch, st);
   }
   if constexpr (std::is_same<T, c128>::value) {
-    if (alpha.y == 0.0 && beta.y == 0.0 && f64_on_tensor_cores(M, N, K, batch, true))
+    if (alpha.y == 0.0 && beta.y == 0.0 && f64_on_tensor_cores(M, N, K, batch, true, digits))
       return gemm_c128_tc(M, N, K, alpha.x, A, lda, sA, B, ldb, sB, beta.x, C, ldc, sC, D, ldd, sD, batch, st);
   }
   if (N <= 8 && K >= 32) {
@@ -1210,7 +1212,7 @@ cudaError_t gemm_batched(int M, int N, int K, T alpha, const T* A, long long lda
 #define HPS_INST_GEMM(T)                                                                          \
   template cudaError_t gemm_batched<T>(int, int, int, T, const T*, long long, long long, const T*, \
                                        long long, long long, T, const T*, long long, long long,    \
-                                       T*, long long, long long, int, cudaStream_t);
+                                       T*, long long, long long, int, cudaStream_t, bool);
 HPS_INST_GEMM(float)
 HPS_INST_GEMM(double)
 HPS_INST_GEMM(c64)

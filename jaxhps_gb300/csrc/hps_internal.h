@@ -12,11 +12,15 @@ struct CUtensorMap_st;   // CUtensorMap of cuda.h
 namespace hps {
 
 // D = alpha*A@B + beta*C over a strided batch (row-major).  C may be null
-// (then beta is ignored) and may alias D.
+// (then beta is ignored) and may alias D.  digits: FP64 and complex128 products
+// may run on the digit kernels (gemm_f64_tc.cu) by the rule for their sizes,
+// where the caller knows that no large entry of A's rows meets only small ones
+// of B's columns.
 template <class T>
 cudaError_t gemm_batched(int M, int N, int K, T alpha, const T* A, long long lda, long long sA,
                          const T* B, long long ldb, long long sB, T beta, const T* C, long long ldc,
-                         long long sC, T* D, long long ldd, long long sD, int batch, cudaStream_t st);
+                         long long sC, T* D, long long ldd, long long sD, int batch, cudaStream_t st,
+                         bool digits = true);
 
 // Batched inverse by Gauss-Jordan elimination with partial (row) pivoting.
 // X may alias A.  info[b] = 0 on success, k+1 if the k-th pivot was zero.
