@@ -42,9 +42,11 @@ REAL_TO_COMPLEX = {torch.float64: torch.complex128, torch.float32: torch.complex
 
 def refines(dtype, n: int) -> bool:
     """Whether a stage's inverses of size n are first refined from the
-    single-precision inverse; a stage in which some matrix does not get there
-    (info = -2, ``unrefined``) is run again by elimination."""
-    return dtype in (torch.float64, torch.complex128) and n > nat.REFINED_ABOVE
+    single-precision inverse; those that do not get there (info = -2,
+    ``unrefined``) are run again by elimination.  Not while a graph is captured:
+    the status words cannot be read then."""
+    return (dtype in (torch.float64, torch.complex128) and n > nat.REFINED_ABOVE
+            and not torch.cuda.is_current_stream_capturing())
 
 
 def unrefined(infos) -> bool:
