@@ -26,7 +26,7 @@ def _inverses(A, batch, flag):
     op = np.zeros((1, n_pts, n_pts))
     op[0, n_cb:, n_cb:] = (A / phase[n_cb:, None]).real if cplx else A
     op[0, n_cb:, :n_cb] = 1.0
-    t = lambda a, d=torch.float64: torch.as_tensor(np.array(a), dtype=d, device="cuda")  # noqa: E731
+    t = lambda a, d=torch.float64: torch.as_tensor(np.array(a, order="C"), dtype=d, device="cuda")  # noqa: E731
     ops, P, Q = t(op), t(np.ones((n_cb, ng)), dt), t(np.ones((ng, n_pts)), dt)
     co = t(np.broadcast_to(phase, (1, batch, n_pts)), dt)
     Y, T, X = (torch.empty(s, dtype=dt, device="cuda") for s in ((batch, n_pts, ng), (batch, ng, ng), (batch, n, n)))
