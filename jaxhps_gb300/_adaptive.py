@@ -299,56 +299,68 @@ def merge_stage_adaptive_3D_DtN(pde_problem, T_arr, h_arr, device=None, return_T
     depth = get_depth(root)
     pan = q ** (g.dim - 1)
     K = g.nch
-    for refined in ([], None):
-        levels: List[List[Bucket]] = []
+
+    def merge_level(level: int, refined):
         infos: list = []
-        for level in range(depth - 1, -1, -1):
-            groups: Dict[tuple, list] = {}
-            for node in get_nodes_at_level(root, level):
-                if not len(node.children):
-                    continue
-                sizes = tuple(_face_sizes(ch) for ch in node.children)
-                proj = projection_lists(node)
-                key = (sizes, tuple(sorted(proj.items())))
-                groups.setdefault(key, []).append(node)
-                if key not in plans:
-                    plans[key] = _build_plan(sizes, proj, q, dev, g)
-            buckets = []
-            for key, nodes in groups.items():
-                plan = plans[key]
-                nm, R = len(nodes), plan.nbr_max
-                Tpad = torch.zeros((nm, K, R, R), dtype=dtype, device=dev)
-                hpad = torch.zeros((nm, K, R, ns), dtype=dtype, device=dev) if ns else None
-                for c in range(K):
-                    Tc = torch.stack([n.children[c].data.T for n in nodes])
-                    nb, nbr = plan.nb[c], plan.nbr[c]
+        groups: Dict[tuple, list] = {}
+        for node in get_nodes_at_level(root, level):
+            if not len(node.children):
+                continue
+            sizes = tuple(_face_sizes(ch) for ch in node.children)
+            proj = projection_lists(node)
+            key = (sizes, tuple(sorted(proj.items())))
+            groups.setdefault(key, []).append(node)
+            if key not in plans:
+                plans[key] = _build_plan(sizes, proj, q, dev, g)
+        buckets = []
+        for key, nodes in groups.items():
+            plan = plans[key]
+            nm, R = len(nodes), plan.nbr_max
+            Tpad = torch.zeros((nm, K, R, R), dtype=dtype, device=dev)
+            hpad = torch.zeros((nm, K, R, ns), dtype=dtype, device=dev) if ns else None
+            for c in range(K):
+                Tc = torch.stack([n.children[c].data.T for n in nodes])
+                nb, nbr = plan.nb[c], plan.nbr[c]
+                if plan.any_compressed[c]:
+                    tmp = torch.empty((nm, nbr, nb), dtype=dtype, device=dev)
+                    _panel_map(0, plan.compress[c], L_rows, Tc, nb, nb * nb, tmp, nb, nbr * nb, nm, nb, pan)
+                    _panel_map(1, plan.compress[c], L_cols, tmp, nb, nbr * nb, Tpad[:, c], R, K * R * R, nm, nbr, pan)
+                else:
+                    Tpad[:, c, :nb, :nb] = Tc
+                if ns:
+                    hc = torch.stack([n.children[c].data.h for n in nodes])
                     if plan.any_compressed[c]:
-                        tmp = torch.empty((nm, nbr, nb), dtype=dtype, device=dev)
-                        _panel_map(0, plan.compress[c], L_rows, Tc, nb, nb * nb, tmp, nb, nbr * nb, nm, nb, pan)
-                        _panel_map(1, plan.compress[c], L_cols, tmp, nb, nbr * nb, Tpad[:, c], R, K * R * R, nm, nbr, pan)
+                        _panel_map(0, plan.compress[c], L_rows, hc, ns, nb * ns, hpad[:, c], ns, K * R * ns, nm, ns,
+                                   pan)
                     else:
-                        Tpad[:, c, :nb, :nb] = Tc
-                    if ns:
-                        hc = torch.stack([n.children[c].data.h for n in nodes])
-                        if plan.any_compressed[c]:
-                            _panel_map(0, plan.compress[c], L_rows, hc, ns, nb * ns, hpad[:, c], ns, K * R * ns, nm, ns,
-                                       pan)
-                        else:
-                            hpad[:, c, :nb] = hc
-                is_root = level == 0
-                S, g_t, T_out, h_out, _, _ = st.merge_level_dtn(
-                    Tpad.view(nm * K, R, R), None if hpad is None else hpad.view(nm * K, R, ns), plan.maps,
-                    need_T=(not is_root) or return_T, infos=infos,
-                    refined=refined)
-                for m, node in enumerate(nodes):
-                    node.data.S = S[m]
-                    node.data.g_tilde = None if g_t is None else g_t[m]
-                    node.data.T = None if T_out is None else T_out[m]
-                    node.data.h = None if h_out is None else h_out[m]
-                buckets.append(Bucket(nodes, plan, S, g_t))
-            levels.append(buckets)
-        if not st.unrefined(refined):
-            break
+                        hpad[:, c, :nb] = hc
+            is_root = level == 0
+            S, g_t, T_out, h_out, _, _ = st.merge_level_dtn(
+                Tpad.view(nm * K, R, R), None if hpad is None else hpad.view(nm * K, R, ns), plan.maps,
+                need_T=(not is_root) or return_T, infos=infos, refined=refined)
+            for m, node in enumerate(nodes):
+                node.data.S = S[m]
+                node.data.g_tilde = None if g_t is None else g_t[m]
+                node.data.T = None if T_out is None else T_out[m]
+                node.data.h = None if h_out is None else h_out[m]
+            buckets.append(Bucket(nodes, plan, S, g_t))
+        return buckets, infos
+
+    order = range(depth - 1, -1, -1)
+    status = [[] for _ in order]
+    merged = [merge_level(level, refined) for level, refined in zip(order, status)]
+    if st.unrefined([i for s in status for i in s]):
+        # from the first level with an inverse that was not refined on, that one by
+        # elimination and the ones above it looked at one by one: the children's
+        # maps are still on the nodes
+        first = next(i for i, s in enumerate(status) if st.unrefined(s))
+        for i in range(first, len(merged)):
+            refined = None if i == first else []
+            merged[i] = merge_level(order[i], refined)
+            if i > first and st.unrefined(refined):
+                merged[i] = merge_level(order[i], None)
+    levels: List[List[Bucket]] = [buckets for buckets, _ in merged]
+    infos = [i for _, lst in merged for i in lst]
     st.raise_on_sync_timeout(infos)
     levels.reverse()          # root level first
     pde_problem._adaptive_levels = levels

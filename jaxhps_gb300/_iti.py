@@ -19,31 +19,34 @@ def merge_stage_uniform_2D_ItI(T_arr, h_arr, l: int, device=None, host_device=No
                                return_T: bool = False, return_h: bool = False):
     """Returns (S_lst, g_tilde_lst[, T_top][, h_top]) like the reference."""
     dev = st._device(device)
-    T = T_arr if isinstance(T_arr, torch.Tensor) else st._as_tensor(T_arr, torch.complex128, dev)
-    T = T.to(dev).contiguous()
-    if not T.is_complex():
-        T = T.to(torch.complex128)
-    if T.dim() == 4:
-        T = T.reshape(-1, T.shape[-2], T.shape[-1])
     multi = h_arr is not None and (h_arr.dim() == 3 if isinstance(h_arr, torch.Tensor) else np.ndim(h_arr) == 3)
-    h = None
-    if h_arr is not None:
-        h = h_arr if isinstance(h_arr, torch.Tensor) else st._as_tensor(h_arr, T.dtype, dev)
-        h = h.to(device=dev, dtype=T.dtype)
-        if h.dim() == 2:
-            h = h.unsqueeze(-1)
-        h = h.reshape(T.shape[0], T.shape[1], -1).contiguous()
-    T_leaf, h_leaf = T, h
-    for refined in ([], None):
-        T, h = T_leaf, h_leaf
-        S_lst, g_lst = [], []
-        for _ in range(max(int(l), 1)):
-            maps = quad_merge_maps_iti(T.shape[1] // 4)
-            S, g_t, T, h, _, _ = st.merge_level_dtn(T, h, maps, iti=True, refined=refined)
-            S_lst.append(S)
-            g_lst.append(g_t if (g_t is None or multi) else g_t[..., 0])
-        if not st.unrefined(refined):
-            break
+
+    def leaves():
+        T = T_arr if isinstance(T_arr, torch.Tensor) else st._as_tensor(T_arr, torch.complex128, dev)
+        T = T.to(dev).contiguous()
+        if not T.is_complex():
+            T = T.to(torch.complex128)
+        if T.dim() == 4:
+            T = T.reshape(-1, T.shape[-2], T.shape[-1])
+        h = None
+        if h_arr is not None:
+            h = h_arr if isinstance(h_arr, torch.Tensor) else st._as_tensor(h_arr, T.dtype, dev)
+            h = h.to(device=dev, dtype=T.dtype)
+            if h.dim() == 2:
+                h = h.unsqueeze(-1)
+            h = h.reshape(T.shape[0], T.shape[1], -1).contiguous()
+        return T, h
+
+    n_levels = max(int(l), 1)
+    S_lst, g_lst = [None] * n_levels, [None] * n_levels
+
+    def level(lvl, T, h, refined):
+        maps = quad_merge_maps_iti(T.shape[1] // 4)
+        S_lst[lvl], g_t, T, h, _, _ = st.merge_level_dtn(T, h, maps, iti=True, refined=refined)
+        g_lst[lvl] = g_t if (g_t is None or multi) else g_t[..., 0]
+        return T, h
+
+    T, h = st.merge_levels(n_levels, leaves, level)
     if subtree_recomp:
         return T, (h if (h is None or multi) else h[..., 0])
     out = (S_lst, g_lst)

@@ -104,23 +104,20 @@ def store_operators(pde_problem, Dinv_lst, BDinv_lst, iti: bool) -> None:
 
 def _nosource_merge(T_arr, l: int, iti: bool, device=None, return_T: bool = False):
     dev = st._device(device)
-    T = T_arr.to(dev).contiguous()
-    T_leaf = T
     n_levels = max(int(l), 1)
-    for refined in ([], None):
-        T = T_leaf
-        S_lst, Dinv_lst, BDinv_lst, infos = [], [], [], []
-        for lvl in range(n_levels):
-            nc = T.shape[1] // 4
-            maps = quad_merge_maps_iti(nc) if iti else quad_merge_maps_dtn(nc)
-            need_T = lvl < n_levels - 1 or return_T
-            S, _, T, _, Dinv, BDinv = st.merge_level_dtn(T, None, maps, keep_D_inv=True, keep_BD_inv=True, iti=iti,
-                                                         need_T=need_T, infos=infos, refined=refined)
-            S_lst.append(S)
-            Dinv_lst.append(Dinv)
-            BDinv_lst.append(BDinv)
-        if not st.unrefined(refined):
-            break
+    S_lst, Dinv_lst, BDinv_lst, infos = ([None] * n_levels for _ in range(4))
+
+    def level(lvl, T, h, refined):
+        nc = T.shape[1] // 4
+        maps = quad_merge_maps_iti(nc) if iti else quad_merge_maps_dtn(nc)
+        need_T = lvl < n_levels - 1 or return_T
+        info = []
+        S_lst[lvl], _, T, _, Dinv_lst[lvl], BDinv_lst[lvl] = st.merge_level_dtn(
+            T, None, maps, keep_D_inv=True, keep_BD_inv=True, iti=iti, need_T=need_T, infos=info, refined=refined)
+        infos[lvl] = info[0]
+        return T, None
+
+    T, _ = st.merge_levels(n_levels, lambda: (T_arr.to(dev).contiguous(), None), level)
     st.raise_on_sync_timeout(infos)
     out = (S_lst, Dinv_lst, BDinv_lst)
     if return_T:

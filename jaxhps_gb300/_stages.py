@@ -57,6 +57,40 @@ def unrefined(infos) -> bool:
     return int(torch.cat([i.reshape(-1) for i in infos]).min()) == nat.INFO_NOT_REFINED
 
 
+def _again(infos: torch.Tensor):
+    """Which leaves run again after ``unrefined``: the indices of those that were not
+    refined, or None for all of them: more than half, or no more leaves than SMs
+    (their eliminations are chains of pivots side by side: 152 of 196 rows take
+    2.0 ms, one 1.0, 4096 take 54)."""
+    idx = torch.nonzero(infos == nat.INFO_NOT_REFINED).reshape(-1)
+    sms = torch.cuda.get_device_properties(infos.device).multi_processor_count
+    return idx if infos.numel() > sms and 2 * idx.numel() <= infos.numel() else None
+
+
+def _leaf_stage(dtype, n: int, info: torch.Tensor, run, per_leaf, outs) -> None:
+    """run(flag, inputs, outs, info) over all leaves, with the inverses of size n
+    refined where ``refines`` says so; the leaves whose inverse was not refined run
+    again without, on copies of their inputs and outputs.  per_leaf: (tensor or
+    None, its dimension of leaves) of the inputs; outs: tensors or None."""
+    if not refines(dtype, n):
+        run(0, [t for t, _ in per_leaf], outs, info)
+        return
+    run(nat.HPS_INVERSE_REFINED, [t for t, _ in per_leaf], outs, info)
+    if not unrefined([info]):
+        return
+    idx = _again(info)
+    if idx is None:
+        run(0, [t for t, _ in per_leaf], outs, info)
+        return
+    ins = [None if t is None else t.index_select(d, idx).contiguous() for t, d in per_leaf]
+    some = [None if t is None else torch.empty((idx.numel(), *t.shape[1:]), dtype=t.dtype, device=t.device) for t in outs]
+    part = torch.zeros(idx.numel(), dtype=info.dtype, device=info.device)
+    run(0, ins, some, part)
+    for t, s in zip([*outs, info], [*some, part]):
+        if t is not None:
+            t.index_copy_(0, idx, s)
+
+
 # Device bytes the leaf stage's workspace (the assembled leaf operators) may
 # take at once; above it the leaves go in chunks.
 LEAF_WORKSPACE_BUDGET = 16 << 30
@@ -237,42 +271,46 @@ def _local_solve_dtn(pde_problem, P_np, Q_np, device, dtype, keep_inverse, sourc
     h = torch.empty((n_leaves, ng, ns), dtype=dtype, device=dev) if ns else None
     Aii = torch.empty((n_leaves, n_i, n_i), dtype=dtype, device=dev)
     info = torch.zeros(n_leaves, dtype=torch.int32, device=dev)
-    for flag in ((nat.HPS_INVERSE_REFINED, 0) if refines(dtype, n_i) else (0,)):
+    es = Y.element_size()
+
+    def run(flag, ins, outs, info):
+        co, f = ins
+        Y, T, v, h, Aii = outs
+        n = info.numel()
         a = nat.LeafDtnArgs(
-            dtype=nat.TORCH_TO_HPS[dtype] | flag, coef_complex=int(cplx), n_leaves=n_leaves, n_pts=n_pts, n_cb=n_cb,
-            n_gauss=ng, nsrc=ns, n_ops=ops_t.shape[0], ops=ops_t.data_ptr(), coeffs=coeffs.data_ptr(),
+            dtype=nat.TORCH_TO_HPS[dtype] | flag, coef_complex=int(cplx), n_leaves=n, n_pts=n_pts, n_cb=n_cb,
+            n_gauss=ng, nsrc=ns, n_ops=ops_t.shape[0], ops=ops_t.data_ptr(), coeffs=co.data_ptr(),
             source=nat.ptr(f), P=P.data_ptr(), Q=Q.data_ptr(), Y=Y.data_ptr(), T=T.data_ptr(), v=nat.ptr(v),
             h=nat.ptr(h), Aii_inv=Aii.data_ptr(), info=info.data_ptr(), workspace=None, workspace_bytes=0)
         wsb = L.hps_local_solve_dtn_workspace_size(C.byref(a))
-        if wsb <= LEAF_WORKSPACE_BUDGET or n_leaves == 1:
+        if wsb <= LEAF_WORKSPACE_BUDGET or n == 1:
             ws = nat.workspace(wsb, dev)
             a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
             nat.check(L.hps_local_solve_dtn(C.byref(a), nat.stream_ptr()), "hps_local_solve_dtn")
-        else:
-            # the assembled leaf operators of every leaf would not fit the budget:
-            # leaves in chunks (the reference chunks its leaf stage as well,
-            # _device_config.py:65-90), one workspace reused by all chunks
-            chunk = max(1, int(n_leaves * LEAF_WORKSPACE_BUDGET // wsb))
-            es = torch.empty((), dtype=dtype).element_size()
-            for lo in range(0, n_leaves, chunk):
-                hi = min(n_leaves, lo + chunk)
-                cc = coeffs[:, lo:hi].contiguous()
-                b = nat.LeafDtnArgs(
-                    dtype=a.dtype, coef_complex=a.coef_complex, n_leaves=hi - lo, n_pts=n_pts, n_cb=n_cb, n_gauss=ng,
-                    nsrc=ns, n_ops=a.n_ops, ops=a.ops, coeffs=cc.data_ptr(),
-                    source=None if f is None else f.data_ptr() + lo * n_pts * ns * es, P=a.P, Q=a.Q,
-                    Y=Y.data_ptr() + lo * n_pts * ng * es, T=T.data_ptr() + lo * ng * ng * es,
-                    v=None if v is None else v.data_ptr() + lo * n_pts * ns * es,
-                    h=None if h is None else h.data_ptr() + lo * ng * ns * es,
-                    Aii_inv=Aii.data_ptr() + lo * n_i * n_i * es, info=info.data_ptr() + lo * 4, workspace=None,
-                    workspace_bytes=0)
-                wsc = L.hps_local_solve_dtn_workspace_size(C.byref(b))
-                ws = nat.workspace(wsc, dev)
-                b.workspace, b.workspace_bytes = ws.data_ptr(), ws.numel()
-                nat.check(L.hps_local_solve_dtn(C.byref(b), nat.stream_ptr()), "hps_local_solve_dtn")
-                del cc
-        if not flag or not unrefined([info]):
-            break
+            return
+        # the assembled leaf operators of every leaf would not fit the budget:
+        # leaves in chunks (the reference chunks its leaf stage as well,
+        # _device_config.py:65-90), one workspace reused by all chunks
+        chunk = max(1, int(n * LEAF_WORKSPACE_BUDGET // wsb))
+        for lo in range(0, n, chunk):
+            hi = min(n, lo + chunk)
+            cc = co[:, lo:hi].contiguous()
+            b = nat.LeafDtnArgs(
+                dtype=a.dtype, coef_complex=a.coef_complex, n_leaves=hi - lo, n_pts=n_pts, n_cb=n_cb, n_gauss=ng,
+                nsrc=ns, n_ops=a.n_ops, ops=a.ops, coeffs=cc.data_ptr(),
+                source=None if f is None else f.data_ptr() + lo * n_pts * ns * es, P=a.P, Q=a.Q,
+                Y=Y.data_ptr() + lo * n_pts * ng * es, T=T.data_ptr() + lo * ng * ng * es,
+                v=None if v is None else v.data_ptr() + lo * n_pts * ns * es,
+                h=None if h is None else h.data_ptr() + lo * ng * ns * es,
+                Aii_inv=Aii.data_ptr() + lo * n_i * n_i * es, info=info.data_ptr() + lo * 4, workspace=None,
+                workspace_bytes=0)
+            wsc = L.hps_local_solve_dtn_workspace_size(C.byref(b))
+            ws = nat.workspace(wsc, dev)
+            b.workspace, b.workspace_bytes = ws.data_ptr(), ws.numel()
+            nat.check(L.hps_local_solve_dtn(C.byref(b), nat.stream_ptr()), "hps_local_solve_dtn")
+            del cc
+
+    _leaf_stage(dtype, n_i, info, run, ((coeffs, 1), (f, 0)), (Y, T, v, h, Aii))
     if v is not None and not multi:
         v, h = v[..., 0], h[..., 0]
     out = (Y, T, v, h)
@@ -319,10 +357,13 @@ def local_solve_stage_uniform_2D_ItI(pde_problem, host_device=None, device=None,
     h = torch.empty((n_leaves, ng, ns), dtype=dtype, device=dev) if ns else None
     Binv = torch.empty((n_leaves, n_pts, n_pts), dtype=dtype, device=dev)
     info = torch.zeros(n_leaves, dtype=torch.int32, device=dev)
-    for flag in ((nat.HPS_INVERSE_REFINED, 0) if refines(dtype, n_pts) else (0,)):
+
+    def run(flag, ins, outs, info):
+        co, f = ins
+        Y, T, v, h, Binv = outs
         a = nat.LeafItiArgs(
-            dtype=nat.TORCH_TO_HPS[dtype] | flag, coef_complex=int(cplx), n_leaves=n_leaves, n_pts=n_pts, n_cb=n_cb,
-            n_gauss=ng, nsrc=ns, n_ops=ops_t.shape[0], ops=ops_t.data_ptr(), coeffs=coeffs.data_ptr(),
+            dtype=nat.TORCH_TO_HPS[dtype] | flag, coef_complex=int(cplx), n_leaves=info.numel(), n_pts=n_pts, n_cb=n_cb,
+            n_gauss=ng, nsrc=ns, n_ops=ops_t.shape[0], ops=ops_t.data_ptr(), coeffs=co.data_ptr(),
             source=nat.ptr(f), G=G.data_ptr(), P=P.data_ptr(), QH=QH.data_ptr(), Y=Y.data_ptr(), T=T.data_ptr(),
             v=nat.ptr(v), h=nat.ptr(h), B_inv=Binv.data_ptr(), info=info.data_ptr(), workspace=None,
             workspace_bytes=0)
@@ -330,8 +371,8 @@ def local_solve_stage_uniform_2D_ItI(pde_problem, host_device=None, device=None,
         ws = nat.workspace(wsb, dev)
         a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
         nat.check(L.hps_local_solve_iti(C.byref(a), nat.stream_ptr()), "hps_local_solve_iti")
-        if not flag or not unrefined([info]):
-            break
+
+    _leaf_stage(dtype, n_pts, info, run, ((coeffs, 1), (f, 0)), (Y, T, v, h, Binv))
     if v is not None and not multi:
         v, h = v[..., 0], h[..., 0]
     out = (Y, T, v, h)
@@ -376,8 +417,8 @@ def merge_level_dtn(T_children: torch.Tensor, h_children, maps, keep_D_inv=False
     (S, g_tilde, T_out, h_out, D_inv, BD_inv) and B when ``keep_B``.
     With ``need_T=False`` the merged map is not formed (T_out is None).  ``refined``,
     a list, lets the inverse be refined where ``refines`` says so and receives
-    its status words: the caller looks at them (``unrefined``) and merges again
-    without the list where one was not refined to double precision."""
+    its status words: the caller looks at them (``unrefined``, ``merge_levels``) and
+    merges again without the list where one was not refined to double precision."""
     L = nat.lib()
     dev = T_children.device
     dtype = T_children.dtype
@@ -450,39 +491,67 @@ def up_level(h_children, D_inv, B, maps, b_is_bd_inv: bool = False, iti: bool = 
     return g_t, h_out
 
 
+def merge_levels(n_levels: int, leaves, level):
+    """level(lvl, T, h, refined) -> (T, h) for lvl = 0 .. n_levels - 1 (leaves first),
+    from leaves() = (T, h).  The status words of all levels are looked at once, after
+    the last: a look per level would leave the GPU idle on small trees.  Where an
+    inverse was not refined, the levels below the first such one run again as they
+    did (their maps are not kept), that level by elimination, and the levels above
+    it are looked at one by one."""
+    T, h = leaves()
+    status = []
+    for lvl in range(n_levels):
+        status.append([])
+        T, h = level(lvl, T, h, status[lvl])
+    if not unrefined([i for s in status for i in s]):
+        return T, h
+    first = next(lvl for lvl, s in enumerate(status) if unrefined(s))
+    T, h = leaves()
+    for lvl in range(n_levels):
+        below = T, h
+        refined = None if lvl == first else []
+        T, h = level(lvl, *below, refined)
+        if lvl > first and unrefined(refined):
+            T, h = level(lvl, *below, None)
+    return T, h
+
+
 def merge_stage_generic(T_arr, h_arr, n_levels: int, maps_fn, device=None, subtree_recomp: bool = False,
                         return_T: bool = False, keep_D_inv: bool = False):
     """Level loop shared by the quad and oct DtN merge stages.  ``maps_fn(nb)``
     gives the merge maps for children with ``nb`` boundary points.  The top
     level's merged map is formed only when it is returned."""
     dev = _device(device)
-    T = T_arr if isinstance(T_arr, torch.Tensor) else _as_tensor(T_arr, torch.float64, dev)
-    T = T.to(dev).contiguous()
-    if T.dim() == 4:
-        T = T.reshape(-1, T.shape[-2], T.shape[-1])
     multi = h_arr is not None and np.ndim(h_arr) == 3 if not isinstance(h_arr, torch.Tensor) else (
         h_arr is not None and h_arr.dim() == 3)
-    h = None
-    if h_arr is not None:
-        h = h_arr if isinstance(h_arr, torch.Tensor) else _as_tensor(h_arr, T.dtype, dev)
-        h = h.to(device=dev, dtype=T.dtype)
-        if h.dim() == 2:
-            h = h.unsqueeze(-1)
-        h = h.reshape(T.shape[0], T.shape[1], -1).contiguous()
-    T_leaf, h_leaf = T, h
-    for refined in ([], None):
-        T, h = T_leaf, h_leaf
-        S_lst, g_lst, Dinv_lst, infos = [], [], [], []
-        for lvl in range(n_levels):
-            maps = maps_fn(T.shape[1])
-            need_T = lvl < n_levels - 1 or return_T or subtree_recomp
-            S, g_t, T, h, D_inv, _ = merge_level_dtn(T, h, maps, keep_D_inv=keep_D_inv, need_T=need_T, infos=infos,
-                                                     refined=refined)
-            S_lst.append(S)
-            g_lst.append(g_t if (g_t is None or multi) else g_t[..., 0])
-            Dinv_lst.append(D_inv)
-        if not unrefined(refined):
-            break
+
+    def leaves():
+        T = T_arr if isinstance(T_arr, torch.Tensor) else _as_tensor(T_arr, torch.float64, dev)
+        T = T.to(dev).contiguous()
+        if T.dim() == 4:
+            T = T.reshape(-1, T.shape[-2], T.shape[-1])
+        h = None
+        if h_arr is not None:
+            h = h_arr if isinstance(h_arr, torch.Tensor) else _as_tensor(h_arr, T.dtype, dev)
+            h = h.to(device=dev, dtype=T.dtype)
+            if h.dim() == 2:
+                h = h.unsqueeze(-1)
+            h = h.reshape(T.shape[0], T.shape[1], -1).contiguous()
+        return T, h
+
+    S_lst, g_lst, Dinv_lst, infos = ([None] * n_levels for _ in range(4))
+
+    def level(lvl, T, h, refined):
+        maps = maps_fn(T.shape[1])
+        need_T = lvl < n_levels - 1 or return_T or subtree_recomp
+        info = []
+        S_lst[lvl], g_t, T, h, Dinv_lst[lvl], _ = merge_level_dtn(T, h, maps, keep_D_inv=keep_D_inv, need_T=need_T,
+                                                                  infos=info, refined=refined)
+        g_lst[lvl] = g_t if (g_t is None or multi) else g_t[..., 0]
+        infos[lvl] = info[0]
+        return T, h
+
+    T, h = merge_levels(n_levels, leaves, level)
     raise_on_sync_timeout(infos)
     if subtree_recomp:
         return T, (h if (h is None or multi) else h[..., 0])
