@@ -424,13 +424,14 @@ static int coop_nct_cap(int n) { return n / 16 < 1 ? 1 : (n / 16 > 1024 ? 1024 :
 
 static size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
-static GjeWs gje_layout(size_t es, int n) {
+static GjeWs gje_layout(int dtype, int n) {
+  const size_t es = dtype_size(dtype);
   GjeWs w;
   w.mat = al256(es * (size_t)n * n);
   w.pan = al256(es * (size_t)n * BP);
   w.u = al256(es * (size_t)n * BP);
   w.g = al256(es * (size_t)BP * n);
-  w.h = al256(es * (size_t)BP * n);
+  w.h = dtype == F64 || dtype == C128 ? al256(es * (size_t)BP * n) : 0;   // FP32 types write the pivot rows directly
   w.e = al256(es * (size_t)BP * BP);
   w.piv = al256(4 * (size_t)n);
   w.rinv = al256(4 * (size_t)n);
@@ -1485,8 +1486,7 @@ static size_t flat_workspace_bytes(int dtype, int n, int batch) {
   if ((dtype == F32 && sblock_fits<float>(n)) || (dtype == F64 && sblock_fits<double>(n)) ||
       (dtype == C64 && sblock_fits<c64>(n)))
     return 0;
-  const size_t es = dtype_size(dtype);
-  return gje_layout(es, n).per * (size_t)batch + 256;
+  return gje_layout(dtype, n).per * (size_t)batch + 256;
 }
 
 // ---------------------------------------------------------------------------
@@ -1695,9 +1695,10 @@ int set_inverse_rec_policy(int policy) {
 static int rec_split(int n) { return (n / 2) & ~3; }
 
 // FP32 workspace of the recursion below for (n, batch): W, S, V of this level,
-// the block info scratch, then the larger of the two half-size sub-problems.
+// then the larger of the two half-size sub-problems; the blocks at its end need
+// their info words only.
 static size_t rec_workspace_bytes(int n, int batch) {
-  if (n <= REC_BLOCK) return al256(sizeof(int) * (size_t)batch) + flat_workspace_bytes(F32, n, batch);
+  if (n <= REC_BLOCK) return al256(sizeof(int) * (size_t)batch);
   const int h1 = rec_split(n), h2 = n - h1;
   const size_t lvl = al256(sizeof(float) * (size_t)batch * ((size_t)h1 * h2 + (size_t)h2 * h2 + (size_t)h2 * h1)) +
                      al256(sizeof(int) * (size_t)batch);
@@ -1997,7 +1998,7 @@ static cudaError_t inverse_batched_flat(int n, const T* A, long long lda, long l
   if (n <= inverse_small_nmax(dtype)) return inverse_small<T>(n, A, lda, sA, X, ldx, sX, batch, info, st);
 
   const size_t es = sizeof(T);
-  const GjeWs L = gje_layout(es, n);
+  const GjeWs L = gje_layout(dtype, n);
   if (ws == nullptr || ws_bytes < L.per * (size_t)batch) {
     set_error("inverse: workspace too small (%zu < %zu)", ws_bytes, L.per * (size_t)batch);
     return cudaErrorInvalidValue;
