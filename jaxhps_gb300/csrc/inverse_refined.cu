@@ -253,7 +253,9 @@ cudaError_t run(int n, const T* A, long long lda, long long sA, T* X, long long 
   if ((size_t)(w - base) > bytes) return cudaErrorInvalidValue;
   const L one_ = one<L>(), zero_ = zero<L>();
   const int gr = (n + RF_NT / 32 - 1) / (RF_NT / 32);   // CTAs for the rows of one matrix
-  const int gl = (n + RF_NT / 8 - 1) / (RF_NT / 8);     // four rows a warp
+  // and for lower_kernel: four rows a warp (fewer flushes) where that fills the SMs
+  // twice, else one (one matrix of 352 took 16 us with four)
+  const int gl = (long long)(n / 32) * cap >= 304 ? (n + RF_NT / 8 - 1) / (RF_NT / 8) : gr;
   const int gx = (int)((nn + RF_NT * 4 - 1) / (RF_NT * 4) < 256 ? (nn + RF_NT * 4 - 1) / (RF_NT * 4) : 256);
   cudaError_t e;
 #define RF_TRY(x)                              \
