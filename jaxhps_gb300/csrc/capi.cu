@@ -467,7 +467,9 @@ static int merge_impl(const hps_merge_args* a, cudaStream_t st, bool iti) {
   const T one_ = one<T>(), zero_ = zero<T>(), mone = make_scalar<T>(-1.0, 0.0);
   // an impedance merge's rows are an identity's and a contraction's: of one scale
   const bool balanced = rscale && !iti && f64_products_on_tensor_cores();
-  if (balanced) HPS_CHECK(balance_rows<T>(nm, ni, ne, with_h ? ns : 0, D, C, with_h ? dh : nullptr, rscale, st));
+  if constexpr (DTypeOf<T>::value == F64 || DTypeOf<T>::value == C128) {
+    if (balanced) HPS_CHECK(balance_rows<T>(nm, ni, ne, with_h ? ns : 0, D, C, with_h ? dh : nullptr, rscale, st));
+  }
   if (nx > 0) {
     // D = [[I, D12], [D21, I]] in colour order; W = I - D12 D21,
     // D^-1 = [[W^-1, -W^-1 D12], [-D21 W^-1, I + D21 W^-1 D12]]

@@ -18,7 +18,9 @@
 // (about 2^-60 of the largest product): the FP64 chain's own rounding is
 // 2^-53 of its partial sums at every step.  An entry of D all of whose large
 // factors meet small ones keeps the bound K 2^-56 max|a_i| max|b_j| only:
-// callers bring rows of such operands to one scale first (leaf_dtn_impl).
+// callers bring rows of such operands to one scale first (leaf_dtn_impl,
+// balance_rows, gje_balance_kernel), and hps_gemm_batched, which knows nothing
+// of its operands, runs here only when asked to.
 //
 // Measured (FP64 chain before, digits): 4096 x (196 x 56 x 196) 21.6 -> 1.22 ms
 // (14.5 TFLOP/s), 512 x (512 x 384 x 512) 82.7 -> 4.2 ms (24.5), 1792^3 10.7
@@ -167,7 +169,8 @@ __device__ __noinline__ double plain_entry(const OzArgs& p, const double* A, con
 // up to 256 columns into consecutive weights' accumulators: A's plane is read
 // from shared memory once for all of them.
 // Registers: 32 columns of 96-bit sums take 96 registers in each of the 256
-// reading threads; the 640 x 96 registers of the launch are divided 144 / 80 / 24.
+// reading threads; the 640 x 96 registers of the launch are divided 144 / 80 / 24,
+// 144 / 72 / 48 with a copying warp (TMA).
 // Every wait is bounded: after one that runs out a warp goes through its loop
 // without waiting (so that the named barrier is met by all) and the CTA frees
 // its tensor memory.

@@ -326,6 +326,8 @@ cudaError_t balance_rows(int nm, int n, int ne, int ns, T* D, T* C, T* dh, doubl
   balance_rows_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(rows, n, ne, ns, D, C, dh, s);
   return cudaGetLastError();
 }
+template cudaError_t balance_rows<double>(int, int, int, int, double*, double*, double*, double*, cudaStream_t);
+template cudaError_t balance_rows<c128>(int, int, int, int, c128*, c128*, c128*, double*, cudaStream_t);
 
 // X[b] (rows x cols, contiguous) with row r scaled by s[b * rows + r].
 template <class T>
@@ -810,7 +812,6 @@ cudaError_t convert(long long n, const S* src, D* dst, cudaStream_t st) {
   template cudaError_t row_equilibrate<T>(int, int, T*, long long, long long, double*, cudaStream_t);              \
   template cudaError_t col_scale<T>(int, int, T*, long long, long long, const double*, cudaStream_t);           \
   template cudaError_t row_scale<T>(int, int, int, T*, const double*, cudaStream_t);                            \
-  template cudaError_t balance_rows<T>(int, int, int, int, T*, T*, T*, double*, cudaStream_t);                  \
   template cudaError_t perm_gather<T>(int, int, int, int, const T*, long long, const int*, int, int, T*,       \
                                       long long, cudaStream_t);                                                  \
   template cudaError_t perm_scatter<T>(int, int, int, int, T*, long long, const int*, int, int, const T*,       \

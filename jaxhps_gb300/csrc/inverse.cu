@@ -1671,9 +1671,10 @@ static cudaError_t launch_block16(int n, const float* A, long long lda, long lon
 }
 
 // The recursion serves n >= REC_MIN and ends at blocks of n <= REC_BLOCK, all
-// on the block Gauss-Jordan (85 us for one block of 112).  Ending at n < 224
-// left blocks of 129 to 223 to the per-column kernel, 325 us each: 84 of them
-// took 27 of 239 ms of the 512-leaf 3D mixed build, the 168 half-size ones 11.
+// on the block Gauss-Jordan (47 us for one block of 112; 85 when this line was
+// drawn).  Ending at n < 224 left blocks of 129 to 223 to the per-column kernel,
+// 325 us each: 84 of them took 27 of 239 ms of the 512-leaf 3D mixed build, the
+// 168 half-size ones 11.
 constexpr int REC_MIN = 224;
 constexpr int REC_BLOCK = 128;
 static int g_inverse_rec_policy = -1;

@@ -1,10 +1,15 @@
 // FP64 and complex128 batched inverses from the single-precision inverse and
 // the residual iteration (Schulz, 1933; its fourth-order form first):
 //
-//   X0 = inverse of A in FP32 / complex64         (pivoted kernels of inverse*.cu)
+//   X0 = inverse of A in FP32 / complex64         (inverse*.cu)
 //   R  = I - A X0,  X1 = X0 + X0 (R + R^2 + R^3)
 //   R  = I - A X1,  X  = X1 + X1 R                where the first R was not small
 //
+// X0 comes from whichever single-precision kernel its size selects, the block
+// inversions among them, which pivot inside blocks of 16 only: on matrices whose
+// leading blocks are nearly singular (indefinite leaves of 400 points and more
+// with two wavelengths and more across) it may be no starting point.  The second
+// residual is what guards the result.
 // The products with A and with X run on the digit kernels (gemm_f64_tc.cu,
 // FP64 and better, or gemm_digits.cu with the digits that a step needs), the
 // powers of R, corrections of R, in single precision: they leave an error of
