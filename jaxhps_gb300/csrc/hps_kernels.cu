@@ -283,6 +283,9 @@ __global__ void __launch_bounds__(256) col_scale_kernel(long long rows_total, in
 // 5e-6, now 1e-16 throughout.  Children that are refined differently give such
 // rows (a DtN row goes as 1 / panel size).  Merges whose rows are of one scale
 // are read once and not written.
+__device__ __forceinline__ uint32_t top_word(double v) { return (uint32_t)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t top_word(c128 v) { return max(top_word(v.x), top_word(v.y)); }
+
 template <class T>
 __global__ void __launch_bounds__(256) balance_rows_kernel(long long rows_total, int n, int ne, int ns, T* D, T* C, T* dh,
                                                            double* s) {
@@ -291,25 +294,19 @@ __global__ void __launch_bounds__(256) balance_rows_kernel(long long rows_total,
   if (row >= rows_total) return;
   const T *first = D + row / n * n * (long long)n;
   T* a = D + row * n;
-  decltype(mag_bits(T())) m = 0, m0 = 0;
+  uint32_t m = 0, m0 = 0;
 #pragma unroll 4
   for (int c = lane; c < n; c += 32) {
-    m = max(m, mag_bits(a[c]));
-    m0 = max(m0, mag_bits(first[c]));
+    m = max(m, top_word(a[c]));
+    m0 = max(m0, top_word(first[c]));
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
-  }
-  const double v = bits_value(m), v0 = bits_value(m0);
-  double f = 1.0;
-  if (v > 0.0 && v0 > 0.0 && v <= 1.7e308 && v0 <= 1.7e308) {
-    const int d = ilogb(v0) - ilogb(v);
-    if (d > 4 || d < -4) f = ldexp(1.0, min(max(d, -1000), 1000));
-  }
+  const int e = (int)(__reduce_max_sync(0xffffffffu, m) >> 20), e0 = (int)(__reduce_max_sync(0xffffffffu, m0) >> 20);
+  // rows of zeros, infinities and NaN stay as they are
+  int d = e > 0 && e0 > 0 && e < 0x7ff && e0 < 0x7ff ? min(max(e0 - e, -1000), 1000) : 0;
+  if (d >= -4 && d <= 4) d = 0;
+  const double f = __hiloint2double((1023 + d) << 20, 0);
   if (lane == 0) s[row] = f;
-  if (f == 1.0) return;
+  if (d == 0) return;
   for (int c = lane; c < n; c += 32) a[c] = scale_by(a[c], f);
   T* x = C + row * ne;
   for (int c = lane; c < ne; c += 32) x[c] = scale_by(x[c], f);
