@@ -90,3 +90,20 @@ def test_the_largest_spans_meet_over_the_rows(cuda):
         A[:, j] *= 2.0 ** -11
         A[j, (j + 1) % n] = 1.0          # its row keeps its scale
         assert set(_inverses(A, 5, nat.HPS_INVERSE_REFINED)[1]) == {nat.INFO_NOT_REFINED}
+
+
+@pytest.mark.parametrize("j", [None, 5, 4097])
+def test_more_columns_than_a_block_keeps(cuda, j):
+    """n = 4100: the columns' spans in two parts.  Accepted and inverted to n 2^-53 times
+    the residual's growth (|X| |A| <= 4 for a diagonal of 3 and rows of norm 1 beside
+    it), or handed back with one column 2^-20 below the others."""
+    n = 4100
+    rng = np.random.default_rng(0)
+    A = rng.standard_normal((n, n)) / np.sqrt(n) + 3 * np.eye(n)
+    if j is not None:
+        A[:, j] *= 2.0 ** -20
+    X, info = _inverses(A, 1, nat.HPS_INVERSE_REFINED)
+    assert info == [0 if j is None else nat.INFO_NOT_REFINED]
+    if j is None:
+        R = torch.as_tensor(A, device="cuda") @ torch.as_tensor(X[0], device="cuda") - torch.eye(n, device="cuda")
+        assert float(R.abs().max()) <= 4 * n * 2.0 ** -53
