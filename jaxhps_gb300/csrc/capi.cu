@@ -809,8 +809,8 @@ int hps_gemm_batched(int dtype, int m, int n, int k, const double* alpha, const 
     set_error("hps_gemm_batched: invalid arguments");
     return HPS_ERR_ARG;
   }
-  DISPATCH(dtype & ~HPS_PRODUCT_DIGITS, gemm_entry, (dtype & HPS_PRODUCT_DIGITS) != 0, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc, strideC, D, ldd,
-           strideD, batch, stream)
+  DISPATCH(dtype & ~HPS_PRODUCT_DIGITS, gemm_entry, (dtype & HPS_PRODUCT_DIGITS) != 0, m, n, k, alpha, A, lda, strideA,
+           B, ldb, strideB, beta, C, ldc, strideC, D, ldd, strideD, batch, stream)
 }
 
 size_t hps_inverse_workspace_size(int dtype, int n, int batch) {

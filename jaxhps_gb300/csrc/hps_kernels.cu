@@ -270,7 +270,8 @@ __global__ void __launch_bounds__(256) col_scale_kernel(long long rows_total, in
 #pragma unroll 4
   for (int c = lane; c < n; c += 32) {
     const double f = s[b * n + c];
-    if (f != 1.0) x[c] = scale_by(x[c], f);
+    const T v = x[c];
+    if (f != 1.0) x[c] = scale_by(v, f);
   }
 }
 
